@@ -207,60 +207,145 @@ __global__ void __launch_bounds__(GS > 256 ? GS : 256)
 // A tile is one 256-thread block over 64 bytes of each operand per thread
 // (2048 u64 limbs).  Tiles take their index from an atomic counter in launch
 // order, so every tile a tile waits for has already started and will finish
-// (no dependence on the scheduler).  A plain addition first reads the 32 limbs
-// below its tile: the nearest one whose sum is not all ones gives the
-// carry-in directly, which settles almost every tile of random data without
-// waiting (the tile then only publishes its inclusive status).  Otherwise, and
-// for 6a + 10b, each tile adds its limbs with carry-in 0,
-// publishes its status word -- inclusive (its true carry-out) when it does not
+// (no dependence on the scheduler); the order goes round the instances, so
+// that few tiles of one instance are in flight at a time.  A plain addition
+// first reads the 32 limbs below its tile: the nearest one whose sum is not
+// all ones gives the carry-in directly, which settles almost every tile of
+// random data without waiting (the tile then only publishes its state).
+// Otherwise, and for 6a + 10b, each tile adds its limbs with carry-in 0,
+// publishes its state -- inclusive (its true carry-out) when it does not
 // propagate a carry or is the first tile of its instance, otherwise an
 // aggregate that says "passes the carry-in through" -- then it walks back
-// over aggregates to the nearest inclusive status, bounded by spin_limit polls
-// of an unpublished word (then the error word is set and the tile carries on
+// over aggregates to the nearest inclusive tile, bounded by spin_limit polls
+// of an unpublished one (then the error word is set and the tile carries on
 // with carry-in 0, so the kernel always completes), publishes its own
-// inclusive status, and the block redoes the carry pass with that carry-in.
-// The walk back is done by a warp, 32 predecessors per step.
-// Status word: bits 0-1 state (1 aggregate, 2 inclusive), bit 2 carry value,
-// bits 3-31 the launch's epoch (a word of another epoch is unpublished).
+// inclusive state, and the block redoes the carry pass with that carry-in.
+//
+// States are two bits per tile, 32 tiles to a 64-bit word (tile i of a word:
+// bit 32 + i inclusive, bit i aggregate or, with bit 32 + i, a carry of one;
+// neither: unpublished), added by the tile itself, so a warp's walk back reads
+// 1024 tiles per step.  (One word per tile, 32 tiles per step, let a run of
+// propagating tiles advance by 32 tiles per round trip to the L2: a number of
+// 2^24 limbs that carries from end to end took 175-197 us; 128 words per step
+// from every waiting tile took 227 us, the polls in each other's way.)  The
+// words need no ordering with other memory, being all that a waiting tile
+// reads of another: relaxed accesses (a release made every tile wait for a
+// memory barrier before its stores: 16 x 2^20 limbs 66.7 us against 61.0).
 
-constexpr uint32_t ST_AGG = 1u, ST_INC = 2u;
-
-__device__ __forceinline__ void st_release(uint32_t* p, uint32_t v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-__device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
-    uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+__device__ __forceinline__ uint64_t ld_status(const uint64_t* p) {
+    uint64_t v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
+__device__ __forceinline__ void add_status(uint64_t* p, uint64_t v) {
+    asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
 
-template <typename L, bool VEC, int OP>
+// Within a tile, warp w owns 32 * Q consecutive limbs (Q = 64 bytes' worth) as
+// R rows of 32 * V: lane i of row r holds V = 16 bytes of limbs on 16-byte
+// aligned rows, V = 1 limb on others, so every load and store of a warp is
+// one contiguous run whatever the alignment (with 64 bytes per thread, rows
+// that allow no 16-byte access were read at a stride of 64 bytes: 16 x 1048573
+// limbs 125 us).  A row's carries are one lookahead over its two ballots, the
+// rows of a warp chained by their one-bit carry; the ballots are kept, so the
+// second pass (with the warp's true carry-in) is integer work only.
+template <typename L, int V>
+__device__ __forceinline__ void load_row(const L* __restrict__ row, uint32_t i, uint32_t m, L (&v)[V]) {
+    if constexpr (V > 1) {
+        if (i + V <= m) {
+            const uint4 q = __ldcs(reinterpret_cast<const uint4*>(row + i));
+            unpack16<L, V>(q, v);
+            return;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < V; ++k) v[k] = i + k < m ? ld_stream(row + i + k) : L(0);
+}
+
+template <typename L, int V>
+__device__ __forceinline__ void store_row(L* __restrict__ row, uint32_t i, uint32_t m, const L (&v)[V]) {
+    if constexpr (V > 1) {
+        if (i + V <= m) {
+            __stcs(reinterpret_cast<uint4*>(row + i), pack16<L, V>(v));
+            return;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < V; ++k)
+        if (i + k < m) st_stream(row + i + k, v[k]);
+}
+
+// High word (at most 15) of the limb 6 a_i + 10 b_i.
+__device__ __forceinline__ uint64_t six_hi(uint64_t ai, uint64_t bi) {
+    const uint64_t pa = ai * 6u, pb = bi * 10u;
+    return __umul64hi(ai, 6u) + __umul64hi(bi, 10u) + uint64_t(pa + pb < pa);
+}
+
+// What a tile needs of the limbs below it, as one byte.  Plain addition: its
+// carry-in (0 or 1) where the nearest of the 32 limbs below whose sum is not
+// all ones gives it, else 2.  6a + 10b: the high word of the limb below.  By
+// the 32 lanes of a warp; i is the tile's first limb.
+template <typename L, int OP>
+__device__ __forceinline__ uint32_t tile_edge(const L* __restrict__ a, const L* __restrict__ b, uint64_t i,
+                                              uint32_t lane) {
+    if constexpr (OP == ADD_SIX) {
+        return uint32_t(six_hi(a[i - 1], b[i - 1]));
+    } else {
+        const L ai = a[i - 1 - lane], bi = b[i - 1 - lane];  // lane 0 is the limb just below the tile
+        const L si = ai + bi;
+        const uint32_t settled = __ballot_sync(MI_FULL_MASK, si != L(~L(0)));
+        const uint32_t gen = __ballot_sync(MI_FULL_MASK, si < ai);
+        return settled ? (gen >> (__ffs(settled) - 1)) & 1u : 2u;
+    }
+}
+
+// In-place calls: the edge bytes of every tile, taken before any tile
+// overwrites the limbs below its neighbour.  One warp per tile.
+template <typename L, int OP>
 __global__ void __launch_bounds__(256)
+    k_wide_edges(const L* __restrict__ a, const L* __restrict__ b, uint32_t m, uint32_t tiles_per, uint32_t n_tiles,
+                 uint8_t* __restrict__ edges) {
+    constexpr uint32_t W = 256u * (64 / uint32_t(sizeof(L)));
+    pdl_wait();  // launched with launch_pdl
+    const uint32_t tile = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+    if (tile >= n_tiles || tile % tiles_per == 0) return;
+    const uint64_t off = uint64_t(tile / tiles_per) * m;
+    const uint32_t e = tile_edge<L, OP>(a + off, b + off, uint64_t(tile % tiles_per) * W, lane);
+    if (lane == 0) edges[tile] = uint8_t(e);
+}
+
+// edges: the bytes of k_wide_edges when r is a or b, else null (each tile then
+// reads the limbs below it itself).
+template <typename L, int V, int OP>
+__global__ void __launch_bounds__(256, sizeof(L) == 8 ? 4 : 2)
     k_add_wide(const L* __restrict__ a, const L* __restrict__ b, L* __restrict__ r, uint8_t* __restrict__ carry,
-               uint32_t m, uint32_t tiles_per, uint32_t n_tiles, uint32_t* status, uint32_t spin_limit,
-               uint32_t withhold, uint64_t base, uint32_t epoch) {
+               uint32_t m, uint32_t tiles_per, uint32_t n_tiles, uint64_t* status, uint64_t* old, uint32_t old_words,
+               unsigned long long* counter, uint32_t* err, uint32_t spin_limit, uint32_t withhold, uint64_t base,
+               const uint8_t* __restrict__ edges) {
     constexpr int Q = 64 / int(sizeof(L));
-    constexpr uint32_t W = 256u * Q;  // limbs per tile
-    __shared__ uint32_t scratch[8];
-    __shared__ uint64_t shift[8];
+    constexpr int R = Q / V;           // rows per warp
+    constexpr uint32_t W = 256u * Q;   // limbs per tile
+    __shared__ uint32_t wflag[8];      // per warp: bit 0 generate (carry-in 0), bit 1 propagate
     __shared__ uint32_t s_tile, s_cin;
     // a monotonic tile counter (this launch's tiles are base .. base+n_tiles-1)
-    // and tile words tagged with the launch's epoch: nothing is cleared
-    // between launches; a word of an older epoch reads as unpublished
-    unsigned long long* counter = reinterpret_cast<unsigned long long*>(status + kWideTiles);
-    uint32_t* err = status + kWideTiles + 2;
+    // and two arrays of state words, taken in turn: each launch clears the
+    // words of the launch before it (old), so nothing is cleared in between
     pdl_wait();  // launched with launch_pdl: the previous launch has completed
     if (threadIdx.x == 0) s_tile = uint32_t(atomicAdd(counter, 1ull) - base);
     __syncthreads();
-    const uint32_t tile = s_tile;
-    if (tile >= n_tiles) return;  // (the grid has exactly n_tiles blocks)
-    const uint32_t inst = tile / tiles_per, j = tile % tiles_per;
-    const uint32_t t = threadIdx.x;
+    if (s_tile >= n_tiles) return;  // (the grid has exactly n_tiles blocks)
+    const uint32_t n_inst = n_tiles / tiles_per;
+    const uint32_t inst = s_tile % n_inst, j = s_tile / n_inst;
+    uint64_t* words = status + size_t(inst) * ((tiles_per + 31) / 32);  // the instance's states
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    for (uint32_t i = s_tile + n_tiles * t; i < old_words; i += n_tiles * 256) old[i] = 0;
     const uint64_t off = uint64_t(inst) * m;
-    const uint32_t start = j * W + t * Q;
-    L x[Q], y[Q], s[Q];
-    load_chunk<L, Q, VEC>(a + off, start, m, true, x);
-    load_chunk<L, Q, VEC>(b + off, start, m, true, y);
+    const uint32_t start = j * W + warp * (32 * Q) + lane * V;  // the thread's limbs of row 0; row r is 32 V r further
+    L x[R][V], y[R][V], s[R][V];
+#pragma unroll
+    for (int k = 0; k < R; ++k) load_row<L, V>(a + off, start + 32 * V * k, m, x[k]);
+#pragma unroll
+    for (int k = 0; k < R; ++k) load_row<L, V>(b + off, start + 32 * V * k, m, y[k]);
     // Carry-in straight from the 32 limbs below the tile: the nearest limb
     // whose sum is not all ones decides it (generate: 1, kill: 0).  Random
     // limbs almost always settle it here and the tile never waits; only a
@@ -268,60 +353,81 @@ __global__ void __launch_bounds__(256)
     uint32_t local_cin = 0;
     bool local_ok = j == 0;
     if (OP == ADD_PLAIN && j > 0 && t < 32) {
-        const uint64_t i = uint64_t(j) * W - 1 - t;  // lane 0 is the limb just below the tile
-        const L ai = a[off + i], bi = b[off + i];
-        const L si = ai + bi;
-        const uint32_t settled = __ballot_sync(MI_FULL_MASK, si != L(~L(0)));
-        const uint32_t gen = __ballot_sync(MI_FULL_MASK, si < ai);
-        if (settled) {
-            local_ok = true;
-            local_cin = (gen >> (__ffs(settled) - 1)) & 1u;
-        }
+        const uint32_t e = edges != nullptr ? edges[inst * tiles_per + j]
+                                            : tile_edge<L, OP>(a + off, b + off, uint64_t(j) * W, lane);
+        local_ok = e < 2;
+        local_cin = e & 1u;
     }
     if constexpr (OP == ADD_SIX) {
-        // 6a + 10b as lo + (hi shifted up one limb), as in k_add; thread 0
-        // recomputes the high word of the limb before its tile
+        // 6a + 10b as lo + (hi shifted up one limb), as in k_add; lane 0 takes
+        // the row before from lane 31, and for its first row recomputes the
+        // high word of the limb before its warp's span
         static_assert(sizeof(L) == 8, "6a + 10b is defined on u64 limbs");
-        L hi[Q];
+        uint64_t before = 0;
+        if (lane == 0 && start > 0 && start - 1 < m)
+            before = warp == 0 && edges != nullptr ? edges[inst * tiles_per + j]
+                                                   : six_hi(a[off + start - 1], b[off + start - 1]);
 #pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            const L pa = x[q] * 6u, pb = y[q] * 10u;
-            const L lo = pa + pb;
-            hi[q] = __umul64hi(x[q], 6u) + __umul64hi(y[q], 10u) + L(lo < pa);
-            x[q] = lo;
-        }
-        uint64_t prev = group_shift_up<256>(hi[Q - 1], t, shift);
-        if (t == 0 && j > 0) {
-            const L xp = a[off + j * W - 1], yp = b[off + j * W - 1];
-            const L pa = xp * 6u, pb = yp * 10u;
-            prev = __umul64hi(xp, 6u) + __umul64hi(yp, 10u) + L(pa + pb < pa);
-        }
-        y[0] = prev;
+        for (int k = 0; k < R; ++k) {
+            L hi[V];
 #pragma unroll
-        for (int q = 1; q < Q; ++q) y[q] = hi[q - 1];
+            for (int v = 0; v < V; ++v) {
+                hi[v] = six_hi(x[k][v], y[k][v]);
+                x[k][v] = x[k][v] * 6u + y[k][v] * 10u;
+            }
+            const uint64_t up = __shfl_up_sync(MI_FULL_MASK, uint64_t(hi[V - 1]), 1);
+            y[k][0] = lane == 0 ? before : up;
+#pragma unroll
+            for (int v = 1; v < V; ++v) y[k][v] = hi[v - 1];
+            before = __shfl_sync(MI_FULL_MASK, uint64_t(hi[V - 1]), 31);  // lane 0's next row
+        }
     }
-    bool g, p;
-    chunk_add<L, Q>(x, y, s, g, p);
-    uint32_t gc0;
-    (void)group_carry<256>(g, p, 0u, &gc0, scratch);
-    const bool P = __syncthreads_and(p) != 0;  // the tile passes a carry-in through
+    uint32_t G[R], P[R], c = 0;  // each row's generate and propagate ballots
+    bool ones = true;
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        bool g, p;
+        chunk_add<L, V>(x[k], y[k], s[k], g, p);
+        G[k] = __ballot_sync(MI_FULL_MASK, g);
+        P[k] = __ballot_sync(MI_FULL_MASK, p);
+        c = uint32_t((uint64_t(G[k] | P[k]) + G[k] + c) >> 32);
+        ones = ones && P[k] == MI_FULL_MASK;
+    }
+    if (lane == 0) wflag[warp] = c | (ones ? 2u : 0u);
+    __syncthreads();
+    // the tile's generate and propagate, and the carry into each warp: a
+    // lookahead over the eight warps
+    uint32_t WG = 0, WP = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+        const uint32_t f = wflag[w];
+        WG |= (f & 1u) << w;
+        WP |= (f >> 1) << w;
+    }
+    const uint32_t gc0 = ((WG | WP) + WG) >> 8;
+    const bool all = WP == 0xffu;  // the tile passes a carry-in through
     if (t < 32) {
-        // warp 0 looks back 32 tiles at a time: lane l reads tile k - l; the
-        // carry-in is the value of the nearest inclusive tile, valid once
-        // every tile between (all propagating aggregates) has published
+        // warp 0 looks back 1024 tiles at a time: lane l reads the states of
+        // word g - l; the carry-in is the value of the nearest inclusive tile,
+        // valid once every tile between (all propagating aggregates) has
+        // published
+        const uint64_t agg = 1ull << (j & 31u), inc = agg << 32;  // the tile's own bits
         uint32_t cin = local_cin;
         if (!local_ok) {
-            if (t == 0) st_release(status + tile, (epoch << 3) | (P ? ST_AGG : (ST_INC | (gc0 << 2))));
-            const int32_t first = int32_t(tile - j);  // the instance's first tile: always inclusive
-            int32_t k = int32_t(tile) - 1;
+            if (t == 0) add_status(words + (j >> 5), all ? agg : (gc0 ? inc + agg : inc));
+            int32_t g = int32_t(j >> 5);
+            uint32_t below = (1u << (j & 31u)) - 1u;  // the tiles of this tile's own word that precede it
             uint32_t spins = 0;
             for (;;) {
-                const int32_t i = k - int32_t(t);
-                const uint32_t raw = i >= first ? ld_acquire(status + i) : ((epoch << 3) | ST_INC);
-                const uint32_t sv = (raw >> 3) == epoch ? (raw & 7u) : 0u;
-                const uint32_t inc = __ballot_sync(MI_FULL_MASK, (sv & 3u) == ST_INC);
-                const uint32_t pending = __ballot_sync(MI_FULL_MASK, (sv & 3u) == 0u);
-                const uint32_t nearest = inc ? uint32_t(__ffs(inc) - 1) : 32u;
+                const int32_t i = g - int32_t(t);
+                const uint64_t w = i >= 0 ? ld_status(words + i) : 1ull << 63;  // (tile 0 is always inclusive)
+                const uint32_t hi = uint32_t(w >> 32), lo = uint32_t(w);
+                const uint32_t stop = ~(lo & ~hi) & (t == 0 ? below : MI_FULL_MASK);  // not aggregates
+                const uint32_t top = 31u - __clz(stop);  // the nearest of them
+                const bool known = stop != 0 && ((hi >> top) & 1u);
+                const uint32_t found = __ballot_sync(MI_FULL_MASK, known);
+                const uint32_t pending = __ballot_sync(MI_FULL_MASK, stop != 0 && !known);
+                const uint32_t nearest = found ? uint32_t(__ffs(found) - 1) : 32u;
                 const uint32_t nearer = nearest == 32u ? MI_FULL_MASK : ((1u << nearest) - 1u);
                 if (pending & nearer) {
                     if (++spins > spin_limit) {
@@ -331,45 +437,57 @@ __global__ void __launch_bounds__(256)
                     __nanosleep(64);
                     continue;
                 }
-                if (inc) {
-                    cin = (__shfl_sync(MI_FULL_MASK, sv, int(nearest)) >> 2) & 1u;
+                if (found) {
+                    cin = __shfl_sync(MI_FULL_MASK, (lo >> (top & 31u)) & 1u, int(nearest));
                     break;
                 }
-                k -= 32;
+                g -= 32;
+                below = MI_FULL_MASK;
             }
         }
         if (t == 0) {
-            if (!(withhold && j == 0))
-                st_release(status + tile, (epoch << 3) | ST_INC | ((gc0 | (P ? cin : 0u)) << 2));
+            const uint32_t cout = gc0 | (all ? cin : 0u);
+            if (local_ok) {
+                if (!(withhold && j == 0)) add_status(words + (j >> 5), cout ? inc + agg : inc);
+            } else if (all) {
+                add_status(words + (j >> 5), cout ? inc : inc - agg);  // the aggregate becomes inclusive
+            }
             s_cin = cin;
         }
     }
     __syncthreads();
-    uint32_t gc;
-    const uint32_t c = group_carry<256>(g, p, s_cin, &gc, scratch);
-    chunk_inc<L, Q>(s, c);
-    store_chunk<L, Q, VEC>(r + off, start, m, true, s);
+    const uint32_t WX = WG | WP, WS = WX + WG + s_cin;
+    c = ((WS ^ WX ^ WG) >> warp) & 1u;  // into the warp
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        const uint64_t X = G[k] | P[k], Y = G[k], S = X + Y + c;
+        chunk_inc<L, V>(s[k], uint32_t((S ^ X ^ Y) >> lane) & 1u);
+        c = uint32_t(S >> 32);
+        store_row<L, V>(r + off, start + 32 * V * k, m, s[k]);
+    }
     if (OP == ADD_PLAIN && carry != nullptr && j == tiles_per - 1) {
         // carry-out: the value at limb m (zero padding plus the carry), or
         // the tile's carry-out when the instance ends with the tile
         if (m % W != 0) {
 #pragma unroll
-            for (int q = 0; q < Q; ++q)
-                if (start + q == m) carry[inst] = uint8_t(s[q]);
+            for (int k = 0; k < R; ++k)
+#pragma unroll
+                for (int v = 0; v < V; ++v)
+                    if (start + 32 * V * k + v == m) carry[inst] = uint8_t(s[k][v]);
         } else if (t == 255) {
-            carry[inst] = uint8_t(gc);
+            carry[inst] = uint8_t(WS >> 8);
         }
     }
 }
 
-// Rounds of whole instances, at most kWideTiles tiles each; every round is a
-// new epoch of the tile words and takes the next n_tiles values of the tile
-// counter, so nothing is cleared between launches (the words are cleared
-// only when the 29-bit epoch wraps).
+// Rounds of whole instances, at most kWideTiles tiles each; every round takes
+// the next n_tiles values of the tile counter and the other array of state
+// words, clearing the words of the round before.
 template <typename L, bool VEC, int OP>
 mi_status launch_wide(const L* a, const L* b, L* r, uint8_t* carry, uint32_t n, uint32_t m, WideState& w,
                       cudaStream_t st) {
     constexpr uint32_t W = 256u * (64 / uint32_t(sizeof(L)));
+    constexpr int V = VEC ? 16 / int(sizeof(L)) : 1;  // limbs per access
     const uint32_t tiles_per = (m + W - 1) / W;
     const uint32_t cap = w.round_tiles < kWideTiles ? w.round_tiles : kWideTiles;
     if (tiles_per > cap) return set_error(MI_EINVAL, "add: %u limbs exceeds the multi-block maximum", m);
@@ -377,16 +495,23 @@ mi_status launch_wide(const L* a, const L* b, L* r, uint8_t* carry, uint32_t n, 
     for (uint32_t i0 = 0; i0 < n; i0 += per_round) {
         const uint32_t k = (n - i0) < per_round ? (n - i0) : per_round;
         const uint32_t n_tiles = k * tiles_per;
-        if (w.epoch >= (1u << 29) - 1) {  // the epoch field wraps: start over from cleared words
-            MI_CUDA_TRY(cudaMemsetAsync(w.status, 0, size_t(kWideTiles) * 4, st));
-            w.epoch = 0;
-        }
-        ++w.epoch;
+        const uint32_t words = k * ((tiles_per + 31) / 32);  // tiles_per >= 2, so at most kWideWords
         const uint64_t o = uint64_t(i0) * m;
-        MI_CUDA_TRY(launch_pdl(k_add_wide<L, VEC, OP>, dim3(n_tiles), dim3(256), 0, st, a + o, b + o, r + o,
-                               carry ? carry + i0 : nullptr, m, tiles_per, n_tiles, w.status, w.spin_limit,
-                               w.withhold, w.issued, w.epoch));
+        uint8_t* edges = nullptr;
+        if (r == a || r == b) {
+            edges = reinterpret_cast<uint8_t*>(w.status + 2 * kWideWords + 2);
+            MI_CUDA_TRY(launch_pdl(k_wide_edges<L, OP>, dim3((n_tiles + 7) / 8), dim3(256), 0, st, a + o, b + o, m,
+                                   tiles_per, n_tiles, edges));
+        }
+        MI_CUDA_TRY(launch_pdl(k_add_wide<L, V, OP>, dim3(n_tiles), dim3(256), 0, st, a + o, b + o, r + o,
+                               carry ? carry + i0 : nullptr, m, tiles_per, n_tiles,
+                               w.status + w.parity * kWideWords, w.status + (w.parity ^ 1u) * kWideWords,
+                               w.old_words, reinterpret_cast<unsigned long long*>(w.status + 2 * kWideWords),
+                               reinterpret_cast<uint32_t*>(w.status + 2 * kWideWords + 1), w.spin_limit, w.withhold,
+                               w.issued, edges));
         w.issued += n_tiles;  // every block of the launch takes one counter value
+        w.old_words = words;
+        w.parity ^= 1u;
     }
     return MI_OK;
 }

@@ -10,23 +10,28 @@ namespace mi {
 
 enum AddOp : int { ADD_PLAIN = 0, ADD_SIX = 1 };
 
-// Batched addition on u64 or u32 limbs (op = ADD_PLAIN or ADD_SIX).
-// Arguments are already validated; n > 0, limbs > 0.
 // Device state of the additions wider than one block (decoupled look-back):
-// `status` holds kWideTiles tile words, then the 64-bit tile counter, then the
-// error word (set when a bounded wait gave up).  One per context; wide
-// additions on one context must not overlap on the device.  The host side
-// keeps the epoch of the last launch and the counter values issued so far.
-constexpr uint32_t kWideTiles = 1u << 16;
+// `status` holds two arrays of kWideWords words of tile states (32 tiles per
+// word, two bits each), then the tile counter, then the error word (set when
+// a bounded wait gave up), then one byte per tile for in-place calls.  One per context; wide additions on one context
+// must not overlap on the device.  The host side keeps which array the next
+// launch takes, how many words of the other the last one used, and the
+// counter values issued so far.
+constexpr uint32_t kWideTiles = 1u << 16;  // per launch
+constexpr uint32_t kWideWords = kWideTiles / 2;  // an instance has at least two tiles and starts a word
+constexpr size_t kWideBytes = (2 * size_t(kWideWords) + 2) * 8 + kWideTiles;
 struct WideState {
-    uint32_t* status = nullptr;    // kWideTiles + 4 words
-    uint32_t epoch = 0;            // of the last launch (tile words carry it)
+    uint64_t* status = nullptr;    // kWideBytes
+    uint32_t parity = 0;           // array of the next launch
+    uint32_t old_words = 0;        // words of the other array to clear
     uint64_t issued = 0;           // tile counter values taken by earlier launches
     uint32_t spin_limit = 1u << 20;  // polls of an unpublished predecessor before giving up
     uint32_t withhold = 0;         // tests only: first tiles never publish (makes the waits run out)
     uint32_t round_tiles = kWideTiles;  // tiles per launch (at most kWideTiles)
 };
 
+// Batched addition on u64 or u32 limbs (op = ADD_PLAIN or ADD_SIX).
+// Arguments are already validated; n > 0, limbs > 0.
 // thread_bytes: operand bytes each thread owns (16, 32 or 64; raised where the
 // instance would need a group of more than 1024 threads).  Instances wider
 // than one group (limbs above kAddMaxLimbs64 u64 limbs) take the multi-block

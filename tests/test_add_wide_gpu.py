@@ -126,3 +126,30 @@ def test_wide_add_timeout_is_reported_and_context_survives(wctx, devmem):
     wctx.host_add(a, b, r, c, 3, m)
     assert np.array_equal(r, ra) and np.array_equal(c, ca)
     assert wctx.device_status() == midint.MI_OK
+
+
+@pytest.mark.parametrize("n,m,bits", [(3, 31 * 2048, 64), (3, 33 * 2048 + 5, 64), (4, 1030 * 2048 + 1, 64),
+                                      (700, 5000, 64), (701, 4099, 64), (3, 33 * 4096 + 7, 32)])
+@pytest.mark.parametrize("op", ["add", "add_in_a", "add_in_b", "six", "six_in_a"])
+def test_wide_add_words_of_states_and_in_place(wctx, devmem, n, m, bits, op):
+    # 31, 33 and 1030 tiles per instance (one word of 32 tile states, two, more
+    # than the 1024 of one look-back step), many instances in turn, and results
+    # over an operand
+    if bits == 32 and op.startswith("six"):
+        pytest.skip("6a + 10b is defined on u64 limbs")
+    a, b = carry_stress(n, m, seed=n + m, dtype=np.uint64 if bits == 64 else np.uint32)
+    words = a.view(np.uint32).size
+    _, pa = keep_a = devmem.put(a, 0)
+    _, pb = keep_b = devmem.put(b, 0)
+    _, pr = keep_r = keep_a if op.endswith("in_a") else keep_b if op.endswith("in_b") else devmem.empty_words(words, 0)
+    dc = torch.zeros(n, dtype=torch.uint8, device="cuda:0")
+    s = torch.cuda.current_stream().cuda_stream
+    if op.startswith("six"):
+        wctx.add6(pa, pb, pr, n, m, stream=s)
+        want, carry = O.add6(a, b, m), np.zeros(n, np.uint8)
+    else:
+        wctx.add(pa, pb, pr, n, m, carry=dc.data_ptr(), limb_bits=bits, stream=s)
+        want, carry = O.add(a, b, m)
+    assert wctx.device_status() == midint.MI_OK
+    assert np.array_equal(devmem.get(keep_r[0], words, 0, a.dtype), want)
+    assert np.array_equal(dc.cpu().numpy(), carry)

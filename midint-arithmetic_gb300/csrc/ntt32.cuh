@@ -133,14 +133,14 @@ struct Plan {
 };
 
 // Moves the thread's 8 residues of each of NA arrays (each with its own LX
-// words of `sh`) from layout (stride) d_from to d_to through shared memory.
+// words of `sh`, GAP words apart) from layout (stride) d_from to d_to through shared memory.
 // In a layout of stride d <= 32 the residues of a warp are the 256
 // consecutive words of its own block, so an exchange between two such
 // layouts only synchronises the warp; the others synchronise the block.  The
 // first barrier makes every earlier read of the words about to be written
 // complete (the transforms start with a block-wide exchange, and between
 // transforms `sh` is only read by the thread that wrote it).
-template <int LG, int NA>
+template <int LG, int NA, int GAP = Plan<LG>::LX>
 __device__ __forceinline__ void exchange(uint32_t (&x)[NA][8], uint32_t* sh, int d_from, int d_to) {
     using P = Plan<LG>;
     const uint32_t t = threadIdx.x % P::NT;
@@ -148,7 +148,7 @@ __device__ __forceinline__ void exchange(uint32_t (&x)[NA][8], uint32_t* sh, int
     if (local) __syncwarp(); else __syncthreads();
 #pragma unroll
     for (int q = 0; q < NA; ++q) {
-        uint32_t* s = sh + q * P::LX;
+        uint32_t* s = sh + q * GAP;
         const uint32_t b = P::xbase(d_from, t);
         if (d_from == 1) {
 #pragma unroll
@@ -162,7 +162,7 @@ __device__ __forceinline__ void exchange(uint32_t (&x)[NA][8], uint32_t* sh, int
     if (local) __syncwarp(); else __syncthreads();
 #pragma unroll
     for (int q = 0; q < NA; ++q) {
-        const uint32_t* s = sh + q * P::LX;
+        const uint32_t* s = sh + q * GAP;
         const uint32_t b = P::xbase(d_to, t);
         if (d_to == 1) {
 #pragma unroll
@@ -185,8 +185,9 @@ __device__ __forceinline__ void exchange(uint32_t (&x)[NA][8], uint32_t* sh, int
 // (natural order), values in [0, 2p).  Out: layout stride 1 (x[q][j] = slot
 // 8t+j of the bit-reversed spectrum), values in [0, 2p).  HALF: residues
 // L/2.. are zero (x[q][4..7] are not read), so the first stage of the first
-// pass is x[j + 4] = x[j] w with x[j] unchanged.
-template <int LG, int NA, bool HALF = false>
+// pass is x[j + 4] = x[j] w with x[j] unchanged.  GAP: words between the
+// arrays' exchange buffers.
+template <int LG, int NA, bool HALF = false, int GAP = Plan<LG>::LX>
 __device__ __forceinline__ void forward(uint32_t (&x)[NA][8], uint32_t* sh, const uint2* __restrict__ tw_all,
                                         const Field& f) {
     using P = Plan<LG>;
@@ -204,7 +205,7 @@ __device__ __forceinline__ void forward(uint32_t (&x)[NA][8], uint32_t* sh, cons
 #pragma unroll
     for (int k = 0; k < P::NF; ++k) {
         const int d = P::d(k);
-        if (k > 0) exchange<LG, NA>(x, sh, P::d(k - 1), d);
+        if (k > 0) exchange<LG, NA, GAP>(x, sh, P::d(k - 1), d);
         const uint32_t off = t % d, e0 = TwLayout::pass(LG, k) + off;
         if (HALF && k == 0) {
 #pragma unroll
@@ -226,7 +227,7 @@ __device__ __forceinline__ void forward(uint32_t (&x)[NA][8], uint32_t* sh, cons
         for (int j = 0; j < 8; j += 2) bf(j, j + 1, e0 + 6 * d);
     }
     if constexpr (P::R > 0) {
-        exchange<LG, NA>(x, sh, P::d(P::NF - 1), 1);
+        exchange<LG, NA, GAP>(x, sh, P::d(P::NF - 1), 1);
         if constexpr (P::R == 2) {
             const uint2 w1 = __ldg(tw + TwLayout::quarter(LG));
 #pragma unroll
@@ -251,7 +252,7 @@ __device__ __forceinline__ void forward(uint32_t (&x)[NA][8], uint32_t* sh, cons
     }
 }
 
-// Inverse transform without the 1/L scaling (DIT).  In: stride-1 layout of a
+// Inverse transforms of NA arrays in lockstep, without the 1/L scaling (DIT).  In: stride-1 layout of a
 // bit-reversed spectrum, values in [0, 2p); out: x[j] = residue t + L/8*j in
 // natural order, values in [0, 2p).  In between the values are kept in
 // [0, 4p) (Harvey's lazy butterflies): a butterfly brings its unmultiplied
@@ -259,38 +260,45 @@ __device__ __forceinline__ void forward(uint32_t (&x)[NA][8], uint32_t* sh, cons
 // other is in [0, 2p) for any 32-bit input, and both outputs u + v and
 // u - v + 2p stay below 4p < 2^32 -- two integer instructions per butterfly
 // fewer than reducing both outputs.
-template <int LG>
-__device__ __forceinline__ void inverse(uint32_t (&x)[8], uint32_t* sh, const uint2* __restrict__ itw_all,
+template <int LG, int NA>
+__device__ __forceinline__ void inverse(uint32_t (&x)[NA][8], uint32_t* sh, const uint2* __restrict__ itw_all,
                                         const Field& f) {
-    uint32_t(&xs)[1][8] = reinterpret_cast<uint32_t(&)[1][8]>(x);
     using P = Plan<LG>;
     const uint32_t t = threadIdx.x % P::NT;
     const uint2* __restrict__ itw = itw_all + TwLayout::base(LG);
     auto bf = [&](int j, int k, uint32_t e) {
-        const uint32_t u = f.reduce2(x[j]), v = f.shoup(x[k], __ldg(itw + e));
-        x[j] = u + v;
-        x[k] = u + f.p2 - v;
+        const uint2 w = __ldg(itw + e);
+#pragma unroll
+        for (int q = 0; q < NA; ++q) {
+            const uint32_t u = f.reduce2(x[q][j]), v = f.shoup(x[q][k], w);
+            x[q][j] = u + v;
+            x[q][k] = u + f.p2 - v;
+        }
     };
     if constexpr (P::R > 0) {
 #pragma unroll
-        for (int j = 0; j < 8; j += 2) {  // twiddle 1; inputs in [0, 2p)
-            const uint32_t u = x[j], v = x[j + 1];
-            x[j] = u + v;
-            x[j + 1] = u + f.p2 - v;
-        }
+        for (int q = 0; q < NA; ++q)
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) {  // twiddle 1; inputs in [0, 2p)
+                const uint32_t u = x[q][j], v = x[q][j + 1];
+                x[q][j] = u + v;
+                x[q][j + 1] = u + f.p2 - v;
+            }
         if constexpr (P::R == 2) {
             const uint2 w1 = __ldg(itw + TwLayout::quarter(LG));
 #pragma unroll
-            for (int j = 0; j < 8; j += 4) {
-                const uint32_t u0 = f.reduce2(x[j]), v0 = f.reduce2(x[j + 2]);
-                const uint32_t u1 = f.reduce2(x[j + 1]), v1 = f.shoup(x[j + 3], w1);
-                x[j] = u0 + v0;
-                x[j + 2] = u0 + f.p2 - v0;
-                x[j + 1] = u1 + v1;
-                x[j + 3] = u1 + f.p2 - v1;
-            }
+            for (int q = 0; q < NA; ++q)
+#pragma unroll
+                for (int j = 0; j < 8; j += 4) {
+                    const uint32_t u0 = f.reduce2(x[q][j]), v0 = f.reduce2(x[q][j + 2]);
+                    const uint32_t u1 = f.reduce2(x[q][j + 1]), v1 = f.shoup(x[q][j + 3], w1);
+                    x[q][j] = u0 + v0;
+                    x[q][j + 2] = u0 + f.p2 - v0;
+                    x[q][j + 1] = u1 + v1;
+                    x[q][j + 3] = u1 + f.p2 - v1;
+                }
         }
-        exchange<LG, 1>(xs, sh, 1, P::d(P::NF - 1));
+        exchange<LG, NA>(x, sh, 1, P::d(P::NF - 1));
     }
 #pragma unroll
     for (int k = P::NF - 1; k >= 0; --k) {
@@ -305,10 +313,18 @@ __device__ __forceinline__ void inverse(uint32_t (&x)[8], uint32_t* sh, const ui
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) bf(j, j + 4, e0 + d * j);
-        if (k > 0) exchange<LG, 1>(xs, sh, d, P::d(k - 1));
+        if (k > 0) exchange<LG, NA>(x, sh, d, P::d(k - 1));
     }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) x[j] = f.reduce2(x[j]);
+    for (int q = 0; q < NA; ++q)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[q][j] = f.reduce2(x[q][j]);
+}
+
+template <int LG>
+__device__ __forceinline__ void inverse(uint32_t (&x)[8], uint32_t* sh, const uint2* __restrict__ itw_all,
+                                        const Field& f) {
+    inverse<LG, 1>(reinterpret_cast<uint32_t(&)[1][8]>(x), sh, itw_all, f);
 }
 
 }  // namespace ntt32

@@ -107,3 +107,16 @@ def test_poly_rejects_bad_arguments(ctx):
     with pytest.raises(midint.MidintError):
         ctx.poly(16, 16, 16 + 8, 1, 2049)
     ctx.poly(16, 16, 4096, 0, 4)  # empty batch: nothing launched
+
+
+@pytest.mark.parametrize("n,m", [(1900, 130), (1900, 190), (950, 260), (950, 380), (470, 520), (470, 760)])
+def test_poly_ntt_several_instances_per_block(ctx, devmem, n, m):
+    # more instances than resident blocks at 512, 1024 and 2048 points, both
+    # digit modes: a block's shared-memory pieces are reused from one to the next
+    old = ctx.get_tuning(midint.TUNE_POLY_NTT_MIN)
+    ctx.set_tuning(midint.TUNE_POLY_NTT_MIN, 0, 1)
+    try:
+        a, b = carry_stress(n, m, seed=m)
+        assert np.array_equal(gpu_poly(ctx, devmem, a, b, m), O.poly(a, b, m))
+    finally:
+        ctx.set_tuning(midint.TUNE_POLY_NTT_MIN, 0, old)

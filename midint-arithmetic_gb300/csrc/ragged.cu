@@ -301,6 +301,16 @@ __device__ __forceinline__ Task decode_tab(const FamTab& tab, uint32_t t) {
     return T;
 }
 
+// At the end of a task kernel: the grid completes only after the task kernel
+// launched before it.  One block waits for that; the others leave their SM to
+// the kernels that follow (when every block waited, the blocks of a family
+// with few tasks held their registers until the previous family was done, and
+// the families of a short list ran one after another: 400 operations of 512 to
+// 32768 bits 87 us against RAGFIG).
+__device__ __forceinline__ void pdl_join() {
+    if (blockIdx.x == 0) pdl_wait();
+}
+
 // --- NTT family ----------------------------------------------------------------
 
 template <int LG, int DM>
@@ -353,7 +363,7 @@ __global__ void __launch_bounds__(256, DM == ntt32::DM64 ? 3 : 2) k_rg_ntt(Param
         }
         __syncthreads();  // the next index is visible; this one is read by all
     }
-    if (DM != ntt32::DM64) pdl_wait();  // complete only after the task kernel launched before it
+    if (DM != ntt32::DM64) pdl_join();
 }
 
 // --- classical family ----------------------------------------------------------
@@ -803,7 +813,7 @@ __global__ void __launch_bounds__(256, 2) k_rg_classic(Params P) {
         }
         __syncwarp();
     }
-    pdl_wait();  // complete only after the task kernel launched before it
+    pdl_join();
 }
 
 // 32-thread products over rounds (shorter operand of 17..128 limbs below the
@@ -829,7 +839,7 @@ __global__ void __launch_bounds__(256, 2) k_rg_r32(Params P) {
         if (lane == 0) next = atomicAdd(P.scr + Scratch::QUEUE + 7, 1u);
         rect32_task(P, decode_tab<7>(tab, t), wsm);
     }
-    pdl_wait();  // complete only after the task kernel launched before it
+    pdl_join();
 }
 
 // Comb products (shorter operand of at most 8 limbs): a family and a kernel
@@ -856,7 +866,7 @@ __global__ void __launch_bounds__(256, 2) k_rg_comb(Params P) {
         else comb_task<32>(P, tk);
         __syncwarp();
     }
-    pdl_wait();  // complete only after the task kernel launched before it
+    pdl_join();
 }
 
 // Products whose shorter operand has 129..256 limbs (below the NTT crossover):
@@ -878,7 +888,7 @@ __global__ void __launch_bounds__(256, 2) k_rg_c64(Params P) {
         classic_task<64>(P, decode_tab<3>(tab, t), smem32, scr_warp);
         __syncthreads();  // the next index is visible; shared memory is reused
     }
-    pdl_wait();  // complete only after the task kernel launched before it
+    pdl_join();
 }
 
 // --- addition family -------------------------------------------------------------
@@ -1016,7 +1026,7 @@ __global__ void __launch_bounds__(256, 3) k_rg_add(Params P) {
         }
         __syncwarp();
     }
-    pdl_wait();  // complete only after the task kernel launched before it
+    pdl_join();
 }
 
 // --- host side -------------------------------------------------------------------

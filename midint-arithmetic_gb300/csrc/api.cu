@@ -67,6 +67,21 @@ mi_status ensure_dyn_smem(const void* kern, size_t bytes) {
     return MI_OK;
 }
 
+mi_status ResidentBlocks::lookup(const void* kern, int threads, size_t smem, int* blocks_per_sm) {
+    int dev = 0;
+    MI_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return set_error(MI_ENODEV, "device index %d out of range", dev);
+    int v = cached_[dev].load(std::memory_order_acquire);
+    if (v == 0) {
+        MI_TRY(ensure_dyn_smem(kern, smem));
+        MI_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kern, threads, smem));
+        if (v < 1) v = 1;
+        cached_[dev].store(v, std::memory_order_release);
+    }
+    *blocks_per_sm = v;
+    return MI_OK;
+}
+
 }  // namespace mi
 
 using namespace mi;

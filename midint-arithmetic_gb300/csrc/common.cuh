@@ -10,6 +10,7 @@
 
 #include <cstdint>
 #include <cstddef>
+#include <atomic>
 #include <cuda_runtime.h>
 
 #include "../../include/midint.h"
@@ -48,6 +49,22 @@ template <typename K>
 inline mi_status ensure_dyn_smem(K* kern, size_t bytes) {
     return ensure_dyn_smem(reinterpret_cast<const void*>(kern), bytes);
 }
+
+// Resident blocks per SM of one kernel at one block size and shared-memory
+// request, looked up once per device (the query costs about a microsecond and
+// a half of every call's launch path); also raises the kernel's
+// shared-memory limit.  One static instance per launch site.
+class ResidentBlocks {
+  public:
+    template <typename K>
+    mi_status get(K* kern, int threads, size_t smem, int* blocks_per_sm) {
+        return lookup(reinterpret_cast<const void*>(kern), threads, smem, blocks_per_sm);
+    }
+
+  private:
+    mi_status lookup(const void* kern, int threads, size_t smem, int* blocks_per_sm);
+    std::atomic<int> cached_[64] = {};
+};
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 inline bool aligned8(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7u) == 0; }
@@ -92,6 +109,51 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
+// Thread-block clusters: the block's rank, the cluster barrier in its two
+// halves (arrive releases, wait acquires; every thread of every block of the
+// cluster takes part), and a store to the same shared-memory word of another
+// block of the cluster.
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_arrive() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint32_t cluster_addr(const void* shared, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                 : "=r"(a)
+                 : "r"(uint32_t(__cvta_generic_to_shared(shared))), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void cluster_store(uint32_t addr, uint32_t v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+
+// launch_pdl in clusters of `cluster` blocks (at most 8).
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_cluster(void (*kern)(KArgs...), uint32_t cluster, dim3 grid, dim3 block, size_t smem,
+                                  cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 

@@ -52,26 +52,83 @@ __global__ void __launch_bounds__((1 << LG) / 8, 768 / ((1 << LG) / 8))
               uint32_t m, uint32_t rlen, NttMulParams P) {
     extern __shared__ __align__(16) uint32_t smem32[];
     uint32_t* scratch = smem32 + ntt32::MulSmem<LG>::WORDS32;
+    pdl_wait();  // small batches are launched with launch_pdl
+    pdl_trigger();
     for (uint64_t inst = blockIdx.x; inst < n; inst += gridDim.x)
         ntt32::mul_one<LG, 5 - NP, true, LOW>(a + inst * m, m, b + inst * m, m, r + inst * rlen, rlen, P, smem32,
                                               scratch);  // L = pow2ceil(2m): both operands in the lower half
 }
 
+// Small batches: one cluster of NP blocks per instance, block q running the
+// transforms of prime q; the residues of all of them are stored into block 0's
+// shared memory (each word once, across the cluster's SMs), and block 0
+// recombines the product.
+template <int LG, int NP, bool LOW>
+__global__ void __launch_bounds__((1 << LG) / 8)
+    k_ntt_mul_cluster(const uint64_t* __restrict__ a, const uint64_t* __restrict__ b, uint64_t* __restrict__ r,
+                      uint32_t n, uint32_t m, uint32_t rlen, NttMulParams P) {
+    using Pl = ntt32::Plan<LG>;
+    extern __shared__ __align__(16) uint32_t smem32[];
+    uint32_t* sh = smem32;
+    uint32_t* res = smem32 + 2 * Pl::LX;
+    uint32_t* scratch = smem32 + ntt32::MulSmem<LG>::WORDS32;
+    const uint32_t q = cluster_rank(), t = threadIdx.x;
+    const uint64_t inst = blockIdx.x / NP;  // the grid has exactly n clusters
+    const uint32_t to = cluster_addr(res + q * Pl::L, 0);
+    cluster_arrive();  // this block has started
+    pdl_wait();
+    pdl_trigger();
+    uint32_t x[8];
+    ntt32::mul_residues<LG, 5 - NP, true>(a + inst * m, m, b + inst * m, m, P, int(q), sh, x);
+    cluster_wait();  // block 0 has started: its shared memory may be written
+#pragma unroll
+    for (int j = 0; j < (LOW ? 4 : 8); ++j) cluster_store(to + 4 * ntt32::swz(t + Pl::NT * j), x[j]);
+    cluster_arrive();
+    cluster_wait();  // every residue is in block 0
+    if (q == 0)
+        ntt32::mul_recombine<LG, 5 - NP, LOW>(res, r + inst * rlen, rlen, P, reinterpret_cast<uint64_t*>(sh), scratch);
+}
+
+// The cluster form while its n NP blocks fit a few per SM (by transform
+// length; 4096-point blocks are one per SM by their shared memory): the latency
+// of an instance is then that of one prime, not of NP in turn.  Products of m
+// limbs against a block each: m = 1024, n = 20 18.4 -> 6.8 us, n = 75 18.5 ->
+// 14.3; m = 2048, n = 20 32.8 -> 11.6; m = 256, n = 60 12.3 -> 5.6.  Beyond
+// it the blocks of a cluster wait for one another and for a place (m = 1024,
+// n = 152 22.8 us against 16.5; n = 1024 140 against 89; m = 400, n = 152
+// 13.2 against 11.2; m = 256, n = 300 11.4 against 10.4).
+constexpr uint32_t cluster_blocks_per_sm(int lg) { return lg == 8 ? 16 : lg == 9 ? 7 : lg <= 11 ? 3 : 2; }
+
 template <int LG, int NP>
 mi_status launch_lg(const uint64_t* a, const uint64_t* b, uint64_t* r, uint32_t n, uint32_t m, uint32_t rlen,
                     const NttMulParams& P, cudaStream_t st) {
     using S = NttShape<LG>;
-    auto kern = rlen <= m ? k_ntt_mul<LG, NP, true> : k_ntt_mul<LG, NP, false>;  // the low half alone
-    MI_TRY(ensure_dyn_smem(kern, S::SMEM));
+    const bool low = rlen <= m;  // the low half alone
+    if (uint64_t(n) * NP < uint64_t(sm_count()) * cluster_blocks_per_sm(LG)) {
+        auto kern = low ? k_ntt_mul_cluster<LG, NP, true> : k_ntt_mul_cluster<LG, NP, false>;
+        static ResidentBlocks site[2];
+        int per_sm = 0;
+        MI_TRY(site[low].get(kern, S::NT, S::SMEM, &per_sm));
+        MI_CUDA_TRY(launch_cluster(kern, NP, dim3(n * NP), dim3(S::NT), S::SMEM, st, a, b, r, n, m, rlen, P));
+        return MI_OK;
+    }
+    auto kern = low ? k_ntt_mul<LG, NP, true> : k_ntt_mul<LG, NP, false>;
+    static ResidentBlocks site[2];
     int per_sm = 0;
-    MI_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, S::NT, S::SMEM));
-    uint64_t blocks = uint64_t(sm_count()) * (per_sm > 0 ? per_sm : 1);
+    MI_TRY(site[low].get(kern, S::NT, S::SMEM, &per_sm));
+    uint64_t blocks = uint64_t(sm_count()) * uint64_t(per_sm);
     if (blocks > n) blocks = n;
-    // A plain launch: the grid is persistent with a fixed stride over the
-    // instances, and a programmatic dependent launch, whose blocks become
-    // resident one by one during the previous launch's tail, put the blocks
-    // with one instance more on the same SMs (measured 0.108 ms against
-    // 0.0996 ms per 1024 x 65536-bit batch).
+    // Up to two instances per SM, a programmatic dependent launch (m = 1024,
+    // n = 152 18.5 -> 16.5 us, n = 304 28.7 -> 27.3).  Above that a plain one:
+    // the blocks of a dependent launch become resident one by one during the
+    // previous launch's tail and pile up on some SMs (m = 512, n = 600 40.9 us
+    // against 26.8), and with a fixed stride over the instances those with one
+    // instance more end up on the same ones (1024 of m = 1024 108 us against
+    // 99.6).
+    if (n <= 2 * uint32_t(sm_count())) {
+        MI_CUDA_TRY(launch_pdl(kern, dim3(uint32_t(blocks)), dim3(S::NT), S::SMEM, st, a, b, r, n, m, rlen, P));
+        return MI_OK;
+    }
     kern<<<dim3(uint32_t(blocks)), dim3(S::NT), S::SMEM, st>>>(a, b, r, n, m, rlen, P);
     MI_CUDA_TRY(cudaGetLastError());
     return MI_OK;

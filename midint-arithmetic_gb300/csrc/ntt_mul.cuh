@@ -167,65 +167,58 @@ __device__ __forceinline__ void finish_block(const uint64_t (&s)[SW], uint64_t* 
     }
 }
 
-// r[0..rlen) = a*b for a of la limbs, b of lb limbs, with ntt_digits(la) +
-// ntt_digits(lb) <= L in digit mode DM (and, for DM40, the shorter operand
-// within kD40MaxDigits digits); every output limb, including the carry out of
-// the top coefficient, falls inside the OUT*L/8 limbs the group produces;
-// limbs beyond rlen are dropped.  `sm` is the group's MulSmem, `scr` per-warp
-// scratch of the block.  Every thread of the block must call this with the
-// same LG and DM (the exchanges synchronise the block).  HALF: both operands'
-// digits lie below L/2 (balanced products: L = pow2ceil(2m)), so the upper
-// half of each transform input is zero and is neither converted nor added
-// (a compile-time choice: as a run-time flag in the ragged tasks it cost more
-// than it saved).  LOW: only the low half of a balanced product is stored
-// (rlen at most m limbs, all of them below digit L/2); the coefficients below
-// L/2 alone determine those limbs, so only they are kept and recombined.
-template <int LG, int DM, bool HALF = false, bool LOW = false>
-__device__ __forceinline__ void mul_one(const uint64_t* __restrict__ ar, uint32_t la, const uint64_t* __restrict__ br,
-                                        uint32_t lb, uint64_t* __restrict__ rr, uint32_t rlen, const NttMulParams& P,
-                                        uint32_t* sm, uint32_t* scr) {
+// The residues mod prime q of the thread's coefficients t + L/8 j (j < 8) of
+// the product a*b (arguments as in mul_one); `sh` are the group's exchange
+// buffers.
+template <int LG, int DM, bool HALF>
+__device__ __forceinline__ void mul_residues(const uint64_t* __restrict__ ar, uint32_t la,
+                                             const uint64_t* __restrict__ br, uint32_t lb, const NttMulParams& P, int q,
+                                             uint32_t* sh, uint32_t (&out)[8]) {
+    using Pl = Plan<LG>;
+    const uint32_t t = threadIdx.x % Pl::NT;
+    const Field f{P.p[q], 2 * P.p[q], P.pinv[q]};
+    // a unscaled; b times 2^32 / L (the Montgomery pointwise product takes
+    // out 2^32, and the inverse transform needs no 1/L pass)
+    const uint2 c32 = P.kb[q][0];
+    const uint2 kb0 = P.ka_by_lg[q][LG - 8][1], kb1 = P.kb_by_lg[q][LG - 8];
+    uint32_t x[2][8];  // a and b, transformed in lockstep
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const uint32_t i = t + Pl::NT * j;
+        if (HALF && j >= 4) {
+            x[0][j] = x[1][j] = 0u;
+            continue;
+        }
+        if constexpr (DM == DM64) {
+            const uint64_t da = i < la ? __ldg(ar + i) : 0ull;
+            x[0][j] = reduce_digit(uint32_t(da), uint32_t(da >> 32), f, c32);
+            x[1][j] = (i < lb) ? convert(__ldg(br + i), f, kb0, kb1) : 0u;
+        } else {
+            const uint2 da = digit_at<DM>(ar, la, i);
+            const uint2 db = digit_at<DM>(br, lb, i);
+            x[0][j] = reduce_digit(da.x, da.y, f, c32);
+            x[1][j] = f.add(f.shoup(db.x, kb0), f.shoup(db.y, kb1));
+        }
+    }
+    forward<LG, 2, HALF>(x, sh, P.tw[q], f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[0][j] = f.mont(x[0][j], x[1][j]);
+    inverse<LG>(x[0], sh, P.itw[q], f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) out[j] = f.reduce(x[0][j]);
+}
+
+// The product's limbs r[0..rlen) from the residues of all its coefficients
+// (res[q L + swz(i)], visible to the group): Garner, digit sums, carries.
+// `ov` is scratch of 3 x 8 bytes per thread, free by the call.
+template <int LG, int DM, bool LOW>
+__device__ __forceinline__ void mul_recombine(const uint32_t* res, uint64_t* __restrict__ rr, uint32_t rlen,
+                                              const NttMulParams& P, uint64_t* ov, uint32_t* scr) {
     using Pl = Plan<LG>;
     using Dg = Digits<DM>;
     constexpr int NP = Dg::NP;
     constexpr int SW = 11;  // digit-sum words: 8 limbs + 3 overflow, 6 + 2 or 5 + 1 (+ headroom)
-    uint32_t* sh = sm;                // exchange buffers of a and b (2 LX)
-    uint32_t* res = sm + 2 * Pl::LX;  // res[q][slot], q < NP
     const uint32_t t = threadIdx.x % Pl::NT;
-#pragma unroll 1
-    for (int q = 0; q < NP; ++q) {
-        const Field f{P.p[q], 2 * P.p[q], P.pinv[q]};
-        // a unscaled; b times 2^32 / L (the Montgomery pointwise product takes
-        // out 2^32, and the inverse transform needs no 1/L pass)
-        const uint2 c32 = P.kb[q][0];
-        const uint2 kb0 = P.ka_by_lg[q][LG - 8][1], kb1 = P.kb_by_lg[q][LG - 8];
-        uint32_t x[2][8];  // a and b, transformed in lockstep
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const uint32_t i = t + Pl::NT * j;
-            if (HALF && j >= 4) {
-                x[0][j] = x[1][j] = 0u;
-                continue;
-            }
-            if constexpr (DM == DM64) {
-                const uint64_t da = i < la ? __ldg(ar + i) : 0ull;
-                x[0][j] = reduce_digit(uint32_t(da), uint32_t(da >> 32), f, c32);
-                x[1][j] = (i < lb) ? convert(__ldg(br + i), f, kb0, kb1) : 0u;
-            } else {
-                const uint2 da = digit_at<DM>(ar, la, i);
-                const uint2 db = digit_at<DM>(br, lb, i);
-                x[0][j] = reduce_digit(da.x, da.y, f, c32);
-                x[1][j] = f.add(f.shoup(db.x, kb0), f.shoup(db.y, kb1));
-            }
-        }
-        forward<LG, 2, HALF>(x, sh, P.tw[q], f);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) x[0][j] = f.mont(x[0][j], x[1][j]);
-        inverse<LG>(x[0], sh, P.itw[q], f);
-#pragma unroll
-        for (int j = 0; j < (LOW ? 4 : 8); ++j) res[q * Pl::L + swz(t + Pl::NT * j)] = f.reduce(x[0][j]);
-    }
-    __syncthreads();
-
     // Garner: y0 = r0, y_i = (...((r_i - y0) c_0i - y1) c_1i ... - y_(i-1)) c_(i-1)i
     // mod p_i with c_ji = p_j^-1 mod p_i; x = y0 + p0 (y1 + p1 (y2 + ...)),
     // below the product of the NP primes (2^150, 2^120 or 2^90), evaluated in
@@ -279,9 +272,41 @@ __device__ __forceinline__ void mul_one(const uint64_t* __restrict__ ar, uint32_
             }
         }
     }
-    // the overflow words go to the right neighbour through the exchange buffer
-    uint64_t* ov = reinterpret_cast<uint64_t*>(sh);  // 3 x 8 bytes x L/8 threads: fits the 9L bytes of sh
+    // the overflow words go to the right neighbour through ov
     finish_block<Pl::NT, Dg::OUT, Dg::OVW>(s, ov, rr, rlen, t, scr);
+}
+
+// r[0..rlen) = a*b for a of la limbs, b of lb limbs, with ntt_digits(la) +
+// ntt_digits(lb) <= L in digit mode DM (and, for DM40, the shorter operand
+// within kD40MaxDigits digits); every output limb, including the carry out of
+// the top coefficient, falls inside the OUT*L/8 limbs the group produces;
+// limbs beyond rlen are dropped.  `sm` is the group's MulSmem, `scr` per-warp
+// scratch of the block.  Every thread of the block must call this with the
+// same LG and DM (the exchanges synchronise the block).  HALF: both operands'
+// digits lie below L/2 (balanced products: L = pow2ceil(2m)), so the upper
+// half of each transform input is zero and is neither converted nor added
+// (a compile-time choice: as a run-time flag in the ragged tasks it cost more
+// than it saved).  LOW: only the low half of a balanced product is stored
+// (rlen at most m limbs, all of them below digit L/2); the coefficients below
+// L/2 alone determine those limbs, so only they are kept and recombined.
+template <int LG, int DM, bool HALF = false, bool LOW = false>
+__device__ __forceinline__ void mul_one(const uint64_t* __restrict__ ar, uint32_t la, const uint64_t* __restrict__ br,
+                                        uint32_t lb, uint64_t* __restrict__ rr, uint32_t rlen, const NttMulParams& P,
+                                        uint32_t* sm, uint32_t* scr) {
+    using Pl = Plan<LG>;
+    uint32_t* sh = sm;                // exchange buffers of a and b (2 LX)
+    uint32_t* res = sm + 2 * Pl::LX;  // res[q][slot], q < NP
+    const uint32_t t = threadIdx.x % Pl::NT;
+#pragma unroll 1
+    for (int q = 0; q < Digits<DM>::NP; ++q) {
+        uint32_t x[8];
+        mul_residues<LG, DM, HALF>(ar, la, br, lb, P, q, sh, x);
+#pragma unroll
+        for (int j = 0; j < (LOW ? 4 : 8); ++j) res[q * Pl::L + swz(t + Pl::NT * j)] = x[j];
+    }
+    __syncthreads();
+    // the overflow words take the exchange buffers: 3 x 8 bytes x L/8 threads fit their 9L bytes
+    mul_recombine<LG, DM, LOW>(res, rr, rlen, P, reinterpret_cast<uint64_t*>(sh), scr);
     __syncthreads();  // sh and res are reused by the next call
 }
 

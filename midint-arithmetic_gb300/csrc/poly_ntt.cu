@@ -283,10 +283,10 @@ mi_status launch_lg(const uint64_t* a, const uint64_t* b, uint64_t* r, uint32_t 
     constexpr int NT = (1 << LG) / 8;
     const size_t smem = PolySmem<LG, D48>::WORDS32 * 4 + size_t(NT / 32 + 1) * 4;
     auto kern = k_poly_ntt<LG, D48>;
-    MI_TRY(ensure_dyn_smem(kern, smem));
+    static ResidentBlocks site;
     int per_sm = 0;
-    MI_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem));
-    uint64_t blocks = uint64_t(sm_count()) * (per_sm > 0 ? per_sm : 1);
+    MI_TRY(site.get(kern, NT, smem, &per_sm));
+    uint64_t blocks = uint64_t(sm_count()) * uint64_t(per_sm);
     if (blocks > n) blocks = n;
     kern<<<dim3(uint32_t(blocks)), dim3(NT), smem, st>>>(a, b, r, n, m, P);
     MI_CUDA_TRY(cudaGetLastError());

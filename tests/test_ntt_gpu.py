@@ -210,3 +210,34 @@ def test_size_dispatch_on_misaligned_rows_matches_oracle(ctx, devmem, m):
     ctx.mul_lo(pa, pb, pr2, 3, m, stream=_stream())
     torch.cuda.synchronize()
     assert np.array_equal(devmem.get(br2, 2 * a.size, 1), O.mul(a, b, m, False))
+
+
+@pytest.mark.parametrize("low", [False, True])
+@pytest.mark.parametrize("m", [70, 90, 128, 140, 190, 256, 320, 380, 512, 520, 700, 1024, 1040, 1400, 2048])
+def test_mul_ntt_batch_sizes(ctx, devmem, m, low):
+    # every transform length and digit mode with one product, batches on either
+    # side of the cluster form's limit (3 to 5 blocks per product against 2 to
+    # 16 blocks per SM), of two products per SM, and a partial wave of blocks
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    lg = max(8, (2 * m - 1).bit_length())
+    per_sm = {8: 16, 9: 7, 10: 3, 11: 3, 12: 2}[lg]
+    ns = {1, 2 * sms, 2 * sms + 1} if m <= 1024 else {1}
+    ns |= {(sms * per_sm - 1) // np_ + d for np_ in (3, 4, 5) for d in (0, 1)}
+    old = ctx.get_tuning(midint.TUNE_LO_NTT_MIN)
+    ctx.set_tuning(midint.TUNE_LO_NTT_MIN, 0, 1)
+    try:
+        big = max(ns)
+        a, b = carry_stress(big, m, seed=m)
+        want = O.mul(a, b, m, full=not low)
+        _, pa = keep_a = devmem.put(a)
+        _, pb = keep_b = devmem.put(b)
+        row = m if low else 2 * m
+        for n in sorted(ns):
+            br, pr = devmem.empty_words(2 * row * n)
+            (ctx.mul_lo if low else ctx.mul_ntt)(pa, pb, pr, n, m, stream=_stream())
+            torch.cuda.synchronize()
+            assert np.array_equal(devmem.get(br, 2 * row * n), want[:n * row]), n
+            assert (br[2 * row * n:].cpu().numpy() == -1).all(), "result written past the batch"
+        del keep_a, keep_b
+    finally:
+        ctx.set_tuning(midint.TUNE_LO_NTT_MIN, 0, old)

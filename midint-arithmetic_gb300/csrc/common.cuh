@@ -114,8 +114,8 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
 
 // Thread-block clusters: the block's rank, the cluster barrier in its two
 // halves (arrive releases, wait acquires; every thread of every block of the
-// cluster takes part), and a store to the same shared-memory word of another
-// block of the cluster.
+// cluster takes part), and loads and stores of another block's shared memory
+// at the address that it has in this one.
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -134,6 +134,11 @@ __device__ __forceinline__ uint32_t cluster_addr(const void* shared, uint32_t ra
 }
 __device__ __forceinline__ void cluster_store(uint32_t addr, uint32_t v) {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_load(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
 }
 
 // launch_pdl in clusters of `cluster` blocks (at most 8).

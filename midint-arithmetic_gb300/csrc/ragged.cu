@@ -10,6 +10,7 @@
 //     family, with the keys of each family in descending cost order;
 //  3. scatter: op indices grouped by key (each block reserves its slots of a
 //     key with one atomic);
+//     (lists of up to kBinMaxOps ops: the three in one launch of one cluster)
 //  4. one persistent kernel per family, each popping tasks from its atomic
 //     queue, chained so that each kernel's blocks start on the SMs the
 //     previous kernel's last tasks leave idle (ragged_launch):
@@ -161,7 +162,7 @@ __host__ __device__ __forceinline__ uint32_t ops_per_task(uint32_t key) {
 // kBinRange ops and count their keys in shared memory, so the global counters
 // take one atomic per (block, key) instead of one per op.
 constexpr uint32_t kBinRange = 1024;
-static_assert(K <= 256, "one shared counter per thread");
+static_assert(K < 255, "one shared counter per thread, and a byte per key");
 
 __global__ void __launch_bounds__(256) k_classify(const mi_op* __restrict__ ops, uint32_t n,
                                                   uint32_t* __restrict__ scr, uint32_t ntt_min, uint32_t ntt40_min) {
@@ -191,17 +192,22 @@ static_assert(fam_base(1) - fam_base(0) <= 32 && fam_base(2) - fam_base(1) <= 32
                   fam_base(7) - fam_base(6) <= 32 && fam_base(8) - fam_base(7) <= 32,
               "a family's keys fit one warp");
 
-// One warp per family scans its keys in c_order (shuffle scans): op offsets
-// by key (global over the families), task starts by order position with one
-// sentinel per family, task counts; the queues restart at 0.
-__global__ void __launch_bounds__(32 * NFAM) k_scan(uint32_t* __restrict__ scr) {
+// One warp per family scans its keys in c_order (shuffle scans) from the
+// counts by key: op offsets by key (global over the families), task starts by
+// order position with one sentinel per family, task counts; the queues
+// restart at 0.  Called by NFAM whole warps of a block (and its other threads,
+// which only take part in the barrier); opoff is the offsets' destination,
+// write says whether this block stores the rest into the scratch.
+__device__ __forceinline__ void scan_families(const uint32_t* counts, uint32_t* opoff, uint32_t* __restrict__ scr,
+                                              bool write) {
     __shared__ uint32_t fam_ops[NFAM];
     const int f = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int base = fam_base(f), nk = fam_base(f + 1) - base;
+    const bool mine = f < NFAM;
+    const int base = fam_base(mine ? f : 0), nk = mine ? fam_base(f + 1) - base : 0;
     uint32_t key = 0, c = 0, tk = 0;
     if (lane < nk) {
         key = c_order[base + lane];
-        c = scr[Scratch::COUNTS + key];
+        c = counts[key];
         const uint32_t opt = ops_per_task(key);
         tk = (c + opt - 1) / opt;
     }
@@ -214,19 +220,83 @@ __global__ void __launch_bounds__(32 * NFAM) k_scan(uint32_t* __restrict__ scr) 
             ti += v;
         }
     }
-    if (lane == 31) fam_ops[f] = ci;
+    if (mine && lane == 31) fam_ops[f] = ci;
     __syncthreads();
+    if (!mine) return;
     uint32_t before = 0;
     for (int g = 0; g < f; ++g) before += fam_ops[g];
     if (lane < nk) {
-        scr[Scratch::OPOFF + key] = before + ci - c;
-        scr[Scratch::TS + f + base + lane] = ti - tk;
+        opoff[key] = before + ci - c;
+        if (write) scr[Scratch::TS + f + base + lane] = ti - tk;
     }
-    if (lane == 31) {
+    if (lane == 31 && write) {
         scr[Scratch::TS + f + base + nk] = ti;  // sentinel
         scr[Scratch::NTASKS + f] = ti;
         scr[Scratch::QUEUE + f] = 0;
     }
+}
+
+__global__ void __launch_bounds__(32 * NFAM) k_scan(uint32_t* __restrict__ scr) {
+    scan_families(scr + Scratch::COUNTS, scr + Scratch::OPOFF, scr, true);
+}
+
+// The whole binning of a shorter list in one launch of one cluster: each block
+// classifies a contiguous range of the ops (a byte of shared memory per op
+// keeps its key), the blocks read each other's counts across the cluster, every
+// block scans the totals, and each scatters its range.  It writes every word of
+// the scratch that the task kernels read, so nothing is cleared before.  One
+// block up to kBinOne ops, which it classifies one per thread, kBinBlocks
+// beyond; eight SMs classify some 5 ops per ns, so that up to kBinMaxOps this
+// costs less than a clear and three launches over all of them (14 us: lists of
+// 400 operations of 512 to 32768 bits 53 -> 41 us, 400 of at most 4000 bits
+// 34.5 -> 22.3, 20000 143 -> 131; 200000 1465 -> 1481, which keep the three).
+constexpr uint32_t kBinBlocks = 8, kBinOne = 1024;
+constexpr uint32_t kBinMaxOps = 65536;
+
+__global__ void __launch_bounds__(1024) k_bin(const mi_op* __restrict__ ops, uint32_t n, uint32_t* __restrict__ scr,
+                                              uint32_t ntt_min, uint32_t ntt40_min) {
+    extern __shared__ uint8_t keys8[];  // this block's keys, 255 for an invalid op
+    __shared__ uint32_t hist[K + 1], total[K + 1], cursor[K];
+    const uint32_t t = threadIdx.x, rank = cluster_rank(), blocks = gridDim.x;  // the grid is one cluster
+    const uint32_t per = (n + blocks - 1) / blocks, lo = min(n, rank * per), cnt = min(n - lo, per);
+    if (t <= K) hist[t] = 0;
+    pdl_wait();  // launched with launch_cluster
+    pdl_trigger();
+    __syncthreads();
+    for (uint32_t i = t; i < cnt; i += 1024) {
+        const uint32_t key = classify(ops[lo + i], ntt_min, ntt40_min);
+        keys8[i] = uint8_t(key);
+        atomicAdd(&hist[key == KEY_INVALID ? K : key], 1u);
+    }
+    __syncthreads();
+    cluster_arrive();
+    cluster_wait();
+    uint32_t before = 0;  // ops of key t in the blocks before this one
+    if (t <= K) {
+        uint32_t sum = 0;
+        for (uint32_t r = 0; r < blocks; ++r) {
+            const uint32_t c = cluster_load(cluster_addr(hist + t, r));
+            if (r < rank) before += c;
+            sum += c;
+        }
+        total[t] = sum;
+        if (rank == 0) scr[t < K ? Scratch::COUNTS + t : Scratch::INVALID] = sum;
+    }
+    cluster_arrive();  // the other blocks' counts have been read
+    __syncthreads();
+    scan_families(total, cursor, scr, rank == 0);
+    __syncthreads();
+    if (t < K) {
+        if (rank == 0) scr[Scratch::OPOFF + t] = cursor[t];
+        cursor[t] += before;
+    }
+    __syncthreads();
+    uint32_t* sorted = scr + Scratch::sorted(n);
+    for (uint32_t i = t; i < cnt; i += 1024) {
+        const uint32_t key = keys8[i];
+        if (key != 255u) sorted[atomicAdd(&cursor[key], 1u)] = lo + i;
+    }
+    cluster_wait();  // this block's counts have been read: it may end
 }
 
 __global__ void __launch_bounds__(256) k_scatter(uint32_t n, uint32_t* __restrict__ scr) {
@@ -345,6 +415,7 @@ __global__ void __launch_bounds__(256, DM == ntt32::DM64 ? 3 : 2) k_rg_ntt(Param
     uint32_t* scr_warp = smem + ntt32::MulSmem<11>::WORDS32;  // after the groups' shared memory
     __shared__ uint32_t s_task[2];  // this task and the next, fetched while this one runs
     __shared__ FamTab tab;
+    if (DM == ntt32::DM64) pdl_wait();  // the first task kernel: the binning is complete
     const uint32_t ntasks = P.scr[Scratch::NTASKS + F];
     pdl_trigger();  // the next family's kernel may start as this one's blocks finish
     load_tab(tab, P.scr, F);
@@ -1070,11 +1141,15 @@ mi_status init_device() {
     return MI_OK;
 }
 
-int persistent_grid(const void* kern, size_t smem) {
+// Launches a task kernel as a programmatic dependent with as many 256-thread
+// blocks as are resident at once (no more than there are ops).
+template <typename Kern>
+mi_status launch_tasks(Kern* kern, ResidentBlocks& site, size_t smem, const Params& P, cudaStream_t st) {
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem) != cudaSuccess || per_sm < 1)
-        per_sm = 1;
-    return sm_count() * per_sm;
+    MI_TRY(site.get(kern, 256, smem, &per_sm));
+    const uint32_t grid = std::min(uint32_t(sm_count() * per_sm), P.n_ops);
+    MI_CUDA_TRY(launch_pdl(kern, dim3(grid), dim3(256), smem, st, P));
+    return MI_OK;
 }
 
 }  // namespace rg
@@ -1098,27 +1173,38 @@ mi_status ragged_launch(mi_ctx ctx, const mi_op* ops, uint32_t n_ops, const uint
     P.ntt_min = ntt_min < 1 ? 1 : (ntt_min > 257 ? 257 : ntt_min);
     P.ntt40_min = ctx->ragged_ntt40_min < 1 ? 1 : (ctx->ragged_ntt40_min > 257 ? 257 : ctx->ragged_ntt40_min);
     P.ntt = ctx->ntt.params;
-    MI_CUDA_TRY(cudaMemsetAsync(P.scr, 0, (Scratch::KEYS) * 4, st));
-    const uint32_t blocks = (n_ops + kBinRange - 1) / kBinRange;
-    k_classify<<<blocks, 256, 0, st>>>(ops, n_ops, P.scr, P.ntt_min, P.ntt40_min);
-    k_scan<<<1, 32 * NFAM, 0, st>>>(P.scr);  // the cursors were zeroed with the counts
-    k_scatter<<<blocks, 256, 0, st>>>(n_ops, P.scr);
-    // The task kernels: the first waits for the binning like any launch; each later one is a programmatic dependent launch that does not
-    // wait at its start -- the families read the binned lists and write
-    // disjoint results, so a kernel's blocks may start on the SMs that the
-    // previous kernel's last tasks leave idle -- and waits for its predecessor
-    // only before it completes, so that the last kernel completes after all.
-    k_rg_ntt<0><<<persistent_grid((const void*)k_rg_ntt<0>, kNttSmem), 256, kNttSmem, st>>>(P);
-    MI_CUDA_TRY(cudaGetLastError());
-    MI_CUDA_TRY(launch_pdl(k_rg_ntt<1>, persistent_grid((const void*)k_rg_ntt<1>, kNttSmem), 256, kNttSmem, st, P));
-    MI_CUDA_TRY(launch_pdl(k_rg_ntt<2>, persistent_grid((const void*)k_rg_ntt<2>, kNttSmem), 256, kNttSmem, st, P));
-    MI_CUDA_TRY(launch_pdl(k_rg_r32, persistent_grid((const void*)k_rg_r32, kR32Smem), 256, kR32Smem, st, P));
-    MI_CUDA_TRY(launch_pdl(k_rg_classic, persistent_grid((const void*)k_rg_classic, kClsSmem), 256, kClsSmem, st, P));
+    static ResidentBlocks sites[9];
+    if (n_ops <= kBinMaxOps) {
+        const uint32_t cluster = n_ops <= kBinOne ? 1u : kBinBlocks;
+        const size_t smem = (n_ops + cluster - 1) / cluster;
+        int per_sm = 0;
+        MI_TRY(sites[8].get(k_bin, 1024, kBinMaxOps / kBinBlocks, &per_sm));
+        MI_CUDA_TRY(launch_cluster(k_bin, cluster, dim3(cluster), dim3(1024), smem, st, ops, n_ops, P.scr, P.ntt_min,
+                                   P.ntt40_min));
+    } else {
+        MI_CUDA_TRY(cudaMemsetAsync(P.scr, 0, (Scratch::KEYS) * 4, st));
+        const uint32_t blocks = (n_ops + kBinRange - 1) / kBinRange;
+        k_classify<<<blocks, 256, 0, st>>>(ops, n_ops, P.scr, P.ntt_min, P.ntt40_min);
+        k_scan<<<1, 32 * NFAM, 0, st>>>(P.scr);  // the cursors were zeroed with the counts
+        k_scatter<<<blocks, 256, 0, st>>>(n_ops, P.scr);
+        MI_CUDA_TRY(cudaGetLastError());
+    }
+    // The task kernels, each a programmatic dependent launch.  The first waits
+    // for the binning at its start; the later ones start only once every block
+    // of it has done so, and do not wait there -- the families read the binned
+    // lists and write disjoint results, so a kernel's blocks may start on the
+    // SMs that the previous kernel's last tasks leave idle -- but one block of
+    // each waits for its predecessor before it completes, so that the last
+    // kernel completes after all.
+    MI_TRY(launch_tasks(k_rg_ntt<0>, sites[0], kNttSmem, P, st));
+    MI_TRY(launch_tasks(k_rg_ntt<1>, sites[1], kNttSmem, P, st));
+    MI_TRY(launch_tasks(k_rg_ntt<2>, sites[2], kNttSmem, P, st));
+    MI_TRY(launch_tasks(k_rg_r32, sites[3], kR32Smem, P, st));
+    MI_TRY(launch_tasks(k_rg_classic, sites[4], kClsSmem, P, st));
     // 64-thread classical groups serve shorter operands of 129..256 limbs below the crossover
-    if (P.ntt_min > 129)
-        MI_CUDA_TRY(launch_pdl(k_rg_c64, persistent_grid((const void*)k_rg_c64, kC64Smem), 256, kC64Smem, st, P));
-    MI_CUDA_TRY(launch_pdl(k_rg_comb, persistent_grid((const void*)k_rg_comb, 0), 256, 0, st, P));
-    MI_CUDA_TRY(launch_pdl(k_rg_add, persistent_grid((const void*)k_rg_add, 0), 256, 0, st, P));
+    if (P.ntt_min > 129) MI_TRY(launch_tasks(k_rg_c64, sites[5], kC64Smem, P, st));
+    MI_TRY(launch_tasks(k_rg_comb, sites[6], 0, P, st));
+    MI_TRY(launch_tasks(k_rg_add, sites[7], 0, P, st));
     return MI_OK;
 }
 

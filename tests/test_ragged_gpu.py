@@ -170,3 +170,26 @@ def test_ragged_full_workload_matches_plain_form(ctx):
     adds = ops["kind"] == 0
     assert np.array_equal(carry[adds], p_carry[adds])
     oracle_check(ops, pool, out, carry, sample=range(0, ops.size, 997))
+
+
+@pytest.mark.parametrize("n", [1, 31, 1023, 1024, 1025, 8191, 8193, 65536, 65537, 100003])
+def test_ragged_binning_sizes(ctx, n):
+    # one binning block, a cluster of eight with uneven ranges, its largest
+    # list and the three-launch form beyond: one-limb operations of 32-bit
+    # values (so a product fits one limb), every 7th of an unknown kind
+    kind = (np.arange(n) % 3 == 1).astype(np.uint32)
+    kind[::7] = 9
+    one = np.ones(n, np.uint32)
+    ops, pool, out_limbs = W.pack_ops(kind, one, one, n)
+    pool >>= np.uint64(32)
+    ones = np.flatnonzero(kind == 0)[::5]
+    pool[2 * ones] = np.uint64(2**64 - 1)     # these sums may carry out
+    a, b = pool[0::2], pool[1::2]
+    out, carry, invalid = run_ragged(ctx, ops, pool, out_limbs)
+    assert invalid == int((kind == 9).sum())
+    at = ops["r_off"].astype(np.int64)
+    add, mul = kind == 0, kind == 1
+    assert np.array_equal(out[at[add]], (a + b)[add])
+    assert np.array_equal(carry[add], ((a + b) < a)[add].astype(np.uint8))
+    assert np.array_equal(out[at[mul]], (a * b)[mul]) and not out[at[mul] + 1].any()
+    assert (out[at[kind == 9]] == np.uint64(2**64 - 1)).all()

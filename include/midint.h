@@ -117,7 +117,11 @@ mi_status mi_ctx_set_crossover(mi_ctx ctx, uint32_t ragged_ntt_min, uint32_t pla
  *                            the whole batch, as for the copies);
  *                            3: when the results are mapped pinned memory,
  *                            the operands are copied in by chunks and the
- *                            kernels write the results in place */
+ *                            kernels write the results in place.
+ *                            Modes 1 and 2 also use ordinary (pageable) memory
+ *                            in place where the GPU reaches it through the
+ *                            host's page tables, up to 32 MiB of buffers per
+ *                            call; otherwise such buffers are copied */
 enum {
     MI_TUNE_PLAIN_NTT_MIN = 0,
     MI_TUNE_RAGGED_NTT_MIN = 1,

@@ -15,6 +15,9 @@
 #include <mutex>
 #include <utility>
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include "common.cuh"
 #include "ctx.h"
 #include "kernels.h"
@@ -199,18 +202,54 @@ mi_status ensure_stage(mi_ctx ctx, size_t bytes) {
     return MI_OK;
 }
 
-// The device address of a mapped pinned host buffer that kernels may read or
-// write in place, or null.  Buffers that are not 8-byte aligned are not used
-// in place (the staging buffers of the copy path are): the u64 and NTT
-// kernels read whole 8-byte words.
-void* mapped_host(const void* p) {
+// How kernels can reach a host buffer in place.
+enum class HostKind { Copied, Mapped, Pageable };
+
+// The device address of a host buffer that kernels may read or write in
+// place, or null: a mapped pinned buffer (Mapped), or, where the GPU walks the
+// host's page tables (ctx->host_page_tables), any ordinary one (Pageable).
+// Buffers that are not 8-byte aligned are not used in place (the staging
+// buffers of the copy path are): the u64 and NTT kernels read whole 8-byte
+// words.
+void* host_in_place(mi_ctx ctx, const void* p, HostKind* kind) {
+    *kind = HostKind::Copied;
     if (!aligned8(p)) return nullptr;
     cudaPointerAttributes attr;
     if (cudaPointerGetAttributes(&attr, p) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
     }
-    return attr.type == cudaMemoryTypeHost ? attr.devicePointer : nullptr;
+    if (attr.type == cudaMemoryTypeHost) {
+        if (attr.devicePointer != nullptr) *kind = HostKind::Mapped;
+        return attr.devicePointer;
+    }
+    if (attr.type == cudaMemoryTypeUnregistered && ctx->host_page_tables) {
+        *kind = HostKind::Pageable;
+        return const_cast<void*>(p);
+    }
+    return nullptr;
+}
+void* mapped_host(mi_ctx ctx, const void* p) {
+    HostKind kind;
+    void* d = host_in_place(ctx, p, &kind);
+    return kind == HostKind::Mapped ? d : nullptr;
+}
+
+// Gives every page of an ordinary host buffer its place in host memory before
+// a kernel uses the buffer in place (pages that the program never wrote have
+// none yet, and would be placed by the GPU's own faults).  False where the
+// kernel cannot, for an address that the program may not use among others: the
+// caller then copies, as for any buffer.
+bool populate_pages(const void* p, size_t bytes, bool write) {
+#if defined(MADV_POPULATE_READ) && defined(MADV_POPULATE_WRITE)
+    static const uintptr_t page = uintptr_t(sysconf(_SC_PAGESIZE));
+    const uintptr_t lo = reinterpret_cast<uintptr_t>(p) / page * page;
+    const uintptr_t hi = (reinterpret_cast<uintptr_t>(p) + bytes + page - 1) / page * page;
+    return madvise(reinterpret_cast<void*>(lo), hi - lo, write ? MADV_POPULATE_WRITE : MADV_POPULATE_READ) == 0;
+#else
+    (void)p, (void)bytes, (void)write;
+    return false;
+#endif
 }
 
 // MI_ETIMEOUT (and the error word cleared) when a multi-block addition of the
@@ -229,8 +268,8 @@ mi_status wide_status(mi_ctx ctx) {
 // mapped pinned operands: the kernels read the operands in place and only the
 // results go through the staging slots and the copy-out stream (the two
 // directions of the host link then run at once).  Zero-copy mode 1 with
-// every buffer mapped pinned memory: one
-// launch reads and writes them in place.  Mode 3 with mapped pinned results:
+// every buffer mapped pinned memory (or ordinary memory that the GPU can
+// reach): one launch reads and writes them in place.  Mode 3 with mapped pinned results:
 // the operands go through the staging slots on the copy-in stream and the
 // kernels write the results in place (no copy-out).  Otherwise the batch is cut into
 // chunks that cycle through kSlots device staging slots: chunk c copies in on
@@ -247,32 +286,61 @@ mi_status host_pipeline(mi_ctx ctx, int cls, const void* h_a, const void* h_b, v
     if (n == 0) return MI_OK;
     MI_TRY(check_ctx(ctx));
     std::lock_guard<std::mutex> lk(ctx->mu);
-    // zero-copy reads of the operands (modes 1 and 2) when both are mapped
-    const char* za = nullptr;
-    const char* zb = nullptr;
     const uint32_t mode = ctx->host_zero_copy[cls];
+    // Every buffer in place: mode 1, and either mode where one of them is
+    // ordinary memory, which the copy engines move at a fraction of the link's
+    // rate (4096 low products of 64 limbs between ordinary arrays 174 us, in
+    // place 60; 512 of them 138 and 31; 12000 242 and 139; into a new array
+    // that was never written 1396 and 148).  Up to
+    // kPageableMax bytes in all: beyond, transforms, which read their
+    // operands once per prime (2000 products of 1000 limbs, 48 MB, 901 us
+    // against 547), and very many short rows (300000 of 16 limbs, 115 MB, 1395
+    // against 863) lose it again.  Additions wider than a block, whose waits
+    // are bounded, and calls whose result overlaps an operand use mapped
+    // pinned buffers only.
+    constexpr size_t kPageableMax = size_t(32) << 20;
     if (mode == 1 || mode == 2) {
-        za = static_cast<const char*>(mapped_host(h_a));
-        zb = static_cast<const char*>(mapped_host(h_b));
-        if (!za || !zb) za = zb = nullptr;
-    }
-    if (za && mode == 1) {
-        void* dr = mapped_host(h_r);
-        void* dc = h_carry ? mapped_host(h_carry) : nullptr;
-        if (dr && (dc || !h_carry)) {
-            MI_TRY(launch(const_cast<char*>(za), const_cast<char*>(zb), dr, static_cast<uint8_t*>(dc), n,
-                          ctx->pipe[2], ctx->host_zc_blocks[cls]));
+        HostKind kind[4] = {HostKind::Mapped, HostKind::Mapped, HostKind::Mapped, HostKind::Mapped};
+        void* d[4] = {host_in_place(ctx, h_a, &kind[0]), host_in_place(ctx, h_b, &kind[1]),
+                      host_in_place(ctx, h_r, &kind[2]), nullptr};
+        if (h_carry) d[3] = host_in_place(ctx, h_carry, &kind[3]);
+        const void* host[4] = {h_a, h_b, h_r, h_carry};
+        const size_t in = size_t(n) * in_row, out = size_t(n) * out_row, bytes[4] = {in, in, out, n};
+        bool go = true, pageable = false;
+        for (HostKind k : kind) {
+            go = go && k != HostKind::Copied;
+            pageable = pageable || k == HostKind::Pageable;
+        }
+        if (!pageable)
+            go = go && mode == 1;
+        else
+            go = go && !one_compute_stream && 2 * in + out <= kPageableMax && !any_overlap(h_r, out, h_a, in) &&
+                 !any_overlap(h_r, out, h_b, in) &&
+                 (!h_carry || (!any_overlap(h_carry, n, h_a, in) && !any_overlap(h_carry, n, h_b, in) &&
+                               !any_overlap(h_carry, n, h_r, out)));
+        for (int i = 0; i < 4 && go; ++i)
+            if (kind[i] == HostKind::Pageable) go = populate_pages(host[i], bytes[i], i >= 2);
+        if (go) {
+            MI_TRY(launch(d[0], d[1], d[2], static_cast<uint8_t*>(d[3]), n, ctx->pipe[2], ctx->host_zc_blocks[cls]));
             MI_CUDA_TRY(cudaStreamSynchronize(ctx->pipe[2]));
             return MI_OK;
         }
+    }
+    // mode 2: zero-copy reads of the operands when both are mapped
+    const char* za = nullptr;
+    const char* zb = nullptr;
+    if (mode == 1 || mode == 2) {
+        za = static_cast<const char*>(mapped_host(ctx, h_a));
+        zb = static_cast<const char*>(mapped_host(ctx, h_b));
+        if (!za || !zb) za = zb = nullptr;
     }
     // mode 3: the operands are copied in by chunks and the kernels write the
     // results in place when they (and the carries) are mapped pinned memory
     char* zr = nullptr;
     uint8_t* zc = nullptr;
     if (mode == 3) {
-        zr = static_cast<char*>(mapped_host(h_r));
-        zc = h_carry ? static_cast<uint8_t*>(mapped_host(h_carry)) : nullptr;
+        zr = static_cast<char*>(mapped_host(ctx, h_r));
+        zc = h_carry ? static_cast<uint8_t*>(mapped_host(ctx, h_carry)) : nullptr;
         if (h_carry && !zc) zr = nullptr;
     }
     const size_t per_inst = 2 * in_row + out_row + (h_carry ? 1 : 0);
@@ -375,6 +443,10 @@ mi_status mi_ctx_create(int device, mi_ctx* out) {
             cudaEventCreateWithFlags(&ctx->ev_k[i], cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&ctx->ev_out[i], cudaEventDisableTiming) != cudaSuccess)
             st = set_error(MI_ECUDA, "mi_ctx_create: event creation failed");
+    int access = 0, tables = 0;
+    if (st == MI_OK && cudaDeviceGetAttribute(&access, cudaDevAttrPageableMemoryAccess, device) == cudaSuccess &&
+        cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device) == cudaSuccess)
+        ctx->host_page_tables = access != 0 && tables != 0;
     if (st == MI_OK) st = ntt_tables_create(&ctx->ntt);
     if (st == MI_OK) {
         const size_t wb = kWideBytes;

@@ -26,6 +26,8 @@ struct mi_ctx_s {
     uint32_t host_zero_copy[2] = {mi::tuned::kHostZeroCopy[0], mi::tuned::kHostZeroCopy[1]};
     // zero-copy mode 1: resident blocks per SM of the classical product (0: all that fit)
     uint32_t host_zc_blocks[2] = {mi::tuned::kHostZcBlocks[0], mi::tuned::kHostZcBlocks[1]};
+    // the GPU reaches ordinary host memory through the host's page tables
+    bool host_page_tables = false;
     std::mutex mu;  // serialises host-pointer calls on one context
     // ragged batches: products whose shorter operand has at least this many
     // u64 limbs go through the NTT kernel (at most 257: classical groups hold

@@ -264,3 +264,33 @@ def test_calib_host_link(ctx):
     with pytest.raises(midint.MidintError) as e:
         midint.calib_host_link(src, dst, nb - 16)
     assert e.value.status == midint.MI_EINVAL
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2, 3])
+@pytest.mark.parametrize("n,m", [(1, 1), (9, 5), (513, 64), (1500, 128), (40, 700), (30000, 33), (400, 2048)])
+def test_ordinary_arrays(hctx, mode, n, m):
+    """Ordinary (pageable) arrays, which modes 1 and 2 use in place up to
+    32 MiB where the GPU can: results that were never written before, operands
+    at the edge of a page, a result over an operand, mixed with pinned ones."""
+    for cls in (0, 1):
+        hctx.set_tuning(midint.TUNE_HOST_ZERO_COPY, cls, mode)
+    a, b = carry_stress(n, m, seed=n + m)
+    full, (ra, ca) = O.mul(a, b, m, True), O.add(a, b, m)
+    r = np.empty(2 * n * m + 2, np.uint64)
+    r[0] = r[-1] = 77
+    hctx.host_mul_full(a, b, r[1:-1], n, m)
+    assert np.array_equal(r[1:-1], full) and r[0] == r[-1] == 77
+    s, c = np.empty(n * m, np.uint64), np.empty(n + 8, np.uint8)
+    c[n:] = 7
+    hctx.host_add(a, b, s, c, n, m)
+    assert np.array_equal(s, ra) and np.array_equal(c[:n], ca) and (c[n:] == 7).all()
+    pr = torch.zeros(2 * n * m, dtype=torch.int64).pin_memory()
+    hctx.host_mul_full(a, _pinned(b), pr, n, m)
+    assert np.array_equal(pr.numpy().view(np.uint64), full)
+    over = a.copy()
+    hctx.host_add(over, b, over, None, n, m)   # in place: as the device call
+    assert np.array_equal(over, ra)
+    # at four bytes past a multiple of eight: copied, whatever the mode
+    odd = np.zeros(4 * n * m + 4, np.uint32)[1:]
+    hctx.host_mul_full(a, b, odd[:4 * n * m], n, m)
+    assert np.array_equal(odd[:4 * n * m].copy().view(np.uint64), full)

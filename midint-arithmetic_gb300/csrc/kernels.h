@@ -51,7 +51,14 @@ uint32_t add_size_class(uint64_t bytes);
 mi_status launch_mul_classic(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32,
                              bool full, cudaStream_t st, uint32_t max_per_sm = 0);
 
-// Low n32 limbs of a*b per instance (u32 limb views), n32 > 8.
+// The same, full or low half, on groups of any number of lanes (mul_flex.cu):
+// flex_rounds says with how many rounds (1..3), or 0 where the power-of-two
+// groups are faster or hold the product alone.
+uint32_t flex_rounds(uint32_t n, uint32_t n32, bool full);
+mi_status launch_mul_flex(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32, bool full,
+                          uint32_t rounds, cudaStream_t st);
+
+// Low n32 limbs of a*b per instance (u32 limb views) on power-of-two groups, n32 > 128.
 mi_status launch_mul_lo(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32, cudaStream_t st);
 
 // ((a^2 + b)(b^2 + b) + ab) mod 2^(32*n32) per instance (u32 limb views).

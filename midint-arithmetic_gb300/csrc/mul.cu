@@ -1,19 +1,20 @@
-// mul.cu -- batched classical (quadratic) multiplication on 32-bit limbs.
+// mul.cu -- batched classical (quadratic) full products on 32-bit limbs, on
+// power-of-two groups of threads, and the dispatch of all classical products.
 //
 // Counterpart of the reference's bmulKerQ (cuda/ker-classic-mul.cu.h:468-498),
-// which returns the low half of the product of two m-limb operands.  Each
-// instance is one square product of mul_core.cuh, computed by a group of
-// NT = pow2ceil(n32/8) threads.  Groups of 16 or 32 threads run in blocks of
-// one warp, launched as one block per warp's worth of instances: the blocks
-// of an SM then start and finish at different times, so one warp's carry
-// resolution overlaps the others' tile loops, and the last wave spreads
-// evenly over the SMs (persistent blocks striding over the batch stay in phase
-// and measured 8-10 % slower; eight instances per 256-thread block 3 %
-// slower).  Other sizes, and launches capped at a few resident blocks per SM
-// (the zero-copy host path, whose cap was tuned on them), use blocks of
-// max(256, NT) threads that stride over the batch.  `full` selects the 2*n32-limb product or its low n32 limbs (the
-// reference's semantics); low halves of more than one block of limbs go to the
-// half-work kernel of mul_lo.cu.
+// which returns the low half of the product of two m-limb operands (here
+// mul_lo.cu and mul_flex.cu).  Each instance is one square product of
+// mul_core.cuh, computed by a group of NT = pow2ceil(n32/8) threads.  Groups of
+// 16 or 32 threads run in blocks of one warp, launched as one block per warp's
+// worth of instances: the blocks of an SM then start and finish at different
+// times, so one warp's carry resolution overlaps the others' tile loops, and
+// the last wave spreads evenly over the SMs (persistent blocks striding over
+// the batch stay in phase and measured 8-10 % slower; eight instances per
+// 256-thread block 3 % slower).  Other sizes, and launches capped at a few
+// resident blocks per SM (the zero-copy host path, whose cap was tuned on
+// them), use blocks of max(256, NT) threads that stride over the batch; groups
+// of fewer than 16 threads serve only those launches (mul_flex.cu the others:
+// over the host link 100000 x 4 limbs take 88 us here, 140 there).
 #include <cstdio>
 
 #include "common.cuh"
@@ -47,7 +48,7 @@ struct MulShape {
 template <int NT, bool VEC, bool WB>
 __global__ void __launch_bounds__(MulShape<NT, WB>::BLOCK, MulShape<NT, WB>::MIN_BLOCKS)
     k_mul(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b, uint32_t* __restrict__ r, uint32_t n,
-          uint32_t n32, bool full) {
+          uint32_t n32) {
     using S = MulShape<NT, WB>;
     extern __shared__ __align__(16) uint32_t smem[];
     uint32_t* sA = smem;
@@ -60,14 +61,14 @@ __global__ void __launch_bounds__(MulShape<NT, WB>::BLOCK, MulShape<NT, WB>::MIN
     uint4* gB4 = reinterpret_cast<uint4*>(sB + grp * S::WPAD);
     uint2* slots = reinterpret_cast<uint2*>(sT) + grp * NT * classic::PAIRS;
     uint32_t* scr = sA;  // only used after the tile loop, by groups wider than a warp
-    const uint32_t rlen = full ? 2 * n32 : n32;
+    const uint32_t rlen = 2 * n32;
     const uint32_t nb = (n32 + T - 1) / T;  // blocks holding limbs; the rest of the NT are zero padding
     const uint64_t stride = uint64_t(gridDim.x) * S::IPB;
     pdl_wait();  // launched with launch_pdl
     pdl_trigger();
 
     if constexpr ((NT == 16 || NT == 32) && !S::WARP && VEC) {
-        if (full && n32 == NT * T) {
+        if (n32 == NT * T) {
             // The capped launches of the zero-copy host path, whose rows are
             // host-mapped: each group reads the operands of its next instance
             // into registers while it multiplies this one, and its product
@@ -124,7 +125,7 @@ __global__ void __launch_bounds__(MulShape<NT, WB>::BLOCK, MulShape<NT, WB>::MIN
         if (valid) {
             uint32_t* rr = r + inst * rlen;
             classic::store_block<VEC>(rr, t * T, rlen, ulo);
-            if (full) classic::store_block<VEC>(rr, (t + NT) * T, rlen, uhi);
+            classic::store_block<VEC>(rr, (t + NT) * T, rlen, uhi);
         }
         group_sync<NT>();  // shared memory is reused by the next instance
     }
@@ -147,7 +148,7 @@ mi_status capped_smem(size_t smem, uint32_t max_per_sm, size_t* out) {
 }
 
 template <int NT, bool VEC, bool WB>
-mi_status launch_shape(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32, bool full,
+mi_status launch_shape(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32,
                        cudaStream_t st, uint32_t max_per_sm) {
     using S = MulShape<NT, WB>;
     auto kern = k_mul<NT, VEC, WB>;
@@ -159,33 +160,33 @@ mi_status launch_shape(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32
     // stride over the batch from a grid of a few waves
     const uint64_t cap = S::WARP ? (uint64_t(1) << 24) : uint64_t(sm_count()) * 32;
     if (blocks > cap) blocks = cap;
-    MI_CUDA_TRY(launch_pdl(kern, dim3(uint32_t(blocks)), dim3(S::BLOCK), smem, st, a, b, r, n, n32, full));
+    MI_CUDA_TRY(launch_pdl(kern, dim3(uint32_t(blocks)), dim3(S::BLOCK), smem, st, a, b, r, n, n32));
     return MI_OK;
 }
 
 template <int NT, bool VEC>
-mi_status launch_nt(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32, bool full,
+mi_status launch_nt(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32,
                     cudaStream_t st, uint32_t max_per_sm) {
     if constexpr (NT == 16 || NT == 32)
-        if (max_per_sm == 0) return launch_shape<NT, VEC, true>(a, b, r, n, n32, full, st, 0);
-    return launch_shape<NT, VEC, false>(a, b, r, n, n32, full, st, max_per_sm);
+        if (max_per_sm == 0) return launch_shape<NT, VEC, true>(a, b, r, n, n32, st, 0);
+    return launch_shape<NT, VEC, false>(a, b, r, n, n32, st, max_per_sm);
 }
 
 template <bool VEC>
-mi_status dispatch(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32, bool full,
+mi_status dispatch(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32,
                    cudaStream_t st, uint32_t cap) {
     const uint32_t nt = pow2ceil((n32 + T - 1) / T);
     switch (nt) {
-        case 1: return launch_nt<1, VEC>(a, b, r, n, n32, full, st, cap);
-        case 2: return launch_nt<2, VEC>(a, b, r, n, n32, full, st, cap);
-        case 4: return launch_nt<4, VEC>(a, b, r, n, n32, full, st, cap);
-        case 8: return launch_nt<8, VEC>(a, b, r, n, n32, full, st, cap);
-        case 16: return launch_nt<16, VEC>(a, b, r, n, n32, full, st, cap);
-        case 32: return launch_nt<32, VEC>(a, b, r, n, n32, full, st, cap);
-        case 64: return launch_nt<64, VEC>(a, b, r, n, n32, full, st, cap);
-        case 128: return launch_nt<128, VEC>(a, b, r, n, n32, full, st, cap);
-        case 256: return launch_nt<256, VEC>(a, b, r, n, n32, full, st, cap);
-        case 512: return launch_nt<512, VEC>(a, b, r, n, n32, full, st, cap);
+        case 1: return launch_nt<1, VEC>(a, b, r, n, n32, st, cap);
+        case 2: return launch_nt<2, VEC>(a, b, r, n, n32, st, cap);
+        case 4: return launch_nt<4, VEC>(a, b, r, n, n32, st, cap);
+        case 8: return launch_nt<8, VEC>(a, b, r, n, n32, st, cap);
+        case 16: return launch_nt<16, VEC>(a, b, r, n, n32, st, cap);
+        case 32: return launch_nt<32, VEC>(a, b, r, n, n32, st, cap);
+        case 64: return launch_nt<64, VEC>(a, b, r, n, n32, st, cap);
+        case 128: return launch_nt<128, VEC>(a, b, r, n, n32, st, cap);
+        case 256: return launch_nt<256, VEC>(a, b, r, n, n32, st, cap);
+        case 512: return launch_nt<512, VEC>(a, b, r, n, n32, st, cap);
         default: return set_error(MI_EINVAL, "mul: %u u32 limbs exceeds the classical maximum", n32);
     }
 }
@@ -194,11 +195,13 @@ mi_status dispatch(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n
 
 mi_status launch_mul_classic(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32, bool full,
                              cudaStream_t st, uint32_t max_per_sm) {
+    if (!full || max_per_sm == 0) {
+        const uint32_t rounds = flex_rounds(n, n32, full);
+        if (rounds != 0) return launch_mul_flex(a, b, r, n, n32, full, rounds, st);
+    }
+    if (!full) return launch_mul_lo(a, b, r, n, n32, st);  // half the partial products of a full product
     const bool vec = aligned16(a) && aligned16(b) && aligned16(r) && (n32 % 4 == 0);
-    if (!full && n32 > T)  // low halves: half the partial products of a full product
-        return launch_mul_lo(a, b, r, n, n32, st);
-    return vec ? dispatch<true>(a, b, r, n, n32, full, st, max_per_sm)
-               : dispatch<false>(a, b, r, n, n32, full, st, max_per_sm);
+    return vec ? dispatch<true>(a, b, r, n, n32, st, max_per_sm) : dispatch<false>(a, b, r, n, n32, st, max_per_sm);
 }
 
 }  // namespace mi

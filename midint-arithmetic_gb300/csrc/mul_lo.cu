@@ -3,7 +3,9 @@
 // The reference's bmulKerQ (cuda/ker-classic-mul.cu.h:468-498) returns the low
 // m limbs of m-limb products.  Only the anti-diagonals below the middle of the
 // partial-product grid reach those limbs, so this kernel uses
-// classic::low_product (half the partial products of a full product).
+// classic::low_product (half the partial products of a full product), on groups
+// of 16 threads (17 blocks of limbs) and more; mul_flex.cu takes the smaller
+// ones and the larger ones that it does in fewer steps.
 #include <cstdio>
 
 #include "mul_lo.cuh"
@@ -42,11 +44,11 @@ __global__ void __launch_bounds__(NH > 256 ? NH : 256, 3)
         classic::stage_planes<S::NB, NH, VEC>(gB4, b + off, n32, valid, t);
         group_sync<NH>();
         uint32_t ulo[T], uhi[T];
-        if (nb == S::NB)  // no padding: a compile-time trip count, unrolled in full for 9..65 steps
+        if (nb == S::NB)  // no padding: a compile-time trip count, unrolled in full for 33 and 65 steps
             // each step's operands read one step ahead for 16- and 32-thread groups
             // on aligned rows (8192-bit batch 0.0776 -> 0.0757 ms; the other shapes
             // would spill more)
-            classic::low_product<NH, (NH >= 4 && NH <= 32) ? 2 * NH + 1 : (NH >= 16 ? 8 : 2),
+            classic::low_product<NH, (NH <= 32) ? 2 * NH + 1 : 8,
                                  VEC && (NH == 16 || NH == 32)>(gA4, gB4, slots, scr, t, ulo, uhi, S::NB);
         else
             classic::low_product<NH>(gA4, gB4, slots, scr, t, ulo, uhi, nb);
@@ -64,10 +66,9 @@ mi_status dispatch(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n
     switch (lo_threads(n32)) {
 #define MI_LO_CASE(NH) \
     case NH: return launch_lo<NH>(k_mul_lo<NH, VEC>, a, b, r, n, n32, st);
-        MI_LO_CASE(1) MI_LO_CASE(2) MI_LO_CASE(4) MI_LO_CASE(8) MI_LO_CASE(16) MI_LO_CASE(32) MI_LO_CASE(64)
-        MI_LO_CASE(128) MI_LO_CASE(256)
+        MI_LO_CASE(16) MI_LO_CASE(32) MI_LO_CASE(64) MI_LO_CASE(128) MI_LO_CASE(256)
 #undef MI_LO_CASE
-        default: return set_error(MI_EINVAL, "mul: %u u32 limbs exceeds the classical maximum", n32);
+        default: return set_error(MI_EINVAL, "mul: %u u32 limbs outside the range of the power-of-two groups", n32);
     }
 }
 

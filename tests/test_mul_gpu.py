@@ -134,3 +134,21 @@ def test_host_mul_full(ctx):
     r = np.zeros(700 * 256, np.uint64)
     ctx.host_mul_full(a, b, r, 700, 128)
     assert np.array_equal(r, O.mul(a, b, 128, True))
+
+
+@pytest.mark.parametrize("full", [True, False])
+@pytest.mark.parametrize("m", [1, 7, 8, 9, 23, 39, 41, 56, 72, 88, 104, 129, 136, 145, 160, 184, 193, 249, 255, 257,
+                               264, 301, 320, 345, 520, 767, 1025, 1536])
+def test_mul_lane_groups(ctx, devmem, m, full):
+    # block counts whose groups are any number of lanes (5 to 32, several
+    # products per warp, up to three rounds of anti-diagonals per lane), with a
+    # few products and with enough for the rule to take more rounds
+    big = 9000 if m <= 72 else 4000 if m <= 320 else 700
+    a, b = carry_stress(big, m, seed=m, dtype=np.uint32)
+    a[3 * m:4 * m] = b[3 * m:4 * m] = 0xFFFFFFFF
+    want = O.mul(a, b, m, full)
+    rl = 2 * m if full else m
+    for n in (1, 37, 1216, big):
+        if n <= big:
+            got = gpu_mul(ctx, devmem, a[:n * m], b[:n * m], m, full, limb_bits=32, offset=n & 1)
+            assert np.array_equal(got, want[:n * rl]), n

@@ -191,7 +191,12 @@ mi_status mi_add6_u64(mi_ctx ctx, const uint64_t* a, const uint64_t* b, uint64_t
  *                low limbs only, from MI_TUNE_LO_NTT_MIN limbs on (tuned:
  *                where the NTT's full product costs less than the classical
  *                low half); the result is the same either way.
- * mi_mul_full_*: r = a*b                      (n*2*limbs limbs).
+ *                mi_mul_lo_u32 does the same for even numbers of limbs on
+ *                8-byte aligned rows.
+ * mi_mul_full_*: r = a*b                      (n*2*limbs limbs).  From 129
+ *                u64 limbs on (even numbers of u32 limbs, 8-byte aligned
+ *                rows, and MI_TUNE_PLAIN_NTT_MIN permitting) the exact NTT
+ *                kernel, with the same result.
  * r must not overlap a or b.
  * ------------------------------------------------------------------------- */
 mi_status mi_mul_lo_u64(mi_ctx ctx, const uint64_t* a, const uint64_t* b, uint64_t* r,

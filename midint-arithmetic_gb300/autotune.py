@@ -111,8 +111,11 @@ def crossover_pick(sizes: list[int], ntt_faster: dict[int, bool], never: int = 2
 def tune_plain_crossover(ctx, stream, dev) -> tuple[int, dict]:
     import torch
 
-    sizes = [64, 96, 128, 160, 192, 256, 320, 384, 512, 640, 768, 1024]
+    import midint
+
+    sizes = [64, 80, 96, 112, 128, 160, 192, 256, 320, 384, 512, 640, 768, 1024]
     record, ntt_faster = {}, {}
+    ctx.set_tuning(midint.TUNE_PLAIN_NTT_MIN, 0, 2049)  # mul_full: classical at every size
     for m in sizes:
         n = max(512, (64 << 20) // (8 * m))
         a = torch.randint(-2**62, 2**62, (n * m,), dtype=torch.int64, device=dev)
@@ -127,6 +130,7 @@ def tune_plain_crossover(ctx, stream, dev) -> tuple[int, dict]:
         del a, b, r
         torch.cuda.empty_cache()
     pick = crossover_pick(sizes, ntt_faster)
+    ctx.set_tuning(midint.TUNE_PLAIN_NTT_MIN, 0, pick)
     return pick, record
 
 
@@ -138,7 +142,7 @@ def tune_lo_crossover(ctx, stream, dev) -> tuple[int, dict]:
 
     import midint
 
-    sizes = [256, 320, 384, 448, 512, 640, 768, 1024, 1536, 2048]
+    sizes = [160, 192, 224, 256, 288, 320, 384, 448, 512, 640, 768, 1024, 1536, 2048]
     record, ntt_faster = {}, {}
     sp = stream.cuda_stream
     for m in sizes:

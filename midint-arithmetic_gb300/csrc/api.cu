@@ -9,6 +9,7 @@
 // through staging buffers the context keeps.
 #include <cstdarg>
 #include <cstdio>
+#include <algorithm>
 #include <cstring>
 #include <atomic>
 #include <map>
@@ -137,11 +138,32 @@ mi_status add_any(mi_ctx ctx, const void* a, const void* b, void* r, uint8_t* ca
                           static_cast<uint32_t*>(r), carry, n, limbs, tb, st, &ctx->wide);
 }
 
-// pick_ntt: a low half of at least ctx->lo_ntt_min u64 limbs comes from the
-// NTT kernel (same result; the NTT's cost grows as L lg L, the classical low
-// half's as limbs^2)
+// Full products of more limbs than one warp's classical groups hold (128) go
+// to the NTT kernel, unless the context's crossover keeps them from it: there
+// the classical groups need two warps and more (8192 products of 200 limbs
+// 212 us against 146, 400 of 380 limbs 61 against 18).
+constexpr uint32_t kFullNttMin = 129;
+
+// The crossover for a batch of n products of m limbs where the context's is
+// ntt_min (which is measured on batches that fill the GPU): a batch small enough for a
+// cluster per product takes the NTT from a third of it on (full products; a
+// sixth for low halves, half the classical work), since its time is the
+// latency of one product -- 4.1 to 4.3 us for up to 300 products of up to 128
+// limbs, which the classical groups' own chain of steps passes at some 40
+// limbs (20 products of 24 limbs 4.1 us classical, of 40 5.0, of 64 6.8, of 96
+// 9.1).  A crossover above every size (2049) stays one.
+uint32_t batch_ntt_min(uint32_t n, uint32_t m, uint32_t ntt_min, bool full) {
+    if (ntt_min > kNttMaxLimbs || m > kNttMaxLimbs || !ntt_small_batch(n, m)) return ntt_min;
+    return ntt_min / (full ? 3 : 6);
+}
+
+// Low halves of at least ctx->lo_ntt_min u64 limbs, and full products as
+// above, come from the NTT kernel (same result; its cost grows as L lg L, the
+// classical one's as limbs^2).  An even number of u32 limbs is half as many
+// u64 limbs; the NTT kernels read 8-byte words, so rows that are only 4-byte
+// aligned take the classical kernels, which read 32-bit words.
 mi_status mul_any(mi_ctx ctx, const void* a, const void* b, void* r, uint32_t n, uint32_t limbs, mi_stream stream,
-                  int limb_bytes, bool full, bool pick_ntt = false) {
+                  int limb_bytes, bool full) {
     const uint32_t maxl = kMulMaxN32 / (limb_bytes / 4);
     MI_TRY(check_batch(a, b, r, limbs, maxl, full ? "mul_full" : "mul_lo"));
     const size_t in_bytes = size_t(n) * limbs * limb_bytes;
@@ -150,13 +172,12 @@ mi_status mul_any(mi_ctx ctx, const void* a, const void* b, void* r, uint32_t n,
         return set_error(MI_EINVAL, "mul: result overlaps an operand");
     if (n == 0) return MI_OK;
     MI_TRY(check_ctx(ctx));
-    // (the NTT kernels read 8-byte words: rows that are only 4-byte aligned
-    // take the classical kernel, which reads 32-bit words)
-    if (pick_ntt && !full && limb_bytes == 8 && limbs >= ctx->lo_ntt_min && limbs <= kNttMaxLimbs &&
-        aligned8(a) && aligned8(b) && aligned8(r))
-        return launch_mul_ntt(static_cast<const uint64_t*>(a), static_cast<const uint64_t*>(b),
-                              static_cast<uint64_t*>(r), n, limbs, ctx->ntt.params, pick_stream(ctx, stream), true);
     const uint32_t n32 = limbs * uint32_t(limb_bytes / 4);
+    uint32_t ntt_min = batch_ntt_min(n, n32 / 2, full ? ctx->plain_ntt_min : ctx->lo_ntt_min, full);
+    if (full && ntt_min == ctx->plain_ntt_min) ntt_min = std::max(ntt_min, kFullNttMin);
+    if (n32 % 2 == 0 && n32 / 2 >= ntt_min && n32 / 2 <= kNttMaxLimbs && aligned8(a) && aligned8(b) && aligned8(r))
+        return launch_mul_ntt(static_cast<const uint64_t*>(a), static_cast<const uint64_t*>(b),
+                              static_cast<uint64_t*>(r), n, n32 / 2, ctx->ntt.params, pick_stream(ctx, stream), !full);
     return launch_mul_classic(static_cast<const uint32_t*>(a), static_cast<const uint32_t*>(b),
                               static_cast<uint32_t*>(r), n, n32, full, pick_stream(ctx, stream));
 }
@@ -616,7 +637,7 @@ mi_status mi_add6_u64(mi_ctx ctx, const uint64_t* a, const uint64_t* b, uint64_t
 
 mi_status mi_mul_lo_u64(mi_ctx ctx, const uint64_t* a, const uint64_t* b, uint64_t* r, uint32_t n, uint32_t limbs,
                         mi_stream stream) {
-    return mul_any(ctx, a, b, r, n, limbs, stream, 8, false, true);
+    return mul_any(ctx, a, b, r, n, limbs, stream, 8, false);
 }
 mi_status mi_mul_lo_u32(mi_ctx ctx, const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t limbs,
                         mi_stream stream) {
@@ -693,7 +714,8 @@ mi_status mi_mul_ntt_u64(mi_ctx ctx, const uint64_t* a, const uint64_t* b, uint6
 mi_status mi_mul_u64(mi_ctx ctx, const uint64_t* a, const uint64_t* b, uint64_t* r, uint32_t n, uint32_t limbs,
                      mi_stream stream) {
     if (ctx == nullptr) return set_error(MI_EINVAL, "null context");
-    if (limbs >= ctx->plain_ntt_min && limbs <= kNttMaxLimbs && aligned8(a) && aligned8(b) && aligned8(r))
+    if (limbs <= kNttMaxLimbs && aligned8(a) && aligned8(b) && aligned8(r) &&
+        limbs >= batch_ntt_min(n, limbs, ctx->plain_ntt_min, true))
         return mul_ntt(ctx, a, b, r, n, limbs, stream);
     return mul_any(ctx, a, b, r, n, limbs, stream, 8, true);
 }

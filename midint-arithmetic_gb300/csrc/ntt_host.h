@@ -46,6 +46,10 @@ void ntt_tables_destroy(NttTables* T);
 mi_status launch_mul_ntt(const uint64_t* a, const uint64_t* b, uint64_t* r, uint32_t n, uint32_t m,
                          const NttMulParams& P, cudaStream_t st, bool low = false);
 
+// Whether launch_mul_ntt runs n products of m limbs on clusters (a block per
+// prime), where a call takes little more than the latency of one prime.
+bool ntt_small_batch(uint32_t n, uint32_t m);
+
 // One transform or one cyclic convolution on a single prime (device buffers).
 struct NttRawArgs {
     const uint64_t* a;

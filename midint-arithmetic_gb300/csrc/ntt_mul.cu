@@ -99,12 +99,16 @@ __global__ void __launch_bounds__((1 << LG) / 8)
 // 13.2 against 11.2; m = 256, n = 300 11.4 against 10.4).
 constexpr uint32_t cluster_blocks_per_sm(int lg) { return lg == 8 ? 16 : lg == 9 ? 7 : lg <= 11 ? 3 : 2; }
 
+bool cluster_fits(uint32_t n, int np, int lg) {
+    return uint64_t(n) * uint32_t(np) < uint64_t(sm_count()) * cluster_blocks_per_sm(lg);
+}
+
 template <int LG, int NP>
 mi_status launch_lg(const uint64_t* a, const uint64_t* b, uint64_t* r, uint32_t n, uint32_t m, uint32_t rlen,
                     const NttMulParams& P, cudaStream_t st) {
     using S = NttShape<LG>;
     const bool low = rlen <= m;  // the low half alone
-    if (uint64_t(n) * NP < uint64_t(sm_count()) * cluster_blocks_per_sm(LG)) {
+    if (cluster_fits(n, NP, LG)) {
         auto kern = low ? k_ntt_mul_cluster<LG, NP, true> : k_ntt_mul_cluster<LG, NP, false>;
         static ResidentBlocks site[2];
         int per_sm = 0;
@@ -211,6 +215,12 @@ __global__ void __launch_bounds__((1 << LG) / 8)
 }
 
 }  // namespace
+
+bool ntt_small_batch(uint32_t n, uint32_t m) {
+    int lg = ntt32::kLgMin;
+    while ((1u << lg) < 2 * m) ++lg;
+    return lg <= ntt32::kLgMax && cluster_fits(n, 5 - ntt32::ntt_mode(m, m, 1u << lg), lg);
+}
 
 mi_status launch_mul_ntt(const uint64_t* a, const uint64_t* b, uint64_t* r, uint32_t n, uint32_t m,
                          const NttMulParams& base, cudaStream_t st, bool low) {

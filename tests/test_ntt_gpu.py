@@ -241,3 +241,24 @@ def test_mul_ntt_batch_sizes(ctx, devmem, m, low):
         del keep_a, keep_b
     finally:
         ctx.set_tuning(midint.TUNE_LO_NTT_MIN, 0, old)
+
+
+@pytest.mark.parametrize("call", ["mul", "mul_full", "mul_lo"])
+@pytest.mark.parametrize("m", [41, 42, 43, 47, 48, 49, 95, 127, 128, 129, 130, 287, 288])
+def test_product_dispatch_by_batch_size(ctx, devmem, m, call):
+    # either side of the crossovers of small and large batches; rows that are
+    # only 4-byte aligned and u32 views take the same results
+    full = call != "mul_lo"
+    for n in (1, 20, 1500):
+        a, b = carry_stress(n, m, seed=m + n)
+        want = O.mul(a, b, m, full)
+        words = 2 * a.size * (2 if full else 1)
+        for off, bits in ((0, 64), (0, 32), (1, 32)):
+            if call == "mul" and bits == 32:
+                continue
+            (ba, pa), (bb, pb), (br, pr) = devmem.put(a, off), devmem.put(b, off), devmem.empty_words(words, off)
+            kw = {} if call == "mul" else {"limb_bits": bits}
+            getattr(ctx, call)(pa, pb, pr, n, m * 64 // bits, stream=_stream(), **kw)
+            torch.cuda.synchronize()
+            assert np.array_equal(devmem.get(br, words, off), want), (n, off, bits)
+            del ba, bb

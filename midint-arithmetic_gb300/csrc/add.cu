@@ -13,7 +13,8 @@
 // Mapping: a group of GS threads (power of two) owns one instance, thread t of
 // the group owns limbs [t*Q, t*Q+Q).  GS*Q >= limbs; limbs beyond the instance
 // are zero and never stored.  A block of max(256, GS) threads holds 256/GS
-// groups and strides over the batch.
+// groups and strides over the batch.  (Rows that allow no 16-byte access: the
+// group's limbs are dealt in rows instead, k_add_rows.)
 #include <cstdio>
 
 #include "common.cuh"
@@ -74,38 +75,35 @@ __device__ __forceinline__ uint4 pack16(const L* v) {
     return t;
 }
 
-// Loads the chunk [start, start+Q) of one instance row, zero beyond m.
-template <typename L, int Q, bool VEC>
+// Loads the chunk [start, start+Q) of one 16-byte aligned instance row, zero
+// beyond m.
+template <typename L, int Q>
 __device__ __forceinline__ void load_chunk(const L* __restrict__ row, uint32_t start, uint32_t m, bool valid,
                                            L (&v)[Q]) {
     constexpr int PER = 16 / sizeof(L);
-    if constexpr (VEC) {
-        if (valid && start + Q <= m) {
-            const uint4* p = reinterpret_cast<const uint4*>(row + start);
+    if (valid && start + Q <= m) {
+        const uint4* p = reinterpret_cast<const uint4*>(row + start);
 #pragma unroll
-            for (int k = 0; k < Q / PER; ++k) {
-                const uint4 t = __ldcs(p + k);
-                unpack16<L, Q>(t, &v[k * PER]);
-            }
-            return;
+        for (int k = 0; k < Q / PER; ++k) {
+            const uint4 t = __ldcs(p + k);
+            unpack16<L, Q>(t, &v[k * PER]);
         }
+        return;
     }
 #pragma unroll
     for (int q = 0; q < Q; ++q) v[q] = (valid && start + q < m) ? ld_stream(row + start + q) : L(0);
 }
 
-template <typename L, int Q, bool VEC>
+template <typename L, int Q>
 __device__ __forceinline__ void store_chunk(L* __restrict__ row, uint32_t start, uint32_t m, bool valid,
                                             const L (&v)[Q]) {
     constexpr int PER = 16 / sizeof(L);
     if (!valid) return;
-    if constexpr (VEC) {
-        if (start + Q <= m) {
-            uint4* p = reinterpret_cast<uint4*>(row + start);
+    if (start + Q <= m) {
+        uint4* p = reinterpret_cast<uint4*>(row + start);
 #pragma unroll
-            for (int k = 0; k < Q / PER; ++k) __stcs(p + k, pack16<L, Q>(&v[k * PER]));
-            return;
-        }
+        for (int k = 0; k < Q / PER; ++k) __stcs(p + k, pack16<L, Q>(&v[k * PER]));
+        return;
     }
 #pragma unroll
     for (int q = 0; q < Q; ++q)
@@ -141,7 +139,7 @@ __device__ __forceinline__ uint64_t group_shift_up(uint64_t v, uint32_t t, uint6
     }
 }
 
-template <typename L, int Q, int GS, bool VEC, int OP>
+template <typename L, int Q, int GS, int OP>
 __global__ void __launch_bounds__(GS > 256 ? GS : 256)
     k_add(const L* __restrict__ a, const L* __restrict__ b, L* __restrict__ r, uint8_t* __restrict__ carry,
           uint32_t n, uint32_t m) {
@@ -161,8 +159,8 @@ __global__ void __launch_bounds__(GS > 256 ? GS : 256)
         const bool valid = inst < n;
         const uint64_t off = valid ? inst * m : 0;
         L x[Q], y[Q], s[Q];
-        load_chunk<L, Q, VEC>(a + off, start, m, valid, x);
-        load_chunk<L, Q, VEC>(b + off, start, m, valid, y);
+        load_chunk<L, Q>(a + off, start, m, valid, x);
+        load_chunk<L, Q>(b + off, start, m, valid, y);
         uint32_t gc;
         if constexpr (OP == ADD_PLAIN) {
             gc = group_add<L, Q, GS>(x, y, s, scratch);
@@ -186,7 +184,7 @@ __global__ void __launch_bounds__(GS > 256 ? GS : 256)
             for (int q = 1; q < Q; ++q) sh[q] = hi[q - 1];
             gc = group_add<L, Q, GS>(lo, sh, s, scratch);
         }
-        store_chunk<L, Q, VEC>(r + off, start, m, valid, s);
+        store_chunk<L, Q>(r + off, start, m, valid, s);
         if (OP == ADD_PLAIN && carry != nullptr && valid) {
             // The carry-out is the value left at limb position m (a padding
             // limb of zeros plus the carry), or the group's carry-out when the
@@ -195,6 +193,116 @@ __global__ void __launch_bounds__(GS > 256 ? GS : 256)
 #pragma unroll
                 for (int q = 0; q < Q; ++q)
                     if (start + q == m) carry[inst] = uint8_t(s[q]);
+            } else if (t == GS - 1) {
+                carry[inst] = uint8_t(gc);
+            }
+        }
+    }
+}
+
+// High word (at most 15) of the limb 6 a_i + 10 b_i.
+__device__ __forceinline__ uint64_t six_hi(uint64_t ai, uint64_t bi) {
+    const uint64_t pa = ai * 6u, pb = bi * 10u;
+    return __umul64hi(ai, 6u) + __umul64hi(bi, 10u) + uint64_t(pa + pb < pa);
+}
+
+// The same for rows that allow no 16-byte access (odd lengths, 4-byte aligned
+// rows).  With Q consecutive limbs per thread their loads would be Q strided
+// single-limb accesses, each touching every line of the warp's span; here lane
+// c of a warp's WL lanes of the group holds limb c of Q rows of WL consecutive
+// limbs, so every access of the warp is contiguous.  A row's carries are one
+// lookahead over its two ballots, the rows chained by their one-bit carry;
+// groups wider than a warp do it twice, with the carry into the warp from a
+// lookahead over one word per warp in between.  (2048 x 4095 limbs 60.4 ->
+// 38.6 us, 8380 x 1001 42.7 -> 29.9, 1677721 x 5 55.5 -> 30.8, 16760 x 1001
+// 32-bit limbs 67.1 -> 31.8, 2048 x 8191 116.5 -> 54.4.)
+template <typename L, int Q, int GS, int OP>
+__global__ void __launch_bounds__(GS > 256 ? GS : 256)
+    k_add_rows(const L* __restrict__ a, const L* __restrict__ b, L* __restrict__ r, uint8_t* __restrict__ carry,
+               uint32_t n, uint32_t m) {
+    constexpr int BLOCK = GS > 256 ? GS : 256;
+    constexpr int IPB = BLOCK / GS;
+    constexpr int WL = GS < 32 ? GS : 32;  // lanes of the group in a warp
+    constexpr int WARPS = GS / WL;         // warps of the group
+    constexpr uint32_t MASK = WL == 32 ? MI_FULL_MASK : (1u << WL) - 1u;
+    __shared__ uint32_t wflag[WARPS > 1 ? BLOCK / 32 : 1];  // bit 0 generate (carry-in 0), bit 1 propagate
+    const uint32_t grp = threadIdx.x / GS, t = threadIdx.x % GS;
+    const uint32_t c = t % WL, wig = t / WL, gb = (threadIdx.x & 31u) & ~uint32_t(WL - 1);
+    const uint32_t start = wig * (WL * Q) + c;  // the thread's limb of row 0
+    const uint64_t stride = uint64_t(gridDim.x) * IPB;
+    pdl_wait();  // launched with launch_pdl
+    pdl_trigger();
+    for (uint64_t base = uint64_t(blockIdx.x) * IPB; base < n; base += stride) {
+        const uint64_t inst = base + grp;
+        const bool valid = inst < n;
+        const uint64_t off = valid ? inst * m : 0;
+        const uint32_t mm = valid ? m : 0;
+        L x[Q], y[Q], s[Q];
+#pragma unroll
+        for (int k = 0; k < Q; ++k) x[k] = start + WL * k < mm ? ld_stream(a + off + start + WL * k) : L(0);
+#pragma unroll
+        for (int k = 0; k < Q; ++k) y[k] = start + WL * k < mm ? ld_stream(b + off + start + WL * k) : L(0);
+        if constexpr (OP == ADD_SIX) {
+            // 6a + 10b as lo + (hi shifted up one limb), as in k_add
+            static_assert(sizeof(L) == 8, "6a + 10b is defined on u64 limbs");
+            uint64_t before = 0;  // lane 0: the high word of the limb before the row
+            if (WARPS > 1 && c == 0 && start > 0 && start - 1 < mm)
+                before = six_hi(a[off + start - 1], b[off + start - 1]);
+#pragma unroll
+            for (int k = 0; k < Q; ++k) {
+                const uint64_t hi = six_hi(x[k], y[k]);
+                x[k] = x[k] * 6u + y[k] * 10u;
+                const uint64_t up = __shfl_up_sync(MI_FULL_MASK, hi, 1, WL);
+                y[k] = c == 0 ? before : up;
+                before = __shfl_sync(MI_FULL_MASK, hi, WL - 1, WL);
+            }
+        }
+        uint32_t gc = 0;  // the group's carry-out
+        if constexpr (WARPS == 1) {
+#pragma unroll
+            for (int k = 0; k < Q; ++k) {
+                s[k] = x[k] + y[k];
+                const uint64_t Y = (__ballot_sync(MI_FULL_MASK, s[k] < x[k]) >> gb) & MASK;
+                const uint64_t X = ((__ballot_sync(MI_FULL_MASK, s[k] == L(~L(0))) >> gb) & MASK) | Y;
+                const uint64_t S = X + Y + gc;
+                s[k] += L(((S ^ X ^ Y) >> c) & 1u);
+                gc = uint32_t(S >> WL) & 1u;
+            }
+        } else {
+            uint32_t G[Q], P[Q], cw = 0;
+            bool ones = true;
+#pragma unroll
+            for (int k = 0; k < Q; ++k) {
+                s[k] = x[k] + y[k];
+                G[k] = __ballot_sync(MI_FULL_MASK, s[k] < x[k]);
+                P[k] = __ballot_sync(MI_FULL_MASK, s[k] == L(~L(0)));
+                cw = uint32_t((uint64_t(G[k] | P[k]) + G[k] + cw) >> 32);
+                ones = ones && P[k] == MI_FULL_MASK;
+            }
+            if (c == 0) wflag[threadIdx.x >> 5] = cw | (ones ? 2u : 0u);
+            __syncthreads();
+            const uint32_t f = c < WARPS ? wflag[grp * WARPS + c] : 0u;
+            const uint64_t Y = __ballot_sync(MI_FULL_MASK, f & 1u);
+            const uint64_t X = __ballot_sync(MI_FULL_MASK, (f & 2u) != 0) | Y, S = X + Y;
+            gc = uint32_t(S >> WARPS) & 1u;
+            cw = uint32_t((S ^ X ^ Y) >> wig) & 1u;  // into the warp
+#pragma unroll
+            for (int k = 0; k < Q; ++k) {
+                const uint64_t rx = G[k] | P[k], ry = G[k], rs = rx + ry + cw;
+                s[k] += L(((rs ^ rx ^ ry) >> c) & 1u);
+                cw = uint32_t(rs >> 32);
+            }
+            __syncthreads();  // the flags are rewritten by the next instance
+        }
+#pragma unroll
+        for (int k = 0; k < Q; ++k)
+            if (start + WL * k < mm) st_stream(r + off + start + WL * k, s[k]);
+        if (OP == ADD_PLAIN && carry != nullptr && valid) {
+            // as in k_add: the value left at limb position m, or the group's carry-out
+            if (m < uint32_t(GS * Q)) {
+#pragma unroll
+                for (int k = 0; k < Q; ++k)
+                    if (start + WL * k == m) carry[inst] = uint8_t(s[k]);
             } else if (t == GS - 1) {
                 carry[inst] = uint8_t(gc);
             }
@@ -273,12 +381,6 @@ __device__ __forceinline__ void store_row(L* __restrict__ row, uint32_t i, uint3
 #pragma unroll
     for (int k = 0; k < V; ++k)
         if (i + k < m) st_stream(row + i + k, v[k]);
-}
-
-// High word (at most 15) of the limb 6 a_i + 10 b_i.
-__device__ __forceinline__ uint64_t six_hi(uint64_t ai, uint64_t bi) {
-    const uint64_t pa = ai * 6u, pb = bi * 10u;
-    return __umul64hi(ai, 6u) + __umul64hi(bi, 10u) + uint64_t(pa + pb < pa);
 }
 
 // What a tile needs of the limbs below it, as one byte.  Plain addition: its
@@ -524,7 +626,11 @@ mi_status launch_one(const L* a, const L* b, L* r, uint8_t* carry, uint32_t n, u
     // Enough blocks for full residency several times over; the kernel strides.
     const uint64_t cap = uint64_t(sm_count()) * 64;
     if (blocks > cap) blocks = cap;
-    MI_CUDA_TRY(launch_pdl(k_add<L, Q, GS, VEC, OP>, dim3(uint32_t(blocks)), dim3(BLOCK), 0, st, a, b, r, carry, n, m));
+    if constexpr (VEC)
+        MI_CUDA_TRY(launch_pdl(k_add<L, Q, GS, OP>, dim3(uint32_t(blocks)), dim3(BLOCK), 0, st, a, b, r, carry, n, m));
+    else
+        MI_CUDA_TRY(
+            launch_pdl(k_add_rows<L, Q, GS, OP>, dim3(uint32_t(blocks)), dim3(BLOCK), 0, st, a, b, r, carry, n, m));
     return MI_OK;
 }
 
@@ -547,19 +653,35 @@ mi_status dispatch_gs(const L* a, const L* b, L* r, uint8_t* carry, uint32_t n, 
     }
 }
 
-// Q = thread_bytes / sizeof(L) limbs per thread (16, 32 or 64 bytes, raised
-// until the group fits 1024 threads), GS = pow2ceil(m / Q) threads per
-// instance.  VEC needs 16-byte aligned rows.
-template <typename L, bool VEC, int OP>
-mi_status dispatch(const L* a, const L* b, L* r, uint8_t* carry, uint32_t n, uint32_t m, uint32_t thread_bytes,
-                   cudaStream_t st) {
+// k_add, 16-byte aligned rows: Q = thread_bytes / sizeof(L) limbs per thread
+// (16, 32 or 64 bytes, raised until the group fits 1024 threads), GS =
+// pow2ceil(m / Q) threads per instance.
+template <typename L, int OP>
+mi_status dispatch_vec(const L* a, const L* b, L* r, uint8_t* carry, uint32_t n, uint32_t m, uint32_t thread_bytes,
+                       cudaStream_t st) {
     constexpr uint32_t QS = 16 / sizeof(L);  // limbs per 128-bit access
     uint32_t q = thread_bytes >= 64 ? 4 * QS : (thread_bytes >= 32 ? 2 * QS : QS);
     while (q < 4 * QS && pow2ceil((m + q - 1) / q) > 1024) q *= 2;
     const uint32_t gs = pow2ceil((m + q - 1) / q);
-    if (q == QS) return dispatch_gs<L, VEC, OP, QS>(a, b, r, carry, n, m, gs, st);
-    if (q == 2 * QS) return dispatch_gs<L, VEC, OP, 2 * QS>(a, b, r, carry, n, m, gs, st);
-    return dispatch_gs<L, VEC, OP, 4 * QS>(a, b, r, carry, n, m, gs, st);
+    if (q == QS) return dispatch_gs<L, true, OP, QS>(a, b, r, carry, n, m, gs, st);
+    if (q == 2 * QS) return dispatch_gs<L, true, OP, 2 * QS>(a, b, r, carry, n, m, gs, st);
+    return dispatch_gs<L, true, OP, 4 * QS>(a, b, r, carry, n, m, gs, st);
+}
+
+// k_add_rows, all others: four rows per thread (two leave too little in
+// flight, 65 limbs 45.2 us against 30.5 per 2^23 limbs; eight, too few warps,
+// 1001 limbs 35.5 against 29.9), two for up to 4 u64 limbs (38.4 against 51.2
+// for one) and for 25 to 32 (rows of 16 lanes instead of 8: 31.4 against 33.7),
+// eight where four would need a block of 1024 threads (4095 limbs 38.6
+// against 50.1).
+template <typename L, int OP>
+mi_status dispatch_rows(const L* a, const L* b, L* r, uint8_t* carry, uint32_t n, uint32_t m, cudaStream_t st) {
+    const bool two = sizeof(L) == 8 && (m <= 4 || (m > 24 && m <= 32));
+    const uint32_t q = two ? 2 : pow2ceil((m + 3) / 4) > 512 ? 8 : 4;
+    const uint32_t gs = pow2ceil((m + q - 1) / q);
+    if (q == 2) return dispatch_gs<L, false, OP, 2>(a, b, r, carry, n, m, gs, st);
+    if (q == 4) return dispatch_gs<L, false, OP, 4>(a, b, r, carry, n, m, gs, st);
+    return dispatch_gs<L, false, OP, 8>(a, b, r, carry, n, m, gs, st);
 }
 
 }  // namespace
@@ -582,12 +704,11 @@ mi_status launch_add_u64(const uint64_t* a, const uint64_t* b, uint64_t* r, uint
         return vec ? launch_wide<uint64_t, true, ADD_PLAIN>(a, b, r, carry, n, limbs, *wide, st)
                    : launch_wide<uint64_t, false, ADD_PLAIN>(a, b, r, carry, n, limbs, *wide, st);
     }
-    if (op == ADD_SIX) {
-        return vec ? dispatch<uint64_t, true, ADD_SIX>(a, b, r, nullptr, n, limbs, thread_bytes, st)
-                   : dispatch<uint64_t, false, ADD_SIX>(a, b, r, nullptr, n, limbs, thread_bytes, st);
-    }
-    return vec ? dispatch<uint64_t, true, ADD_PLAIN>(a, b, r, carry, n, limbs, thread_bytes, st)
-               : dispatch<uint64_t, false, ADD_PLAIN>(a, b, r, carry, n, limbs, thread_bytes, st);
+    if (op == ADD_SIX)
+        return vec ? dispatch_vec<uint64_t, ADD_SIX>(a, b, r, nullptr, n, limbs, thread_bytes, st)
+                   : dispatch_rows<uint64_t, ADD_SIX>(a, b, r, nullptr, n, limbs, st);
+    return vec ? dispatch_vec<uint64_t, ADD_PLAIN>(a, b, r, carry, n, limbs, thread_bytes, st)
+               : dispatch_rows<uint64_t, ADD_PLAIN>(a, b, r, carry, n, limbs, st);
 }
 
 mi_status launch_add_u32(const uint32_t* a, const uint32_t* b, uint32_t* r, uint8_t* carry, uint32_t n,
@@ -603,7 +724,7 @@ mi_status launch_add_u32(const uint32_t* a, const uint32_t* b, uint32_t* r, uint
         return launch_wide<uint32_t, false, ADD_PLAIN>(a, b, r, carry, n, limbs, *wide, st);
     }
     // Odd limb counts (or 4-byte aligned rows) cannot use 128-bit accesses.
-    return dispatch<uint32_t, false, ADD_PLAIN>(a, b, r, carry, n, limbs, thread_bytes, st);
+    return dispatch_rows<uint32_t, ADD_PLAIN>(a, b, r, carry, n, limbs, st);
 }
 
 }  // namespace mi

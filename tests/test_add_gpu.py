@@ -178,3 +178,29 @@ def test_tuning_rejects_bad_values(ctx):
     ctx.set_tuning(midint.TUNE_PLAIN_NTT_MIN, 0, 1025)
     assert ctx.get_tuning(midint.TUNE_PLAIN_NTT_MIN) == 1025
     ctx.set_tuning(midint.TUNE_PLAIN_NTT_MIN, 0, old)
+
+
+@pytest.mark.parametrize("bits", [64, 32])
+@pytest.mark.parametrize("m", [1, 3, 5, 9, 23, 25, 31, 33, 63, 65, 127, 129, 257, 1001, 2047, 2049, 4095, 8191])
+def test_add_rows_of_odd_lengths(ctx, devmem, m, bits):
+    # rows that allow no 16-byte access: every group width and rows-per-thread
+    # choice, plain (separate, in place, with carries) and 6a + 10b
+    if bits == 64 and m > 4096:
+        pytest.skip("the multi-block kernel")
+    n = 700 if m < 300 else 37
+    a, b = carry_stress(n, m, seed=m + bits, dtype=np.uint64 if bits == 64 else np.uint32)
+    want, carry = O.add(a, b, m)
+    words = a.view(np.uint32).size
+    s = torch.cuda.current_stream().cuda_stream
+    for inplace in (False, True):
+        (ba, pa), (bb, pb), (br, pr) = devmem.put(a), devmem.put(b), devmem.empty_words(words)
+        dc = torch.full((n + 8,), 7, dtype=torch.uint8, device="cuda:0")
+        ctx.add(pa, pb, pb if inplace else pr, n, m, carry=dc.data_ptr(), limb_bits=bits, stream=s)
+        torch.cuda.synchronize()
+        assert np.array_equal(devmem.get(bb if inplace else br, words, 0, a.dtype), want)
+        assert np.array_equal(dc.cpu().numpy()[:n], carry) and (dc.cpu().numpy()[n:] == 7).all()
+        if bits == 64:
+            (ba, pa), (bb, pb) = devmem.put(a), devmem.put(b)
+            ctx.add6(pa, pb, pa if inplace else pr, n, m, stream=s)
+            torch.cuda.synchronize()
+            assert np.array_equal(devmem.get(ba if inplace else br, words), O.add6(a, b, m))

@@ -661,8 +661,14 @@ mi_status mi_poly_u64(mi_ctx ctx, const uint64_t* a, const uint64_t* b, uint64_t
     if (n == 0) return MI_OK;
     MI_TRY(check_ctx(ctx));
     // from the tuned crossover on, the four products run on transforms (the
-    // reference's polyFttKer); below it, the classical form (polyKerQ)
-    if (limbs >= ctx->poly_ntt_min && aligned8(a) && aligned8(b) && aligned8(r))
+    // reference's polyFttKer); below it, the classical form (polyKerQ).  The
+    // crossover is measured on batches that fill the GPU: up to eight instances
+    // per SM, whose time is the latency of one, the transforms are faster from a
+    // quarter of it on (100 x 80 limbs 28.3 us classical against 22.5, 300 x 128
+    // 40.9 against 26.7, 1000 x 80 28.5 against 26.7, 1000 x 64 24.0 against 26.7)
+    uint32_t ntt_min = ctx->poly_ntt_min;
+    if (ntt_min <= kNttMaxLimbs && n <= 8 * uint32_t(sm_count())) ntt_min /= 4;
+    if (limbs >= ntt_min && aligned8(a) && aligned8(b) && aligned8(r))
         return launch_poly_ntt(a, b, r, n, limbs, ctx->ntt.params, pick_stream(ctx, stream));
     return launch_poly(reinterpret_cast<const uint32_t*>(a), reinterpret_cast<const uint32_t*>(b),
                        reinterpret_cast<uint32_t*>(r), n, 2 * limbs, pick_stream(ctx, stream));

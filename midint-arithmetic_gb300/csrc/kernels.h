@@ -52,9 +52,10 @@ mi_status launch_mul_classic(const uint32_t* a, const uint32_t* b, uint32_t* r, 
                              bool full, cudaStream_t st, uint32_t max_per_sm = 0);
 
 // The same, full or low half, on groups of any number of lanes (mul_flex.cu):
-// flex_rounds says with how many rounds (1..3), or 0 where the power-of-two
-// groups are faster or hold the product alone.
-uint32_t flex_rounds(uint32_t n, uint32_t n32, bool full);
+// flex_rounds says with how many rounds (1..max_rounds), or 0 where the
+// power-of-two groups are faster or hold the product alone; below `few` warps
+// per SM those lose on their launch shape.
+uint32_t flex_rounds(uint32_t n, uint32_t n32, bool full, uint32_t max_rounds = 3, uint32_t few = 16);
 mi_status launch_mul_flex(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32, bool full,
                           uint32_t rounds, cudaStream_t st);
 

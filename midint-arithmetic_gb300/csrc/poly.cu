@@ -3,6 +3,7 @@
 // four low-half products (classic::low_product) and three sums in one kernel.
 #include <cstdio>
 
+#include "mul_flex.cuh"
 #include "mul_lo.cuh"
 
 namespace mi {
@@ -142,21 +143,79 @@ __global__ void __launch_bounds__(NH > 256 ? NH : 256, 2)
     }
 }
 
+// The same on groups of any number of lanes of a warp (mul_flex.cuh), one
+// round of anti-diagonals per product.  A group stages a and b, and the rows of
+// each product's output blocks go back into shared memory as the next operand:
+// P3 = ab into a place of its own, T1 = a^2 + b over a, T2 = b^2 + b over b
+// (block by block, after the addend has been read), and r = T1 T2 + P3 into
+// the result row.  Limbs of the intermediates past n32 only reach limbs past
+// n32.  Against the power-of-two groups in blocks of 256 threads: 200 x 16
+// limbs 37.8 -> 10.8 us, 100000 x 6 98 -> 24, 5000 x 80 100 -> 68, 20 x 250
+// 99 -> 74; those keep the batches that fill the GPU with products of 25 to 32
+// and 33 to 64 blocks (4000 x 100 limbs 79.6 us against 82.1).
+template <bool VEC>
+__global__ void __launch_bounds__(32, 16)
+    k_poly_flex(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b, uint32_t* __restrict__ r, uint32_t n,
+                uint32_t n32, FlexShape S) {
+    extern __shared__ __align__(16) uint32_t smem[];
+    const flex::Place L(S);
+    const uint32_t half = S.nb + 1, num = 2 * half;
+    uint4* x = reinterpret_cast<uint4*>(smem + L.grp * S.stride);  // a, then T1
+    uint4* y = x + num;                                            // b, then T2
+    uint4* z = y + num;                                            // ab
+    uint2* slots = reinterpret_cast<uint2*>(smem + S.groups * S.stride);
+    const uint64_t inst = uint64_t(blockIdx.x) * S.groups + L.grp;
+    const bool valid = !L.idle && inst < n;
+    const uint64_t off = valid ? inst * n32 : 0;
+    pdl_wait();  // launched with launch_pdl
+    pdl_trigger();
+    if (!L.idle) flex::stage<VEC, 2>({x, y}, {a + off, b + off}, n32, valid, S, L.t);
+    __syncwarp();
+#pragma unroll 1
+    for (int p = 0; p < 4; ++p) {  // ab, a^2 + b, b^2 + b, T1 T2 + ab
+        flex::rounds<false>(p == 2 ? y : x, p == 1 ? x : y, slots + threadIdx.x, S, L.t);
+        __syncwarp();
+        uint4* to = p == 0 ? z : p == 1 ? x : y;
+        flex::rows<false>(slots + L.base, p == 0 ? nullptr : p == 3 ? z : y, S, L,
+                          [&](uint32_t q, const uint32_t (&v)[T]) {
+                              if (p < 3) {
+                                  to[q] = make_uint4(v[0], v[1], v[2], v[3]);
+                                  to[half + q] = make_uint4(v[4], v[5], v[6], v[7]);
+                              } else if (valid) {
+                                  classic::store_block<VEC>(r + off, q * T, n32, v);
+                              }
+                          });
+        __syncwarp();
+    }
+}
+
+mi_status launch_poly_flex(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32,
+                           uint32_t rounds, cudaStream_t st) {
+    const bool vec = aligned16(a) && aligned16(b) && aligned16(r) && (n32 % 4 == 0);
+    const FlexShape S = flex_shape(n32, false, rounds, 3);
+    auto kern = vec ? k_poly_flex<true> : k_poly_flex<false>;
+    MI_TRY(ensure_dyn_smem(kern, S.smem()));
+    const uint64_t blocks = (uint64_t(n) + S.groups - 1) / S.groups;
+    MI_CUDA_TRY(launch_pdl(kern, dim3(uint32_t(blocks)), dim3(32), S.smem(), st, a, b, r, n, n32, S));
+    return MI_OK;
+}
+
 template <bool VEC>
 mi_status dispatch(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32, cudaStream_t st) {
     switch (lo_threads(n32)) {
 #define MI_LO_CASE(NH) \
     case NH: return launch_lo<NH>(k_poly<NH, VEC>, a, b, r, n, n32, st);
-        MI_LO_CASE(1) MI_LO_CASE(2) MI_LO_CASE(4) MI_LO_CASE(8) MI_LO_CASE(16) MI_LO_CASE(32) MI_LO_CASE(64)
-        MI_LO_CASE(128) MI_LO_CASE(256)
+        MI_LO_CASE(16) MI_LO_CASE(32) MI_LO_CASE(64) MI_LO_CASE(128) MI_LO_CASE(256)
 #undef MI_LO_CASE
-        default: return set_error(MI_EINVAL, "poly: %u u32 limbs exceeds the classical maximum", n32);
+        default: return set_error(MI_EINVAL, "poly: %u u32 limbs outside the range of the power-of-two groups", n32);
     }
 }
 
 }  // namespace
 
 mi_status launch_poly(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32, cudaStream_t st) {
+    const uint32_t rounds = flex_rounds(n, n32, false, 1, 8);  // (3000 x 100 limbs 79.5 us without, 82 with)
+    if (rounds != 0) return launch_poly_flex(a, b, r, n, n32, rounds, st);
     const bool vec = aligned16(a) && aligned16(b) && aligned16(r) && (n32 % 4 == 0);
     return vec ? dispatch<true>(a, b, r, n, n32, st) : dispatch<false>(a, b, r, n, n32, st);
 }

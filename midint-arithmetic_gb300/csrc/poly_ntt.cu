@@ -195,6 +195,8 @@ __global__ void __launch_bounds__((1 << LG) / 8, LG == 12 ? 1 : (LG == 8 ? 512 :
     // exchange of two arrays: two buffers, or one and the last prime's residues
     uint32_t* const sh = smem32 + S::SH;
     constexpr int GAP = S::NX > 1 ? Pl::LX : S::RES + 3 * HALF * (NP - 1);  // of the second buffer
+    pdl_wait();  // small batches are launched with launch_pdl
+    pdl_trigger();
     for (uint64_t inst = blockIdx.x; inst < n; inst += gridDim.x) {
         const uint64_t* ai = a + inst * m;
         const uint64_t* bi = b + inst * m;
@@ -288,6 +290,10 @@ mi_status launch_lg(const uint64_t* a, const uint64_t* b, uint64_t* r, uint32_t 
     MI_TRY(site.get(kern, NT, smem, &per_sm));
     uint64_t blocks = uint64_t(sm_count()) * uint64_t(per_sm);
     if (blocks > n) blocks = n;
+    if (n <= 2 * uint32_t(sm_count())) {  // as the products do (ntt_mul.cu)
+        MI_CUDA_TRY(launch_pdl(kern, dim3(uint32_t(blocks)), dim3(NT), smem, st, a, b, r, n, m, P));
+        return MI_OK;
+    }
     kern<<<dim3(uint32_t(blocks)), dim3(NT), smem, st>>>(a, b, r, n, m, P);
     MI_CUDA_TRY(cudaGetLastError());
     return MI_OK;

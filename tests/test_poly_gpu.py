@@ -120,3 +120,24 @@ def test_poly_ntt_several_instances_per_block(ctx, devmem, n, m):
         assert np.array_equal(gpu_poly(ctx, devmem, a, b, m), O.poly(a, b, m))
     finally:
         ctx.set_tuning(midint.TUNE_POLY_NTT_MIN, 0, old)
+
+
+@pytest.mark.parametrize("m", [1, 4, 6, 11, 12, 20, 35, 63, 64, 65, 68, 80, 81, 96, 100, 127, 128, 130, 200, 255])
+def test_poly_lane_groups_and_batch_sizes(ctx, devmem, m):
+    # one to sixteen instances per warp, several block counts, on either side
+    # of the batch size that sends the composite to the transforms, classical
+    # throughout as well; odd rows
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    big = 8 * sms + 1 if m <= 130 else 300
+    a, b = carry_stress(big, m, seed=m + 2)
+    want = O.poly(a, b, m)
+    old = ctx.get_tuning(midint.TUNE_POLY_NTT_MIN)
+    try:
+        for knob in (old, 2049):
+            ctx.set_tuning(midint.TUNE_POLY_NTT_MIN, 0, knob)
+            for n in (1, 7, 8 * sms, big):
+                if n <= big:
+                    got = gpu_poly(ctx, devmem, a[:n * m], b[:n * m], m, offset=n % 3)
+                    assert np.array_equal(got, want[:n * m]), (n, knob)
+    finally:
+        ctx.set_tuning(midint.TUNE_POLY_NTT_MIN, 0, old)

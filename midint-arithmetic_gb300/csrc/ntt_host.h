@@ -20,14 +20,15 @@ constexpr NttPrime30 kNttPrimes[5] = {
     {1012924417u, 5u}, {1004535809u, 3u}, {998244353u, 3u}, {985661441u, 3u}, {975175681u, 17u},
 };
 
-// Kernel parameter block (passed by value).  Constants with a Shoup
-// companion are (c, floor(c 2^32 / p)) pairs.
+// Kernel parameter block (passed by value).  Constants are Shoup pairs (c,
+// floor(c 2^32 / p)) unless called plain.
 struct NttMulParams {
     uint32_t p[5];
     uint32_t pinv[5];             // -p^-1 mod 2^32
     uint2 ka_by_lg[5][5][2];      // for L = 2^(8+i): (L^-1, 2^32 L^-1) mod p
-    uint2 kb[5][2];               // (2^32, 2^64) mod p
-    uint2 kb_by_lg[5][5];         // for L = 2^(8+i): 2^64 L^-1 mod p (with ka_by_lg[..][1], b's conversion)
+    uint2 c32[5];                 // 2^32 mod p: a's conversion
+    uint2 ka[5];                  // (2^32, 2^64) mod p, plain: the composite's conversions
+    uint2 kb_by_lg[5][5];         // for L = 2^(8+i): (2^64 L^-1, 2^96 L^-1) mod p, plain: b's conversion
     uint2 garner[10];             // p_k^-1 mod p_i, for i = 1..4, k = 0..i-1
     const uint2* tw[5];           // (w^e, companion), w of order 4096, in ntt32::TwLayout order
     const uint2* itw[5];          // (w^-e, companion), the same layout

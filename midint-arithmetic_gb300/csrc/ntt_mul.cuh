@@ -46,20 +46,6 @@ struct MulSmem {
     static constexpr size_t WORDS32 = size_t(2) * Plan<LG>::LX + size_t(5) * L;
 };
 
-// x*K mod p in [0, 2p) for a digit x < 2^64: K0 = K mod p, K1 = 2^32 K mod p
-// (Shoup pairs).
-__device__ __forceinline__ uint32_t convert(uint64_t x, const Field& f, uint2 k0, uint2 k1) {
-    return f.add(f.shoup(uint32_t(x), k0), f.shoup(uint32_t(x >> 32), k1));
-}
-
-// x mod p in [0, 2p) for a digit x = lo + hi 2^32 < 2^64, c32 the Shoup pair
-// of 2^32 mod p: lo is brought below 2p by two conditional subtractions of 2p
-// (lo < 2^32 < 6p), hi 2^32 by one Shoup product -- one product instead of
-// the two of convert() for the operand that takes no scaling.
-__device__ __forceinline__ uint32_t reduce_digit(uint32_t lo, uint32_t hi, const Field& f, uint2 c32) {
-    return f.add(f.reduce2(f.reduce2(lo)), f.shoup(hi, c32));
-}
-
 // Digit modes (see the top of this file).
 enum : int { DM64 = 0, DM48 = 1, DM40 = 2 };
 template <int DM>
@@ -67,7 +53,7 @@ struct Digits {
     static constexpr int NP = 5 - DM;                              // primes
     static constexpr int BITS = DM == DM64 ? 64 : (DM == DM48 ? 48 : 40);
     static constexpr int OUT = BITS / 8;                           // output limbs per thread (8 digits)
-    static constexpr int OVW = DM == DM64 ? 3 : (DM == DM48 ? 2 : 1);  // words overflowing to the next thread
+    static constexpr int OVW = DM == DM40 ? 1 : 2;                 // words overflowing to the next thread
 };
 // The largest digit count of the shorter operand for which 40-bit digits on
 // three primes stay exact: 840 (2^40 - 1)^2 < p0 p1 p2 <= 841 (2^40 - 1)^2.
@@ -117,27 +103,101 @@ __device__ __forceinline__ uint2 digit_at(const uint64_t* __restrict__ row, uint
     return make_uint2(uint32_t(v), uint32_t(v >> 32));
 }
 
-// s[w..) += (x0, x1, x2) (u64 words, little-endian), carries rippling to s[SW-1].
-template <int SW>
-__device__ __forceinline__ void add3_at(uint64_t (&s)[SW], int w, uint64_t x0, uint64_t x1, uint64_t x2) {
-    unsigned __int128 a = (unsigned __int128)s[w] + x0;
-    s[w] = (uint64_t)a;
-    a = (unsigned __int128)s[w + 1] + x1 + (uint64_t)(a >> 64);
-    s[w + 1] = (uint64_t)a;
-    a = (unsigned __int128)s[w + 2] + x2 + (uint64_t)(a >> 64);
-    s[w + 2] = (uint64_t)a;
+// The sum of a thread's 8 coefficients at their digits, taken in order: each
+// coefficient (NP words) plus what the ones before it left above its digit
+// gives one digit and what is left above it -- a chain of NP adds per
+// coefficient (adding each at its place into an 11-word sum rippled its carry
+// through all the words above).
+template <int DM>
+struct DigitSum {
+    static constexpr int NP = Digits<DM>::NP, OUT = Digits<DM>::OUT, OVW = Digits<DM>::OVW;
+    uint32_t w[2 * OUT], c[3], rem;
+    __device__ __forceinline__ DigitSum() : c{0u, 0u, 0u}, rem(0u) {}
+    // the coefficient of digit o = 0, 1, ... (a constant after unrolling)
+    __device__ __forceinline__ void add(int o, const uint32_t* v) {
+        uint32_t t[5] = {v[0], v[1], v[2], NP > 3 ? v[3] : 0u, NP > 4 ? v[4] : 0u};
+        add_cc(t[0], c[0]);
+        addc_cc(t[1], c[1]);
+        if constexpr (NP == 3) {
+            addc(t[2], c[2]);
+        } else {
+            addc_cc(t[2], c[2]);
+            if constexpr (NP > 4) {
+                addc_cc(t[3], 0u);
+                addc(t[4], 0u);
+            } else {
+                addc(t[3], 0u);
+            }
+        }
+        if constexpr (DM == DM64) {  // t < 2^150
+            w[2 * o] = t[0];
+            w[2 * o + 1] = t[1];
+            c[0] = t[2], c[1] = t[3], c[2] = t[4];
+        } else if constexpr (DM == DM48) {  // t < 2^121
+            c[0] = __funnelshift_r(t[1], t[2], 16);
+            c[1] = __funnelshift_r(t[2], t[3], 16);
+            c[2] = t[3] >> 16;
+            if (o % 2 == 0) {
+                w[o / 2 * 3] = t[0];
+                rem = t[1] & 0xffffu;
+            } else {
+                w[o / 2 * 3 + 1] = rem | (t[0] << 16);
+                w[o / 2 * 3 + 2] = __funnelshift_r(t[0], t[1], 16);
+            }
+        } else {  // t < 2^91
+            c[0] = __funnelshift_r(t[1], t[2], 8);
+            c[1] = t[2] >> 8;
+            const int k = o % 4, b = o / 4 * 5;  // four digits make five words
+            const uint32_t top = t[1] & 0xffu;
+            w[b + k] = k == 0 ? t[0] : rem | (t[0] << (8 * k));
+            rem = k == 0 ? top : (t[0] >> (32 - 8 * k)) | (top << (8 * k));
+            if (k == 3) w[b + 4] = rem;
+        }
+    }
+    // the OUT limbs and the OVW words above them
+    __device__ __forceinline__ void get(uint64_t (&s)[OUT + OVW]) const {
 #pragma unroll
-    for (int k = w + 3; k < SW; ++k) {
-        a = (unsigned __int128)s[k] + (uint64_t)(a >> 64);
-        s[k] = (uint64_t)a;
+        for (int i = 0; i < OUT; ++i) s[i] = uint64_t(w[2 * i]) | (uint64_t(w[2 * i + 1]) << 32);
+        s[OUT] = uint64_t(c[0]) | (uint64_t(c[1]) << 32);
+        if constexpr (OVW > 1) s[OUT + 1] = c[2];
+    }
+};
+
+// Garner's mixed-radix digits of a coefficient from its residues y (in place),
+// then its value in NP words: y0 = r0, y_i = (...((r_i - y0) c_0i - y1) c_1i ...
+// - y_(i-1)) c_(i-1)i mod p_i with c_ji = p_j^-1 mod p_i; x = y0 + p0 (y1 + p1
+// (y2 + ...)), below the product of the NP primes (2^150, 2^120 or 2^90), by
+// Horner in 32-bit words.
+template <int NP>
+__device__ __forceinline__ void garner(uint32_t (&y)[NP], const NttMulParams& P, uint32_t (&acc)[5]) {
+    int c = 0;
+#pragma unroll
+    for (int i = 1; i < NP; ++i) {
+        const Field fi{P.p[i], 2 * P.p[i], 0u};
+        uint32_t v = y[i];
+#pragma unroll
+        for (int k = 0; k < i; ++k) v = fi.shoup(v + fi.p2 - y[k], P.garner[c++]);
+        y[i] = fi.reduce(v);
+    }
+    acc[0] = y[NP - 1], acc[1] = acc[2] = acc[3] = acc[4] = 0u;
+#pragma unroll
+    for (int i = NP - 2; i >= 0; --i) {
+        uint64_t carry = y[i];
+#pragma unroll
+        for (int w = 0; w < NP - 1 - i; ++w) {
+            const uint64_t tt = uint64_t(acc[w]) * P.p[i] + carry;
+            acc[w] = uint32_t(tt);
+            carry = tt >> 32;
+        }
+        acc[NP - 1 - i] = uint32_t(carry);
     }
 }
 
 // The thread's block of OUT output limbs from its digit sums s (OUT + OVW
 // words, the top OVW overflowing into the right neighbour), carried over the
 // group, stored to rr[OUT t ..) below rlen.
-template <int NT, int OUT, int OVW, int SW>
-__device__ __forceinline__ void finish_block(const uint64_t (&s)[SW], uint64_t* ov, uint64_t* __restrict__ rr,
+template <int NT, int OUT, int OVW>
+__device__ __forceinline__ void finish_block(const uint64_t (&s)[OUT + OVW], uint64_t* ov, uint64_t* __restrict__ rr,
                                              uint32_t rlen, uint32_t t, uint32_t* scr) {
 #pragma unroll
     for (int w = 0; w < OVW; ++w) ov[OVW * t + w] = s[OUT + w];
@@ -179,8 +239,7 @@ __device__ __forceinline__ void mul_residues(const uint64_t* __restrict__ ar, ui
     const Field f{P.p[q], 2 * P.p[q], P.pinv[q]};
     // a unscaled; b times 2^32 / L (the Montgomery pointwise product takes
     // out 2^32, and the inverse transform needs no 1/L pass)
-    const uint2 c32 = P.kb[q][0];
-    const uint2 kb0 = P.ka_by_lg[q][LG - 8][1], kb1 = P.kb_by_lg[q][LG - 8];
+    const uint2 c32 = P.c32[q], kb = P.kb_by_lg[q][LG - 8];
     uint32_t x[2][8];  // a and b, transformed in lockstep
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -189,16 +248,9 @@ __device__ __forceinline__ void mul_residues(const uint64_t* __restrict__ ar, ui
             x[0][j] = x[1][j] = 0u;
             continue;
         }
-        if constexpr (DM == DM64) {
-            const uint64_t da = i < la ? __ldg(ar + i) : 0ull;
-            x[0][j] = reduce_digit(uint32_t(da), uint32_t(da >> 32), f, c32);
-            x[1][j] = (i < lb) ? convert(__ldg(br + i), f, kb0, kb1) : 0u;
-        } else {
-            const uint2 da = digit_at<DM>(ar, la, i);
-            const uint2 db = digit_at<DM>(br, lb, i);
-            x[0][j] = reduce_digit(da.x, da.y, f, c32);
-            x[1][j] = f.add(f.shoup(db.x, kb0), f.shoup(db.y, kb1));
-        }
+        const uint2 da = digit_at<DM>(ar, la, i), db = digit_at<DM>(br, lb, i);
+        x[0][j] = f.plain_digit(da.x, da.y, c32);
+        x[1][j] = f.digit(db.x, db.y, kb);
     }
     forward<LG, 2, HALF>(x, sh, P.tw[q], f);
 #pragma unroll
@@ -210,67 +262,33 @@ __device__ __forceinline__ void mul_residues(const uint64_t* __restrict__ ar, ui
 
 // The product's limbs r[0..rlen) from the residues of all its coefficients
 // (res[q L + swz(i)], visible to the group): Garner, digit sums, carries.
-// `ov` is scratch of 3 x 8 bytes per thread, free by the call.
+// `ov` is scratch of OVW x 8 bytes per thread, free by the call.
 template <int LG, int DM, bool LOW>
 __device__ __forceinline__ void mul_recombine(const uint32_t* res, uint64_t* __restrict__ rr, uint32_t rlen,
                                               const NttMulParams& P, uint64_t* ov, uint32_t* scr) {
     using Pl = Plan<LG>;
     using Dg = Digits<DM>;
     constexpr int NP = Dg::NP;
-    constexpr int SW = 11;  // digit-sum words: 8 limbs + 3 overflow, 6 + 2 or 5 + 1 (+ headroom)
     const uint32_t t = threadIdx.x % Pl::NT;
-    // Garner: y0 = r0, y_i = (...((r_i - y0) c_0i - y1) c_1i ... - y_(i-1)) c_(i-1)i
-    // mod p_i with c_ji = p_j^-1 mod p_i; x = y0 + p0 (y1 + p1 (y2 + ...)),
-    // below the product of the NP primes (2^150, 2^120 or 2^90), evaluated in
-    // 32-bit words (Horner).
-    uint64_t s[SW];
+    DigitSum<DM> sum;
+    uint64_t s[Dg::OUT + Dg::OVW];
+    if (LOW && 8 * t >= Pl::L / 2) {  // coefficients that reach no stored limb
 #pragma unroll
-    for (int w = 0; w < SW; ++w) s[w] = 0;
+        for (int w = 0; w < Dg::OUT + Dg::OVW; ++w) s[w] = 0;
+    } else {
 #pragma unroll
-    for (int j = 0; j < 8; j += 4) {
-        if (LOW && 8 * t >= Pl::L / 2) break;  // coefficients that reach no stored limb
-        const uint32_t slot = swz(8 * t + j);  // the swizzle keeps the quad slot..slot+3 together
+        for (int j = 0; j < 8; j += 4) {
+            const uint32_t slot = swz(8 * t + j);  // the swizzle keeps the quad slot..slot+3 together
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
-            uint32_t y[NP];
+            for (int h = 0; h < 4; ++h) {
+                uint32_t y[NP], acc[5];
 #pragma unroll
-            for (int q = 0; q < NP; ++q) y[q] = res[q * Pl::L + slot + h];
-            int c = 0;
-#pragma unroll
-            for (int i = 1; i < NP; ++i) {
-                const Field fi{P.p[i], 2 * P.p[i], 0u};
-                uint32_t v = y[i];
-#pragma unroll
-                for (int k = 0; k < i; ++k) v = fi.shoup(v + fi.p2 - y[k], P.garner[c++]);
-                y[i] = fi.reduce(v);
-            }
-            // Horner in 32-bit words: acc = y_(NP-1); acc = acc * p_i + y_i, i = NP-2..0
-            uint32_t acc[kPrimes] = {y[NP - 1], 0u, 0u, 0u, 0u};
-#pragma unroll
-            for (int i = NP - 2; i >= 0; --i) {
-                uint64_t carry = y[i];
-#pragma unroll
-                for (int w = 0; w < NP - 1 - i; ++w) {
-                    const uint64_t tt = uint64_t(acc[w]) * P.p[i] + carry;
-                    acc[w] = uint32_t(tt);
-                    carry = tt >> 32;
-                }
-                acc[NP - 1 - i] = uint32_t(carry);
-            }
-            const uint64_t w0 = uint64_t(acc[0]) | (uint64_t(acc[1]) << 32);
-            const uint64_t w1 = uint64_t(acc[2]) | (uint64_t(acc[3]) << 32);
-            const int o = j + h;  // the coefficient's digit within the thread's block of 8
-            if constexpr (DM == DM64) {
-                add3_at<SW>(s, o, w0, w1, uint64_t(acc[4]));
-            } else {
-                // a value below 2^120 (2^90) at bit BITS*o of the thread's block
-                const int bit = Dg::BITS * o, w = bit >> 6, b = bit & 63;
-                const uint64_t x0 = w0 << b;
-                const uint64_t x1 = b ? (w1 << b) | (w0 >> (64 - b)) : w1;
-                const uint64_t x2 = b ? w1 >> (64 - b) : 0ull;
-                add3_at<SW>(s, w, x0, x1, x2);
+                for (int q = 0; q < NP; ++q) y[q] = res[q * Pl::L + slot + h];
+                garner<NP>(y, P, acc);
+                sum.add(j + h, acc);
             }
         }
+        sum.get(s);
     }
     // the overflow words go to the right neighbour through ov
     finish_block<Pl::NT, Dg::OUT, Dg::OVW>(s, ov, rr, rlen, t, scr);
@@ -305,7 +323,7 @@ __device__ __forceinline__ void mul_one(const uint64_t* __restrict__ ar, uint32_
         for (int j = 0; j < (LOW ? 4 : 8); ++j) res[q * Pl::L + swz(t + Pl::NT * j)] = x[j];
     }
     __syncthreads();
-    // the overflow words take the exchange buffers: 3 x 8 bytes x L/8 threads fit their 9L bytes
+    // the overflow words take the exchange buffers: 2 x 8 bytes x L/8 threads fit their 9L bytes
     mul_recombine<LG, DM, LOW>(res, rr, rlen, P, reinterpret_cast<uint64_t*>(sh), scr);
     __syncthreads();  // sh and res are reused by the next call
 }

@@ -88,61 +88,29 @@ template <int LG, bool D48, typename FA, typename FP>
 __device__ __forceinline__ void recombine(const uint32_t* res, int stride, uint32_t m, const NttMulParams& P,
                                           uint32_t* sh, uint32_t* scr, FA addend, FP put) {
     using Pl = Plan<LG>;
-    constexpr int SW = 11;
-    constexpr int HALF = Pl::L / 2;
+    constexpr int HALF = Pl::L / 2, DM = D48 ? ntt32::DM48 : ntt32::DM64, NP = ntt32::Digits<DM>::NP;
+    constexpr int OUT = ntt32::Digits<DM>::OUT, OVW = ntt32::Digits<DM>::OVW, SW = OUT + OVW;
     const uint32_t t = threadIdx.x % Pl::NT;
     uint64_t s[SW];
 #pragma unroll
     for (int w = 0; w < SW; ++w) s[w] = 0;
     if (8 * t < HALF) {
+        ntt32::DigitSum<DM> sum;
 #pragma unroll
         for (int j = 0; j < 8; j += 4) {
             const uint32_t slot = ntt32::swz(8 * t + j);
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
-                uint32_t yv[ntt32::kPrimes];
+                uint32_t y[NP], acc[5];
 #pragma unroll
-                for (int q = 0; q < ntt32::kPrimes; ++q) yv[q] = (q < 4 || !D48) ? res[q * stride + slot + h] : 0u;
-                int c = 0;
-#pragma unroll
-                for (int i = 1; i < ntt32::kPrimes; ++i) {
-                    if (D48 && i == ntt32::kPrimes - 1) break;
-                    const Field fi{P.p[i], 2 * P.p[i], 0u};
-                    uint32_t v = yv[i];
-#pragma unroll
-                    for (int k = 0; k < i; ++k) v = fi.shoup(v + fi.p2 - yv[k], P.garner[c++]);
-                    yv[i] = fi.reduce(v);
-                }
-                if (D48) yv[ntt32::kPrimes - 1] = 0;
-                uint32_t acc[ntt32::kPrimes] = {yv[ntt32::kPrimes - 1], 0u, 0u, 0u, 0u};
-#pragma unroll
-                for (int i = ntt32::kPrimes - 2; i >= 0; --i) {
-                    uint64_t carry = yv[i];
-#pragma unroll
-                    for (int w = 0; w < ntt32::kPrimes - 1 - i; ++w) {
-                        const uint64_t tt = uint64_t(acc[w]) * P.p[i] + carry;
-                        acc[w] = uint32_t(tt);
-                        carry = tt >> 32;
-                    }
-                    acc[ntt32::kPrimes - 1 - i] = uint32_t(carry);
-                }
-                const uint64_t w0 = uint64_t(acc[0]) | (uint64_t(acc[1]) << 32);
-                const uint64_t w1 = uint64_t(acc[2]) | (uint64_t(acc[3]) << 32);
-                const int o = j + h;
-                if (!D48) {
-                    ntt32::add3_at<SW>(s, o, w0, w1, uint64_t(acc[4]));
-                } else {
-                    const int bit = 48 * o, w = bit >> 6, b = bit & 63;
-                    const uint64_t x0 = w0 << b;
-                    const uint64_t x1 = b ? (w1 << b) | (w0 >> (64 - b)) : w1;
-                    const uint64_t x2 = b ? w1 >> (64 - b) : 0ull;
-                    ntt32::add3_at<SW>(s, w, x0, x1, x2);
-                }
+                for (int q = 0; q < NP; ++q) y[q] = res[q * stride + slot + h];
+                ntt32::garner<NP>(y, P, acc);
+                sum.add(j + h, acc);
             }
         }
+        sum.get(s);
     }
     // the addend's limbs of the thread's block enter the digit sums
-    constexpr int OUT = D48 ? 6 : 8, OVW = D48 ? 2 : 3;
     const uint32_t o0 = OUT * t;
     {
         unsigned __int128 acc = 0;
@@ -204,7 +172,7 @@ __global__ void __launch_bounds__((1 << LG) / 8, LG == 12 ? 1 : (LG == 8 ? 512 :
 #pragma unroll 1
         for (int q = 0; q < NP; ++q) {
             const Field f{P.p[q], 2 * P.p[q], P.pinv[q]};
-            const uint2 c32 = P.kb[q][0], ks = P.ka_by_lg[q][LG - 8][1];
+            const uint2 ka = P.ka[q], ks = P.ka_by_lg[q][LG - 8][1];
             uint32_t v[2][8];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {  // m digits fit L/2: the upper halves are zero
@@ -212,8 +180,8 @@ __global__ void __launch_bounds__((1 << LG) / 8, LG == 12 ? 1 : (LG == 8 ? 512 :
                     [&](uint32_t w) { return __ldg(reinterpret_cast<const uint32_t*>(ai) + w); }, 2 * m, t + Pl::NT * j);
                 const uint2 db = digit_of<D48>(
                     [&](uint32_t w) { return __ldg(reinterpret_cast<const uint32_t*>(bi) + w); }, 2 * m, t + Pl::NT * j);
-                v[0][j] = ntt32::reduce_digit(da.x, da.y, f, c32);
-                v[1][j] = ntt32::reduce_digit(db.x, db.y, f, c32);
+                v[0][j] = f.digit(da.x, da.y, ka);
+                v[1][j] = f.digit(db.x, db.y, ka);
             }
             ntt32::forward<LG, 2, true, GAP>(v, sh, P.tw[q], f);
             uint32_t z[3][8];  // a^2, b^2, ab
@@ -256,15 +224,14 @@ __global__ void __launch_bounds__((1 << LG) / 8, LG == 12 ? 1 : (LG == 8 ? 512 :
         for (int q = 0; q < NP; ++q) {
             const Field f{P.p[q], 2 * P.p[q], P.pinv[q]};
             // T1 unscaled, T2 times 2^32 / L
-            const uint2 c32 = P.kb[q][0];
-            const uint2 kb0 = P.ka_by_lg[q][LG - 8][1], kb1 = P.kb_by_lg[q][LG - 8];
+            const uint2 ka = P.ka[q], kb = P.kb_by_lg[q][LG - 8];
             uint32_t v[2][8];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const uint2 d1 = digit_of<D48>([&](uint32_t w) { return res[mid_word<LG>(0, w)]; }, 2 * m, t + Pl::NT * j);
                 const uint2 d2 = digit_of<D48>([&](uint32_t w) { return res[mid_word<LG>(1, w)]; }, 2 * m, t + Pl::NT * j);
-                v[0][j] = ntt32::reduce_digit(d1.x, d1.y, f, c32);
-                v[1][j] = f.add(f.shoup(d2.x, kb0), f.shoup(d2.y, kb1));
+                v[0][j] = f.digit(d1.x, d1.y, ka);
+                v[1][j] = f.digit(d2.x, d2.y, kb);
             }
             ntt32::forward<LG, 2, true, GAP>(v, sh, P.tw[q], f);
 #pragma unroll

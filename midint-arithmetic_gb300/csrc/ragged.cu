@@ -323,6 +323,14 @@ __global__ void __launch_bounds__(256) k_scatter(uint32_t n, uint32_t* __restric
     }
 }
 
+// Task indices.  A block's (or warp's) first task is its own number, the later
+// ones come from the family's queue: the first round needs no atomic, and warp
+// w of block b takes task w * blocks + b, so that a short family spreads over
+// the SMs (popped, eight tasks at a time went to the eight warps of the blocks
+// that started first: 400 operations 41 us against 38, 4000 of them 70 against 53).
+__device__ __forceinline__ uint32_t first_task() { return (threadIdx.x >> 5) * gridDim.x + blockIdx.x; }
+__device__ __forceinline__ uint32_t warp_tasks() { return (blockDim.x >> 5) * gridDim.x; }
+
 // Task t of a family -> (key, index of its first op in `sorted`, op count).
 struct Task {
     uint32_t key, first, count;
@@ -376,7 +384,7 @@ __device__ __forceinline__ Task decode_tab(const FamTab& tab, uint32_t t) {
 // the kernels that follow (when every block waited, the blocks of a family
 // with few tasks held their registers until the previous family was done, and
 // the families of a short list ran one after another: 400 operations of 512 to
-// 32768 bits 87 us against RAGFIG).
+// 32768 bits 88 us against 53).
 __device__ __forceinline__ void pdl_join() {
     if (blockIdx.x == 0) pdl_wait();
 }
@@ -419,12 +427,12 @@ __global__ void __launch_bounds__(256, DM == ntt32::DM64 ? 3 : 2) k_rg_ntt(Param
     const uint32_t ntasks = P.scr[Scratch::NTASKS + F];
     pdl_trigger();  // the next family's kernel may start as this one's blocks finish
     load_tab(tab, P.scr, F);
-    if (threadIdx.x == 0) s_task[0] = atomicAdd(P.scr + Scratch::QUEUE + F, 1u);
+    if (threadIdx.x == 0) s_task[0] = blockIdx.x;
     __syncthreads();
     for (uint32_t it = 0;; ++it) {
         const uint32_t t = s_task[it & 1];
         if (t >= ntasks) break;
-        if (threadIdx.x == 0) s_task[(it + 1) & 1] = atomicAdd(P.scr + Scratch::QUEUE + F, 1u);
+        if (threadIdx.x == 0) s_task[(it + 1) & 1] = gridDim.x + atomicAdd(P.scr + Scratch::QUEUE + F, 1u);
         const Task tk = decode_tab<F>(tab, t);
         switch (tk.key - KEY0) {
             case 0: ntt_task<8, DM>(P, tk, smem, scr_warp); break;
@@ -867,13 +875,11 @@ __global__ void __launch_bounds__(256, 2) k_rg_classic(Params P) {
     pdl_trigger();
     load_tab(tab, P.scr, 1);
     __syncthreads();
-    // each warp fetches its next task index while the current task runs
-    uint32_t next = 0;
-    if (lane == 0) next = atomicAdd(P.scr + Scratch::QUEUE + 1, 1u);
+    uint32_t next = first_task();  // then fetched while the current task runs
     for (;;) {
         const uint32_t t = __shfl_sync(MI_FULL_MASK, next, 0);
         if (t >= ntasks) break;
-        if (lane == 0) next = atomicAdd(P.scr + Scratch::QUEUE + 1, 1u);
+        if (lane == 0) next = warp_tasks() + atomicAdd(P.scr + Scratch::QUEUE + 1, 1u);
         const Task tk = decode_tab<1>(tab, t);
         switch (tk.key - KEY_CLS) {
             case 0: classic_task<1>(P, tk, wsm, nullptr); break;
@@ -902,12 +908,11 @@ __global__ void __launch_bounds__(256, 2) k_rg_r32(Params P) {
     pdl_trigger();
     load_tab(tab, P.scr, 7);
     __syncthreads();
-    uint32_t next = 0;  // the next task index, fetched while the current task runs
-    if (lane == 0) next = atomicAdd(P.scr + Scratch::QUEUE + 7, 1u);
+    uint32_t next = first_task();  // then fetched while the current task runs
     for (;;) {
         const uint32_t t = __shfl_sync(MI_FULL_MASK, next, 0);
         if (t >= ntasks) break;
-        if (lane == 0) next = atomicAdd(P.scr + Scratch::QUEUE + 7, 1u);
+        if (lane == 0) next = warp_tasks() + atomicAdd(P.scr + Scratch::QUEUE + 7, 1u);
         rect32_task(P, decode_tab<7>(tab, t), wsm);
     }
     pdl_join();
@@ -923,12 +928,11 @@ __global__ void __launch_bounds__(256, 2) k_rg_comb(Params P) {
     pdl_trigger();
     load_tab(tab, P.scr, 5);
     __syncthreads();
-    uint32_t next = 0;  // the next task index, fetched while the current task runs
-    if (lane == 0) next = atomicAdd(P.scr + Scratch::QUEUE + 5, 1u);
+    uint32_t next = first_task();  // then fetched while the current task runs
     for (;;) {
         const uint32_t t = __shfl_sync(MI_FULL_MASK, next, 0);
         if (t >= ntasks) break;
-        if (lane == 0) next = atomicAdd(P.scr + Scratch::QUEUE + 5, 1u);
+        if (lane == 0) next = warp_tasks() + atomicAdd(P.scr + Scratch::QUEUE + 5, 1u);
         const Task tk = decode_tab<5>(tab, t);
         const uint32_t ki = tk.key - KEY_CMB;
         if (ki == 0) comb_task<4>(P, tk);
@@ -950,12 +954,12 @@ __global__ void __launch_bounds__(256, 2) k_rg_c64(Params P) {
     const uint32_t ntasks = P.scr[Scratch::NTASKS + 3];
     pdl_trigger();
     load_tab(tab, P.scr, 3);
-    if (threadIdx.x == 0) s_task[0] = atomicAdd(P.scr + Scratch::QUEUE + 3, 1u);
+    if (threadIdx.x == 0) s_task[0] = blockIdx.x;
     __syncthreads();
     for (uint32_t it = 0;; ++it) {
         const uint32_t t = s_task[it & 1];
         if (t >= ntasks) break;
-        if (threadIdx.x == 0) s_task[(it + 1) & 1] = atomicAdd(P.scr + Scratch::QUEUE + 3, 1u);
+        if (threadIdx.x == 0) s_task[(it + 1) & 1] = gridDim.x + atomicAdd(P.scr + Scratch::QUEUE + 3, 1u);
         classic_task<64>(P, decode_tab<3>(tab, t), smem32, scr_warp);
         __syncthreads();  // the next index is visible; shared memory is reused
     }
@@ -1079,12 +1083,11 @@ __global__ void __launch_bounds__(256, 3) k_rg_add(Params P) {
     pdl_trigger();
     load_tab(tab, P.scr, 2);
     __syncthreads();
-    uint32_t next = 0;  // the next task index, fetched while the current task runs
-    if (lane == 0) next = atomicAdd(P.scr + Scratch::QUEUE + 2, 1u);
+    uint32_t next = first_task();  // then fetched while the current task runs
     for (;;) {
         const uint32_t t = __shfl_sync(MI_FULL_MASK, next, 0);
         if (t >= ntasks) break;
-        if (lane == 0) next = atomicAdd(P.scr + Scratch::QUEUE + 2, 1u);
+        if (lane == 0) next = warp_tasks() + atomicAdd(P.scr + Scratch::QUEUE + 2, 1u);
         const Task tk = decode_tab<2>(tab, t);
         switch (tk.key - KEY_ADD) {
             case 0: add_short<1>(P, tk); break;

@@ -409,6 +409,19 @@ __device__ __forceinline__ void ntt_task(const Params& P, const Task& tk, uint32
         scr_warp);
 }
 
+// One task of an NTT family, by a block.
+template <int DM>
+__device__ __forceinline__ void ntt_block(const Params& P, const Task& tk, uint32_t* smem) {
+    constexpr int KEY0 = DM == ntt32::DM64 ? KEY_NTT : (DM == ntt32::DM48 ? KEY_N48 : KEY_N40);
+    uint32_t* scr_warp = smem + ntt32::MulSmem<11>::WORDS32;  // after the groups' shared memory
+    switch (tk.key - KEY0) {
+        case 0: ntt_task<8, DM>(P, tk, smem, scr_warp); break;
+        case 1: ntt_task<9, DM>(P, tk, smem, scr_warp); break;
+        case 2: ntt_task<10, DM>(P, tk, smem, scr_warp); break;
+        default: ntt_task<11, DM>(P, tk, smem, scr_warp); break;
+    }
+}
+
 // DM: the digit mode of the family (64-bit digits on five primes, 48-bit
 // on four, 40-bit on three: a kernel each, so that no digit mode's code
 // raises another's registers).  The 64-bit family runs three CTAs per SM at
@@ -418,9 +431,7 @@ __device__ __forceinline__ void ntt_task(const Params& P, const Task& tk, uint32
 template <int DM>
 __global__ void __launch_bounds__(256, DM == ntt32::DM64 ? 3 : 2) k_rg_ntt(Params P) {
     constexpr int F = DM == ntt32::DM64 ? 0 : (DM == ntt32::DM48 ? 4 : 6);  // family
-    constexpr int KEY0 = DM == ntt32::DM64 ? KEY_NTT : (DM == ntt32::DM48 ? KEY_N48 : KEY_N40);
     extern __shared__ __align__(16) uint32_t smem[];
-    uint32_t* scr_warp = smem + ntt32::MulSmem<11>::WORDS32;  // after the groups' shared memory
     __shared__ uint32_t s_task[2];  // this task and the next, fetched while this one runs
     __shared__ FamTab tab;
     if (DM == ntt32::DM64) pdl_wait();  // the first task kernel: the binning is complete
@@ -433,13 +444,7 @@ __global__ void __launch_bounds__(256, DM == ntt32::DM64 ? 3 : 2) k_rg_ntt(Param
         const uint32_t t = s_task[it & 1];
         if (t >= ntasks) break;
         if (threadIdx.x == 0) s_task[(it + 1) & 1] = gridDim.x + atomicAdd(P.scr + Scratch::QUEUE + F, 1u);
-        const Task tk = decode_tab<F>(tab, t);
-        switch (tk.key - KEY0) {
-            case 0: ntt_task<8, DM>(P, tk, smem, scr_warp); break;
-            case 1: ntt_task<9, DM>(P, tk, smem, scr_warp); break;
-            case 2: ntt_task<10, DM>(P, tk, smem, scr_warp); break;
-            default: ntt_task<11, DM>(P, tk, smem, scr_warp); break;
-        }
+        ntt_block<DM>(P, decode_tab<F>(tab, t), smem);
         __syncthreads();  // the next index is visible; this one is read by all
     }
     if (DM != ntt32::DM64) pdl_join();
@@ -866,6 +871,25 @@ __device__ __forceinline__ void comb_task(const Params& P, const Task& tk) {
     }
 }
 
+// One task of a family, by a warp (its area of shared memory, its descriptor
+// slots).
+__device__ __forceinline__ void classic_warp(const Params& P, const Task& tk, uint32_t* wsm) {
+    switch (tk.key - KEY_CLS) {
+        case 0: classic_task<1>(P, tk, wsm, nullptr); break;
+        case 1: classic_task<2>(P, tk, wsm, nullptr); break;
+        case 2: classic_task<4>(P, tk, wsm, nullptr); break;
+        case 3: classic_task<8>(P, tk, wsm, nullptr); break;
+        default: classic_task<16>(P, tk, wsm, nullptr); break;
+    }
+}
+__device__ __forceinline__ void comb_warp(const Params& P, const Task& tk) {
+    const uint32_t ki = tk.key - KEY_CMB;
+    if (ki == 0) comb_task<4>(P, tk);
+    else if (ki == 1) comb_task<8>(P, tk);
+    else if (ki == 2) comb_task<16>(P, tk);
+    else comb_task<32>(P, tk);
+}
+
 __global__ void __launch_bounds__(256, 2) k_rg_classic(Params P) {
     extern __shared__ __align__(16) uint32_t smem32[];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -880,14 +904,7 @@ __global__ void __launch_bounds__(256, 2) k_rg_classic(Params P) {
         const uint32_t t = __shfl_sync(MI_FULL_MASK, next, 0);
         if (t >= ntasks) break;
         if (lane == 0) next = warp_tasks() + atomicAdd(P.scr + Scratch::QUEUE + 1, 1u);
-        const Task tk = decode_tab<1>(tab, t);
-        switch (tk.key - KEY_CLS) {
-            case 0: classic_task<1>(P, tk, wsm, nullptr); break;
-            case 1: classic_task<2>(P, tk, wsm, nullptr); break;
-            case 2: classic_task<4>(P, tk, wsm, nullptr); break;
-            case 3: classic_task<8>(P, tk, wsm, nullptr); break;
-            default: classic_task<16>(P, tk, wsm, nullptr); break;
-        }
+        classic_warp(P, decode_tab<1>(tab, t), wsm);
         __syncwarp();
     }
     pdl_join();
@@ -933,12 +950,7 @@ __global__ void __launch_bounds__(256, 2) k_rg_comb(Params P) {
         const uint32_t t = __shfl_sync(MI_FULL_MASK, next, 0);
         if (t >= ntasks) break;
         if (lane == 0) next = warp_tasks() + atomicAdd(P.scr + Scratch::QUEUE + 5, 1u);
-        const Task tk = decode_tab<5>(tab, t);
-        const uint32_t ki = tk.key - KEY_CMB;
-        if (ki == 0) comb_task<4>(P, tk);
-        else if (ki == 1) comb_task<8>(P, tk);
-        else if (ki == 2) comb_task<16>(P, tk);
-        else comb_task<32>(P, tk);
+        comb_warp(P, decode_tab<5>(tab, t));
         __syncwarp();
     }
     pdl_join();
@@ -1075,6 +1087,18 @@ __device__ __forceinline__ void add_rows(const Params& P, const Task& tk, AddDes
     __syncwarp();  // the slots are rewritten by the warp's next task
 }
 
+__device__ __forceinline__ void add_warp(const Params& P, const Task& tk, AddDesc* desc) {
+    switch (tk.key - KEY_ADD) {
+        case 0: add_short<1>(P, tk); break;
+        case 1: add_short<2>(P, tk); break;
+        case 2: add_short<4>(P, tk); break;
+        case 3: add_short<8>(P, tk); break;
+        case 4: add_short<16>(P, tk); break;
+        case 5: add_short<32>(P, tk); break;
+        default: add_rows(P, tk, desc); break;
+    }
+}
+
 __global__ void __launch_bounds__(256, 3) k_rg_add(Params P) {
     const uint32_t lane = threadIdx.x & 31u;
     __shared__ FamTab tab;
@@ -1088,17 +1112,77 @@ __global__ void __launch_bounds__(256, 3) k_rg_add(Params P) {
         const uint32_t t = __shfl_sync(MI_FULL_MASK, next, 0);
         if (t >= ntasks) break;
         if (lane == 0) next = warp_tasks() + atomicAdd(P.scr + Scratch::QUEUE + 2, 1u);
-        const Task tk = decode_tab<2>(tab, t);
-        switch (tk.key - KEY_ADD) {
-            case 0: add_short<1>(P, tk); break;
-            case 1: add_short<2>(P, tk); break;
-            case 2: add_short<4>(P, tk); break;
-            case 3: add_short<8>(P, tk); break;
-            case 4: add_short<16>(P, tk); break;
-            case 5: add_short<32>(P, tk); break;
-            default: add_rows(P, tk, desc[threadIdx.x >> 5]); break;
-        }
+        add_warp(P, decode_tab<2>(tab, t), desc[threadIdx.x >> 5]);
         __syncwarp();
+    }
+    pdl_join();
+}
+
+// --- short lists: two task kernels ------------------------------------------------
+//
+// A kernel of the chain starts about 2 us after the one before it and costs
+// the host 2 us, most of a short list's time.  Here one kernel takes the NTT
+// families' tasks and one the warp tasks of all others, each as one sequence
+// in descending cost.  (At 128 registers and two blocks per SM the additions
+// and the 64-bit digits have fewer warps than in kernels of their own, so
+// longer lists keep the chain.  One kernel for everything, its blocks going
+// from family to family, took 46 us where the chain took 42: each family a
+// block looks into costs it a microsecond.)  Operations of 512 to 32768 bits,
+// chain against this: 400 of them 39 us against 28, 1000 40.4 against 37.0,
+// 2000 42.2 against 43.7; of 512 to 4000 bits, 2000 19.7 against 15.9.
+constexpr uint32_t kSmallMaxOps = 1024;
+
+__global__ void __launch_bounds__(256, 2) k_rg_small_ntt(Params P) {
+    extern __shared__ __align__(16) uint32_t smem[];
+    __shared__ uint32_t s_task[2];
+    __shared__ FamTab tab[3];
+    pdl_wait();  // the binning is complete
+    pdl_trigger();
+    const uint32_t* nt = P.scr + Scratch::NTASKS;
+    const uint32_t e0 = nt[0], e1 = e0 + nt[4], e2 = e1 + nt[6];
+    if (blockIdx.x >= e2) return;
+    load_tab(tab[0], P.scr, 0);
+    load_tab(tab[1], P.scr, 4);
+    load_tab(tab[2], P.scr, 6);
+    if (threadIdx.x == 0) s_task[0] = blockIdx.x;
+    __syncthreads();
+    for (uint32_t it = 0;; ++it) {
+        const uint32_t t = s_task[it & 1];
+        if (t >= e2) break;
+        if (threadIdx.x == 0) s_task[(it + 1) & 1] = gridDim.x + atomicAdd(P.scr + Scratch::QUEUE, 1u);
+        if (t < e0) ntt_block<ntt32::DM64>(P, decode_tab<0>(tab[0], t), smem);
+        else if (t < e1) ntt_block<ntt32::DM48>(P, decode_tab<4>(tab[1], t - e0), smem);
+        else ntt_block<ntt32::DM40>(P, decode_tab<6>(tab[2], t - e1), smem);
+        __syncthreads();  // the next index is visible; this one is read by all
+    }
+}
+
+__global__ void __launch_bounds__(256, 2) k_rg_small_warps(Params P) {
+    extern __shared__ __align__(16) uint32_t smem32[];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    uint32_t* wsm = smem32 + warp * R32_WARP_WORDS;
+    __shared__ FamTab tab[4];
+    __shared__ AddDesc desc[8][kAddRowOps];
+    pdl_trigger();
+    const uint32_t* nt = P.scr + Scratch::NTASKS;
+    const uint32_t e0 = nt[7], e1 = e0 + nt[1], e2 = e1 + nt[5], e3 = e2 + nt[2];
+    if (blockIdx.x < e3) {
+        load_tab(tab[0], P.scr, 7);
+        load_tab(tab[1], P.scr, 1);
+        load_tab(tab[2], P.scr, 5);
+        load_tab(tab[3], P.scr, 2);
+        __syncthreads();
+        uint32_t next = first_task();
+        for (;;) {
+            const uint32_t t = __shfl_sync(MI_FULL_MASK, next, 0);
+            if (t >= e3) break;
+            if (lane == 0) next = warp_tasks() + atomicAdd(P.scr + Scratch::QUEUE + 7, 1u);
+            if (t < e0) rect32_task(P, decode_tab<7>(tab[0], t), wsm);
+            else if (t < e1) classic_warp(P, decode_tab<1>(tab[1], t - e0), wsm);
+            else if (t < e2) comb_warp(P, decode_tab<5>(tab[2], t - e1));
+            else add_warp(P, decode_tab<2>(tab[3], t - e2), desc[warp]);
+            __syncwarp();
+        }
     }
     pdl_join();
 }
@@ -1176,7 +1260,7 @@ mi_status ragged_launch(mi_ctx ctx, const mi_op* ops, uint32_t n_ops, const uint
     P.ntt_min = ntt_min < 1 ? 1 : (ntt_min > 257 ? 257 : ntt_min);
     P.ntt40_min = ctx->ragged_ntt40_min < 1 ? 1 : (ctx->ragged_ntt40_min > 257 ? 257 : ctx->ragged_ntt40_min);
     P.ntt = ctx->ntt.params;
-    static ResidentBlocks sites[9];
+    static ResidentBlocks sites[11];
     if (n_ops <= kBinMaxOps) {
         const uint32_t cluster = n_ops <= kBinOne ? 1u : kBinBlocks;
         const size_t smem = (n_ops + cluster - 1) / cluster;
@@ -1199,6 +1283,12 @@ mi_status ragged_launch(mi_ctx ctx, const mi_op* ops, uint32_t n_ops, const uint
     // SMs that the previous kernel's last tasks leave idle -- but one block of
     // each waits for its predecessor before it completes, so that the last
     // kernel completes after all.
+    if (n_ops <= kSmallMaxOps) {
+        MI_TRY(launch_tasks(k_rg_small_ntt, sites[9], kNttSmem, P, st));
+        MI_TRY(launch_tasks(k_rg_small_warps, sites[10], kR32Smem, P, st));
+        if (P.ntt_min > 129) MI_TRY(launch_tasks(k_rg_c64, sites[5], kC64Smem, P, st));
+        return MI_OK;
+    }
     MI_TRY(launch_tasks(k_rg_ntt<0>, sites[0], kNttSmem, P, st));
     MI_TRY(launch_tasks(k_rg_ntt<1>, sites[1], kNttSmem, P, st));
     MI_TRY(launch_tasks(k_rg_ntt<2>, sites[2], kNttSmem, P, st));

@@ -193,3 +193,29 @@ def test_ragged_binning_sizes(ctx, n):
     assert np.array_equal(carry[add], ((a + b) < a)[add].astype(np.uint8))
     assert np.array_equal(out[at[mul]], (a * b)[mul]) and not out[at[mul] + 1].any()
     assert (out[at[kind == 9]] == np.uint64(2**64 - 1)).all()
+
+
+@pytest.mark.parametrize("n", [1, 7, 300, 1024, 1025])
+def test_ragged_short_list_kernels(ctx, n):
+    # the two-kernel form of short lists and the first list that takes a kernel
+    # per family: every family present (with the 64-thread classical groups
+    # where the crossovers leave them work), worst-case carries
+    rng = np.random.default_rng(n)
+    kind = (np.arange(n) % 2).astype(np.uint32)
+    la = rng.choice(np.array(EDGE, np.uint32), n)
+    lb = np.where(rng.integers(0, 2, n) == 0, la, rng.choice(np.array(EDGE, np.uint32), n)).astype(np.uint32)
+    ops, pool, out_limbs = W.pack_ops(kind, la, lb, n)
+    pool[rng.integers(0, 2, pool.size) == 0] = np.uint64(2**64 - 1)
+    old = ctx.get_tuning(midint.TUNE_RAGGED_NTT_MIN), ctx.get_tuning(midint.TUNE_RAGGED_NTT_MIN, 1)
+    try:
+        for m in (old, (257, 257), (1, 1)):
+            ctx.set_tuning(midint.TUNE_RAGGED_NTT_MIN, 0, m[0])
+            ctx.set_tuning(midint.TUNE_RAGGED_NTT_MIN, 1, m[1])
+            out, carry, invalid = run_ragged(ctx, ops, pool, out_limbs)
+            assert invalid == 0
+            oracle_check(ops, pool, out, carry)
+            out2, carry2, _ = run_ragged(ctx, ops, pool, out_limbs, graph=True, replays=2)
+            assert np.array_equal(out, out2) and np.array_equal(carry, carry2)
+    finally:
+        ctx.set_tuning(midint.TUNE_RAGGED_NTT_MIN, 0, old[0])
+        ctx.set_tuning(midint.TUNE_RAGGED_NTT_MIN, 1, old[1])

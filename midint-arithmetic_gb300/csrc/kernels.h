@@ -59,6 +59,12 @@ uint32_t flex_rounds(uint32_t n, uint32_t n32, bool full, uint32_t max_rounds = 
 mi_status launch_mul_flex(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32, bool full,
                           uint32_t rounds, cudaStream_t st);
 
+// Full products of 25..32 blocks of 8 u32 limbs with one Karatsuba level
+// (mul_kara.cu), and the batches for which that is the fastest form.
+bool kara_pays(uint32_t n, uint32_t n32);
+mi_status launch_mul_kara(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32,
+                          cudaStream_t st);
+
 // Low n32 limbs of a*b per instance (u32 limb views) on power-of-two groups, n32 > 128.
 mi_status launch_mul_lo(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32, cudaStream_t st);
 

@@ -195,6 +195,7 @@ mi_status dispatch(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n
 
 mi_status launch_mul_classic(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32, bool full,
                              cudaStream_t st, uint32_t max_per_sm) {
+    if (full && max_per_sm == 0 && kara_pays(n, n32)) return launch_mul_kara(a, b, r, n, n32, st);
     if (!full || max_per_sm == 0) {
         const uint32_t rounds = flex_rounds(n, n32, full);
         if (rounds != 0) return launch_mul_flex(a, b, r, n, n32, full, rounds, st);

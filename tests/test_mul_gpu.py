@@ -152,3 +152,31 @@ def test_mul_lane_groups(ctx, devmem, m, full):
         if n <= big:
             got = gpu_mul(ctx, devmem, a[:n * m], b[:n * m], m, full, limb_bits=32, offset=n & 1)
             assert np.array_equal(got, want[:n * rl]), n
+
+
+@pytest.mark.parametrize("m", [193, 200, 201, 208, 209, 223, 224, 225, 239, 240, 241, 255, 256])
+def test_mul_karatsuba_batches(ctx, devmem, m):
+    # 25..32 blocks in the batches that take one Karatsuba level (an odd count
+    # leaves half a warp idle): halves of zeros, all ones and random values, equal
+    # halves, halves that differ in one bit, in every combination of signs
+    big = 4301
+    rng = np.random.default_rng(m)
+    half = 8 * ((m + 15) // 16)
+    ops = []
+    for _ in range(2):
+        x = rng.integers(0, 2**32, (big, 2 * half), dtype=np.uint32)
+        lo, hi = x[:, :half], x[:, half:]
+        pick = rng.integers(0, 8, big)
+        lo[pick == 0] = 0
+        hi[pick == 1] = 0
+        lo[pick == 2] = 0xFFFFFFFF
+        hi[pick == 3] = 0xFFFFFFFF
+        hi[pick == 4] = lo[pick == 4]
+        hi[pick == 5] = lo[pick == 5] ^ np.uint32(1)
+        x[pick == 6] = 0xFFFFFFFF
+        ops.append(np.ascontiguousarray(x[:, :m]).reshape(-1))
+    a, b = ops
+    want = O.mul(a, b, m, True)
+    for n, offset in ((big, 0), (big, 1), (1601, 0)):
+        got = gpu_mul(ctx, devmem, a[:n * m], b[:n * m], m, True, limb_bits=32, offset=offset)
+        assert np.array_equal(got, want[:n * 2 * m]), (n, offset)

@@ -51,17 +51,21 @@ uint32_t add_size_class(uint64_t bytes);
 mi_status launch_mul_classic(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32,
                              bool full, cudaStream_t st, uint32_t max_per_sm = 0);
 
-// The same, full or low half, on groups of any number of lanes (mul_flex.cu):
-// flex_rounds says with how many rounds (1..max_rounds), or 0 where the
-// power-of-two groups are faster or hold the product alone; below `few` warps
-// per SM those lose on their launch shape.
-uint32_t flex_rounds(uint32_t n, uint32_t n32, bool full, uint32_t max_rounds = 3, uint32_t few = 16);
+// Dynamic shared memory (at least *smem) for a launch of one-warp blocks that
+// keeps the next launch's early blocks from crowding one scheduler.
+mi_status balanced_smem(uint64_t blocks, uint32_t resident, size_t* smem);
+
+// The same products, full or low half, on groups of any number of lanes
+// (mul_flex.cu): flex_rounds says with how many rounds (1..3), or 0 where the
+// power-of-two groups are faster or hold the product alone; us, where given,
+// is the modelled time.
+uint32_t flex_rounds(uint32_t n, uint32_t n32, bool full, double* us = nullptr);
 mi_status launch_mul_flex(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32, bool full,
                           uint32_t rounds, cudaStream_t st);
 
 // Full products of 25..32 blocks of 8 u32 limbs with one Karatsuba level
 // (mul_kara.cu), and the batches for which that is the fastest form.
-bool kara_pays(uint32_t n, uint32_t n32);
+bool kara_pays(uint32_t n, uint32_t n32, bool vec);
 mi_status launch_mul_kara(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32,
                           cudaStream_t st);
 

@@ -48,7 +48,7 @@ struct MulShape {
 template <int NT, bool VEC, bool WB>
 __global__ void __launch_bounds__(MulShape<NT, WB>::BLOCK, MulShape<NT, WB>::MIN_BLOCKS)
     k_mul(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b, uint32_t* __restrict__ r, uint32_t n,
-          uint32_t n32) {
+          uint32_t n32, uint32_t rlen) {
     using S = MulShape<NT, WB>;
     extern __shared__ __align__(16) uint32_t smem[];
     uint32_t* sA = smem;
@@ -61,7 +61,6 @@ __global__ void __launch_bounds__(MulShape<NT, WB>::BLOCK, MulShape<NT, WB>::MIN
     uint4* gB4 = reinterpret_cast<uint4*>(sB + grp * S::WPAD);
     uint2* slots = reinterpret_cast<uint2*>(sT) + grp * NT * classic::PAIRS;
     uint32_t* scr = sA;  // only used after the tile loop, by groups wider than a warp
-    const uint32_t rlen = 2 * n32;
     const uint32_t nb = (n32 + T - 1) / T;  // blocks holding limbs; the rest of the NT are zero padding
     const uint64_t stride = uint64_t(gridDim.x) * S::IPB;
     pdl_wait();  // launched with launch_pdl
@@ -154,13 +153,14 @@ mi_status launch_shape(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32
     auto kern = k_mul<NT, VEC, WB>;
     size_t smem = S::SMEM;
     MI_TRY(capped_smem(S::SMEM, max_per_sm, &smem));
-    MI_TRY(ensure_dyn_smem(kern, smem));
     uint64_t blocks = (uint64_t(n) + S::IPB - 1) / S::IPB;
+    if (S::WARP) MI_TRY(balanced_smem(blocks, 16, &smem));
+    MI_TRY(ensure_dyn_smem(kern, smem));
     // one block per unit of work for one-warp blocks (see above); the others
     // stride over the batch from a grid of a few waves
     const uint64_t cap = S::WARP ? (uint64_t(1) << 24) : uint64_t(sm_count()) * 32;
     if (blocks > cap) blocks = cap;
-    MI_CUDA_TRY(launch_pdl(kern, dim3(uint32_t(blocks)), dim3(S::BLOCK), smem, st, a, b, r, n, n32));
+    MI_CUDA_TRY(launch_pdl(kern, dim3(uint32_t(blocks)), dim3(S::BLOCK), smem, st, a, b, r, n, n32, 2 * n32));
     return MI_OK;
 }
 
@@ -193,15 +193,30 @@ mi_status dispatch(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n
 
 }  // namespace
 
+// A launch of w one-warp blocks per SM where `resident` fit: the next launch of
+// a stream of them starts early on the places that are left, its last blocks
+// on those that become free, and where the early ones were many and not all
+// (w < resident <= 2 w) one scheduler gets most of the rest: 4 or 5 warps
+// instead of w / 4.  Keeping the places to a multiple of four that just holds
+// the launch leaves each scheduler its share (full products of 1672 x 233
+// words, w = 11, 23.9 us -> 19.7 in k_mul, 30.9 -> 20.7 in k_mul_flex; 3648 x 301
+// low halves in two rounds 48.5 -> 34.2).  Other launches are left alone: with
+// places for both the early start is worth 0.5 us (912 x 225 13.2 against 14.0).
+mi_status balanced_smem(uint64_t blocks, uint32_t resident, size_t* smem) {
+    const uint64_t sms = uint64_t(sm_count()), w = (blocks + sms - 1) / sms, places = (w + 3) / 4 * 4;
+    if (w >= resident || 2 * w < resident) return MI_OK;
+    return capped_smem(*smem, uint32_t(places), smem);
+}
+
 mi_status launch_mul_classic(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32, bool full,
                              cudaStream_t st, uint32_t max_per_sm) {
-    if (full && max_per_sm == 0 && kara_pays(n, n32)) return launch_mul_kara(a, b, r, n, n32, st);
+    const bool vec = aligned16(a) && aligned16(b) && aligned16(r) && (n32 % 4 == 0);
+    if (full && max_per_sm == 0 && kara_pays(n, n32, vec)) return launch_mul_kara(a, b, r, n, n32, st);
     if (!full || max_per_sm == 0) {
         const uint32_t rounds = flex_rounds(n, n32, full);
         if (rounds != 0) return launch_mul_flex(a, b, r, n, n32, full, rounds, st);
     }
     if (!full) return launch_mul_lo(a, b, r, n, n32, st);  // half the partial products of a full product
-    const bool vec = aligned16(a) && aligned16(b) && aligned16(r) && (n32 % 4 == 0);
     return vec ? dispatch<true>(a, b, r, n, n32, st, max_per_sm) : dispatch<false>(a, b, r, n, n32, st, max_per_sm);
 }
 

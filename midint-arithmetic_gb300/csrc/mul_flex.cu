@@ -65,37 +65,51 @@ __global__ void __launch_bounds__(32, MB)
 
 }  // namespace
 
-// The rule counts steps: a warp's steps times the warps a scheduler runs one
-// after another (at least kLone, the cost of a warp on its own), times the
-// measured cost of a step relative to the loops of mul.cu and mul_lo.cu at
-// non-power-of-two sizes -- 1.05 to 1.08, 1.18 and 1.26 to 1.33 for one, two and three
-// rounds (more rounds leave fewer warps per SM for the slots' shared memory).  Those
-// loops run on 16 or more threads per product (32 or more blocks for low
-// halves) only, 0.88 of a step where nb fills the group; below `few` warps per SM
-// their launches overlap less, at 124 registers (full products of 1500 x 68
-// limbs 14.1 us against 12.4), and blocks of eight warps spread badly (low
-// halves of 1000 x 100 limbs 14.1 against 9.9).
-uint32_t flex_rounds(uint32_t n, uint32_t n32, bool full, uint32_t max_rounds, uint32_t few) {
-    constexpr double kLone = 1.2, kStep[2][4] = {{1.0, 1.05, 1.18, 1.26}, {1.0, 1.08, 1.18, 1.33}};  // [full][rounds]
-    const double schedulers = 4.0 * sm_count();
+// Blocks of a shape resident per SM: 16 to 21 for the registers, and what the
+// shared memory allows.
+static uint32_t flex_resident(const FlexShape& S) {
+    return std::min<uint32_t>(18, uint32_t(228 * 1024 / (S.smem() + 1024)));
+}
+
+// The rule compares modelled times.  A launch's time is set by the warps of its
+// busiest scheduler, k = ceil(warps per SM / 4): steps * (A + B k), A the
+// latency of a step on its own, B its share of the scheduler (in units of one
+// B; us per step: 0.164 for k_mul, which is 0.92 of that where nb
+// fills the group, 0.173 and 0.178 for one round, 0.16 for two and 0.15 for
+// three, whose steps share the staging).  k_mul_lo's blocks of eight warps come
+// in pairs of warps per scheduler, and with 13 to 15 warps per SM the third
+// block of a launch meets the first of the next (4256 x 233 words 35.4 us,
+// 4864 x 233 25.5).  More rounds need more shared memory: a second wave of
+// blocks costs its own latency.  Power-of-two groups of fewer than 16 threads
+// serve no launches here.  Against what this replaced, the same with
+// warps / 4 unrounded: 1824 x 177 words 24.4 -> 15.5, 3952 x 177 42.8 -> 30.0,
+// low halves of 3648 x 233 32.5 -> 21.7, 1824 x 511 62 -> 43.
+uint32_t flex_rounds(uint32_t n, uint32_t n32, bool full, double* us) {
+    constexpr double kA[2] = {0.18, 0.145}, kB[2] = {0.166, 0.164};  // [full]: the power-of-two groups
+    constexpr double kFlexA[2][4] = {{0, 0.16, 0.20, 0.19}, {0, 0.18, 0.18, 0.19}};  // [full][rounds]
+    constexpr double kFlexB[2][4] = {{0, 0.178, 0.16, 0.15}, {0, 0.173, 0.158, 0.15}};
+    const double sms = sm_count();
     const uint32_t nb = (n32 + T - 1) / T, steps = full ? nb : nb + 1;
     uint32_t threads = 1;  // of a power-of-two group
     while (threads < (full ? nb : (nb + 1) / 2)) threads *= 2;
     double best = 1e300;
     uint32_t pick = 0;
     if (threads >= 16) {
-        const double warps = double(n) * threads / 32;
-        const bool fills = nb == (full ? threads : 2 * threads);
-        best = steps * (fills ? 0.88 : kStep[full][0]) * std::max(kLone, warps / schedulers);
-        if (warps < double(few) * sm_count()) best *= full ? 1.15 : 1.3;
+        const double w = std::ceil(double(n) * threads / 32) / sms;  // warps per SM
+        double k = std::ceil(w / 4);
+        if (!full) k = w > 12 && w < 16 ? 6 : 2 * std::ceil(w / 8);
+        best = steps * (kA[full] + kB[full] * k);
+        if (nb == (full ? threads : 2 * threads)) best *= 0.92;
     }
-    for (uint32_t rounds = 1; rounds <= max_rounds; ++rounds) {
+    for (uint32_t rounds = 1; rounds <= 3; ++rounds) {
         const FlexShape S = flex_shape(n32, full, rounds, 2);
         if (S.lanes > 32) continue;
-        const double warps = std::ceil(double(n) / S.groups);
-        const double cost = double(rounds) * steps * kStep[full][rounds] * std::max(kLone, warps / schedulers);
+        const double w = std::ceil(double(n) / S.groups) / sms;
+        const double waves = w > flex_resident(S) ? 2 : 1;
+        const double cost = double(rounds) * steps * (kFlexA[full][rounds] * waves + kFlexB[full][rounds] * std::ceil(w / 4));
         if (cost < best) best = cost, pick = rounds;
     }
+    if (us != nullptr) *us = best;
     return pick;
 }
 
@@ -111,8 +125,10 @@ mi_status launch_mul_flex(const uint32_t* a, const uint32_t* b, uint32_t* r, uin
         {{k_mul_flex<false, false, 18>, k_mul_flex<false, true, 18>},
          {k_mul_flex<true, false, 18>, k_mul_flex<true, true, 18>}}};
     const Kernel kern = kernels[blocks <= 16u * uint64_t(sm_count())][full][vec];
-    MI_TRY(ensure_dyn_smem(kern, S.smem()));
-    MI_CUDA_TRY(launch_pdl(kern, dim3(uint32_t(blocks)), dim3(32), S.smem(), st, a, b, r, n, n32, S));
+    size_t smem = S.smem();
+    MI_TRY(balanced_smem(blocks, flex_resident(S), &smem));
+    MI_TRY(ensure_dyn_smem(kern, smem));
+    MI_CUDA_TRY(launch_pdl(kern, dim3(uint32_t(blocks)), dim3(32), smem, st, a, b, r, n, n32, S));
     return MI_OK;
 }
 

@@ -23,6 +23,7 @@
 // 105.5; 60000 x 128 482 -> 417.  With 24 blocks (96 limbs) it loses, 101.9
 // against 105.5; with 33 and more the transforms win, 168 for 129..160 limbs.
 #include <algorithm>
+#include <cmath>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -208,17 +209,22 @@ __global__ void __launch_bounds__(32, 16)
 }  // namespace
 
 // A warp holds two instances where k_mul's holds one, so a batch that leaves
-// the SMs partly empty waits longer for its warps: faster from some 14 of the
-// 16 resident warps per SM on, and where this kernel has two warps on a
-// scheduler and k_mul three or four (beyond 25 blocks: those take lane groups
-// there).  The power-of-two and lane groups against this, us: 4257 x 128 limbs
-// 41.4 against 39.4, 4000 x 128 37.7 against 39.5, 4257 x 100 35.2 against 33.8,
-// 4000 x 100 31.8 against 34.1; 1600 x 112 28.4 against 19.8, 1450 x 112 18.4
-// against 19.7, 2000 x 128 22.9 against 21.7, 2500 x 128 27.7 against 39.3.
-bool kara_pays(uint32_t n, uint32_t n32) {
+// the SMs partly empty waits longer for its warps.  The rule compares modelled
+// times as flex_rounds does: the latency of the 3 h steps and, for each warp of
+// the busiest scheduler, theirs and 2 us of staging and carries, against the
+// form that it would replace (4 % of it in hand, 9 % on
+// unaligned rows).  us against the other
+// forms: 4257 x 128 limbs 39.4 against 41.4, 4000 x 128 39.5 against 37.7, 4257 x
+// 100 33.8 against 35.2, 4000 x 100 34.1 against 31.8, 5000 x 128 48.5 against
+// 46.9, 7000 x 128 56.3 against 61.6, 2280 x 120 21 against 23.7.
+bool kara_pays(uint32_t n, uint32_t n32, bool vec) {
     if (n32 <= 24 * T || n32 > 2 * NT * T) return false;
-    const uint32_t sms = uint32_t(sm_count());
-    return n > 28 * sms || (n32 > 25 * T && n > 10 * sms && n <= 15 * sms);
+    const double w = std::ceil(double(n) / IPB) / sm_count(), steps = 3 * ((n32 + 2 * T - 1) / (2 * T));
+    // the first blocks of a second wave crowd the schedulers that free first
+    const double k = w <= 16 ? std::ceil(w / 4) : std::max(6.0, std::ceil(w / 4 + 0.1));
+    double other = 0;
+    flex_rounds(n, n32, true, &other);
+    return steps * 0.13 + 0.5 + k * (2.05 + 0.131 * steps) < (vec ? 0.96 : 0.91) * other;
 }
 
 mi_status launch_mul_kara(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32,

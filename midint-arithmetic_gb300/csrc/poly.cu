@@ -1,6 +1,8 @@
 // poly.cu -- the fused polynomial composite ((a^2 + b)(b^2 + b) + ab) mod
 // 2^(32*n32), the reference's polyKerQ (cuda/ker-classic-mul.cu.h:500-575), as
 // four low-half products (classic::low_product) and three sums in one kernel.
+#include <algorithm>
+#include <cmath>
 #include <cstdio>
 
 #include "mul_flex.cuh"
@@ -194,9 +196,11 @@ mi_status launch_poly_flex(const uint32_t* a, const uint32_t* b, uint32_t* r, ui
     const bool vec = aligned16(a) && aligned16(b) && aligned16(r) && (n32 % 4 == 0);
     const FlexShape S = flex_shape(n32, false, rounds, 3);
     auto kern = vec ? k_poly_flex<true> : k_poly_flex<false>;
-    MI_TRY(ensure_dyn_smem(kern, S.smem()));
     const uint64_t blocks = (uint64_t(n) + S.groups - 1) / S.groups;
-    MI_CUDA_TRY(launch_pdl(kern, dim3(uint32_t(blocks)), dim3(32), S.smem(), st, a, b, r, n, n32, S));
+    size_t smem = S.smem();
+    MI_TRY(balanced_smem(blocks, std::min<uint32_t>(16, uint32_t(228 * 1024 / (smem + 1024))), &smem));
+    MI_TRY(ensure_dyn_smem(kern, smem));
+    MI_CUDA_TRY(launch_pdl(kern, dim3(uint32_t(blocks)), dim3(32), smem, st, a, b, r, n, n32, S));
     return MI_OK;
 }
 
@@ -213,9 +217,28 @@ mi_status dispatch(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n
 
 }  // namespace
 
+// Lane groups: where they need fewer warps times steps (1.08 of a step there,
+// 0.88 in a loop whose power-of-two group is full), a warp on its own counting
+// 1.2, for all of fewer than nine blocks, and earlier below eight warps per
+// SM, where k_poly's blocks of eight warps spread badly (3000 x 100 limbs 79.5
+// us there, 82 here).
+static bool flex_pays(uint32_t n, uint32_t n32) {
+    constexpr double kLone = 1.2;
+    const double schedulers = 4.0 * sm_count();
+    const uint32_t nb = (n32 + T - 1) / T;
+    const FlexShape S = flex_shape(n32, false, 1, 2);
+    if (S.lanes > 32) return false;
+    uint32_t threads = 1;  // of a power-of-two group
+    while (threads < (nb + 1) / 2) threads *= 2;
+    if (threads < 16) return true;
+    const double warps = double(n) * threads / 32;
+    const double few = warps < 8.0 * sm_count() ? 1.3 : 1.0;
+    return 1.08 * std::max(kLone, std::ceil(double(n) / S.groups) / schedulers) <
+           few * (nb == 2 * threads ? 0.88 : 1.0) * std::max(kLone, warps / schedulers);
+}
+
 mi_status launch_poly(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32, cudaStream_t st) {
-    const uint32_t rounds = flex_rounds(n, n32, false, 1, 8);  // (3000 x 100 limbs 79.5 us without, 82 with)
-    if (rounds != 0) return launch_poly_flex(a, b, r, n, n32, rounds, st);
+    if (flex_pays(n, n32)) return launch_poly_flex(a, b, r, n, n32, 1, st);
     const bool vec = aligned16(a) && aligned16(b) && aligned16(r) && (n32 % 4 == 0);
     return vec ? dispatch<true>(a, b, r, n, n32, st) : dispatch<false>(a, b, r, n, n32, st);
 }

@@ -180,3 +180,14 @@ def test_mul_karatsuba_batches(ctx, devmem, m):
     for n, offset in ((big, 0), (big, 1), (1601, 0)):
         got = gpu_mul(ctx, devmem, a[:n * m], b[:n * m], m, True, limb_bits=32, offset=offset)
         assert np.array_equal(got, want[:n * 2 * m]), (n, offset)
+
+
+@pytest.mark.parametrize("n", [1217, 1400, 1700, 2281, 2432, 3648])
+@pytest.mark.parametrize("m,full", [(137, True), (177, True), (225, True), (137, False), (233, False), (301, False)])
+def test_mul_balanced_launches(ctx, devmem, m, full, n):
+    # batches whose launches keep their places to a multiple of four (a last
+    # block or warp partly empty), on each of the forms the rule picks there
+    a, b = carry_stress(n, m, seed=n + m, dtype=np.uint32)
+    want = O.mul(a, b, m, full)
+    for _ in range(2):
+        assert np.array_equal(gpu_mul(ctx, devmem, a, b, m, full, limb_bits=32), want)

@@ -668,20 +668,39 @@ mi_status dispatch_vec(const L* a, const L* b, L* r, uint8_t* carry, uint32_t n,
     return dispatch_gs<L, true, OP, 4 * QS>(a, b, r, carry, n, m, gs, st);
 }
 
-// k_add_rows, all others: four rows per thread (two leave too little in
-// flight, 65 limbs 45.2 us against 30.5 per 2^23 limbs; eight, too few warps,
-// 1001 limbs 35.5 against 29.9), two for up to 4 u64 limbs (38.4 against 51.2
-// for one) and for 25 to 32 (rows of 16 lanes instead of 8: 31.4 against 33.7),
-// eight where four would need a block of 1024 threads (4095 limbs 38.6
-// against 50.1).
+// Rows per thread of k_add_rows: four (two leave too little in flight, eight too
+// few warps), or what pads less than the next power of two of threads does --
+// five rows where 5/8 of it holds the row of limbs, three or six (the better by
+// length) where 3/4 does.  Short u64 rows differ: with four rows a group of 4 or 8 lanes
+// reads 32 or 64 contiguous bytes at a time, and five are better although they
+// pad more.  us per 2^22 u64 or 2^23 u32 limbs with four rows against the
+// pick: 15 limbs 20.9 -> 16.7, 27 17.6 -> 16.1, 65 17.0 -> 16.0, 95 16.9 -> 15.8, 129
+// 20.8 -> 16.3, 513 18.3 -> 16.1; 33 words 24.6 -> 18.6, 65 23.3 -> 18.3, 129 29.8
+// -> 17.5, 161 25.7 -> 17.0, 333 24.6 -> 20.0.  Eight where four would need a
+// block of 1024 threads (4095 limbs 38.6 against 50.1).
+template <typename L>
+uint32_t rows_per_thread(uint32_t m) {
+    const uint32_t slots = 4 * pow2ceil((m + 3) / 4);
+    if (slots > 4 * 512) return 8;
+    const bool half = 8 * m <= 5 * slots, three = 4 * m <= 3 * slots;
+    if (sizeof(L) == 4) return m <= 4 ? 4 : half ? 5 : three ? (m < 256 ? 6 : 3) : 4;
+    if (m <= 4 || (m >= 30 && m <= 32)) return 2;
+    if ((m >= 13 && m <= 16) || (m >= 25 && m <= 29)) return 5;
+    if (m <= 96) return three && (m < 9 || m > 12) ? 3 : 4;
+    return half ? (m <= 160 ? 6 : 5) : 4;
+}
+
 template <typename L, int OP>
 mi_status dispatch_rows(const L* a, const L* b, L* r, uint8_t* carry, uint32_t n, uint32_t m, cudaStream_t st) {
-    const bool two = sizeof(L) == 8 && (m <= 4 || (m > 24 && m <= 32));
-    const uint32_t q = two ? 2 : pow2ceil((m + 3) / 4) > 512 ? 8 : 4;
-    const uint32_t gs = pow2ceil((m + q - 1) / q);
-    if (q == 2) return dispatch_gs<L, false, OP, 2>(a, b, r, carry, n, m, gs, st);
-    if (q == 4) return dispatch_gs<L, false, OP, 4>(a, b, r, carry, n, m, gs, st);
-    return dispatch_gs<L, false, OP, 8>(a, b, r, carry, n, m, gs, st);
+    const uint32_t q = rows_per_thread<L>(m), gs = pow2ceil((m + q - 1) / q);
+    switch (q) {
+        case 2: return dispatch_gs<L, false, OP, 2>(a, b, r, carry, n, m, gs, st);
+        case 3: return dispatch_gs<L, false, OP, 3>(a, b, r, carry, n, m, gs, st);
+        case 4: return dispatch_gs<L, false, OP, 4>(a, b, r, carry, n, m, gs, st);
+        case 5: return dispatch_gs<L, false, OP, 5>(a, b, r, carry, n, m, gs, st);
+        case 6: return dispatch_gs<L, false, OP, 6>(a, b, r, carry, n, m, gs, st);
+        default: return dispatch_gs<L, false, OP, 8>(a, b, r, carry, n, m, gs, st);
+    }
 }
 
 }  // namespace

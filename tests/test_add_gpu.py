@@ -204,3 +204,26 @@ def test_add_rows_of_odd_lengths(ctx, devmem, m, bits):
             ctx.add6(pa, pb, pa if inplace else pr, n, m, stream=s)
             torch.cuda.synchronize()
             assert np.array_equal(devmem.get(ba if inplace else br, words), O.add6(a, b, m))
+
+
+@pytest.mark.parametrize("bits", [64, 32])
+@pytest.mark.parametrize("m", [6, 7, 10, 13, 16, 24, 27, 30, 41, 48, 80, 96, 97, 131, 160, 161, 191, 193, 319, 320, 321,
+                               385, 513, 640, 641, 765, 1025, 1281, 1537])
+def test_add_rows_per_thread(ctx, devmem, m, bits):
+    # the edges of the rows-per-thread rule (2 to 6 rows), even lengths on rows
+    # that are off by one limb
+    n = 300 if m < 300 else 29
+    a, b = carry_stress(n, m, seed=m + bits, dtype=np.uint64 if bits == 64 else np.uint32)
+    want, carry = O.add(a, b, m)
+    words, off = a.view(np.uint32).size, bits // 32
+    (ba, pa), (bb, pb), (br, pr) = devmem.put(a, off), devmem.put(b, off), devmem.empty_words(words, off)
+    dc = torch.full((n + 8,), 7, dtype=torch.uint8, device="cuda:0")
+    s = torch.cuda.current_stream().cuda_stream
+    ctx.add(pa, pb, pr, n, m, carry=dc.data_ptr(), limb_bits=bits, stream=s)
+    torch.cuda.synchronize()
+    assert np.array_equal(devmem.get(br, words, off, a.dtype), want)
+    assert np.array_equal(dc.cpu().numpy()[:n], carry) and (dc.cpu().numpy()[n:] == 7).all()
+    if bits == 64:
+        ctx.add6(pa, pb, pr, n, m, stream=s)
+        torch.cuda.synchronize()
+        assert np.array_equal(devmem.get(br, words, off, a.dtype), O.add6(a, b, m))

@@ -14,7 +14,9 @@ A step is one batched multiplication over the whole batch.
           pipeline's time is reported beside it).
   roofline: the multiplication kernel against the integer-multiply ceiling
           measured in-process (mi_calib_mul32_peak), in 32x32-bit partial
-          products/s; 65536 partial products per instance.
+          products/s; 65536 partial products per instance (counted as the
+          schoolbook product; the kernel's one Karatsuba level multiplies
+          three quarters of them).
   workloads: the other benchmark rows measured in the same run (addition GB/s
           and %HBM against MEASURED_PEAKS.json, the u32-limb variant).
   cpu_baseline: the oracle's port of the reference CPU path (GMP mpz_mul via
@@ -481,13 +483,14 @@ def run_ours(args):
                    "l2": f"inputs rotate over {sets} operand sets of {set_bytes >> 20} MiB (> 4x L2)"},
         "roofline": {"bound": "int-mul", "achieved": achieved_prod / 1e9, "peak": peak_prod / 1e9,
                      "unit": "G 32x32-bit partial products/s", "frac": achieved_prod / peak_prod,
-                     # dram__bytes_read.sum + dram__bytes_write.sum of one k_mul<32> launch (ncu, cold, single
+                     # dram__bytes_read.sum + dram__bytes_write.sum of one k_mul_kara launch (ncu, cold, single
                      # launch): the 32 MiB of operands read once, the product still in L2 at kernel end
-                     "traffic": 33.62e6 + 0.23e6,
-                     "traffic_source": "ncu --set full of one k_mul<32> launch (summary committed under profiles/)",
+                     "traffic": 33.61e6 + 0.21e6,
+                     "traffic_source": "ncu --set full of one k_mul_kara launch (summary committed under profiles/)",
                      "peak_source": "measured in-process: mi_calib_mul32_peak (independent mad.lo.cc/madc.hi.cc "
                                     "chains, the kernel's own instruction mix)",
-                     "per_unit": f"{prods32_per_inst} partial products per instance",
+                     "per_unit": f"{prods32_per_inst} schoolbook partial products per instance (the kernel's one "
+                                 "Karatsuba level multiplies three quarters of them)",
                      # operands in and products out once: far below the HBM bound
                      "hbm": hbm_position(4 * in_bytes, ms, measured_peaks().get("hbm_gbs"))},
         "gpu_launches": args.steps,
@@ -1046,7 +1049,7 @@ def run_case(args):
 
       add     65536 x 64 u64 limbs, carries        (k_add)
       add6    6a + 10b on the same batch            (k_add, 6a+10b variant)
-      mul     16384 x 128 u64 limbs, full products  (k_mul)
+      mul     16384 x 128 u64 limbs, full products  (k_mul_kara)
       mul_lo  the same batch, low halves            (k_mul_lo)
       poly    the same batch                        (k_poly)
       poly2048  512 x 2048 u64 limbs, the composite on transforms (k_poly_ntt)

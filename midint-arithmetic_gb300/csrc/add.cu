@@ -214,7 +214,7 @@ __device__ __forceinline__ uint64_t six_hi(uint64_t ai, uint64_t bi) {
 // lookahead over its two ballots, the rows chained by their one-bit carry;
 // groups wider than a warp do it twice, with the carry into the warp from a
 // lookahead over one word per warp in between.  (2048 x 4095 limbs 60.4 ->
-// 38.6 us, 8380 x 1001 42.7 -> 29.9, 1677721 x 5 55.5 -> 30.8, 16760 x 1001
+// 38.6 us, 8380 x 1001 42.7 -> 29.9, 16760 x 1001
 // 32-bit limbs 67.1 -> 31.8, 2048 x 8191 116.5 -> 54.4.)
 template <typename L, int Q, int GS, int OP>
 __global__ void __launch_bounds__(GS > 256 ? GS : 256)

@@ -36,7 +36,7 @@ using classic::T;
 
 // MB: blocks per SM at least.  16 (100 registers) for batches that fill the
 // GPU; 18 (96) below that, where two launches then fit the SMs at once and
-// overlap (1500 x 68 limbs 12.1 us against 15.4; 16384 x 68 66.3 against 64.1,
+// overlap (1500 x 68 limbs 11.5 us against 15.4; 16384 x 68 66.3 against 64.1,
 // low halves of 12000 x 301 words 108 against 104.6).
 template <bool FULL, bool VEC, int MB>
 __global__ void __launch_bounds__(32, MB)
@@ -73,8 +73,8 @@ static uint32_t flex_resident(const FlexShape& S) {
 
 // The rule compares modelled times.  A launch's time is set by the warps of its
 // busiest scheduler, k = ceil(warps per SM / 4): steps * (A + B k), A the
-// latency of a step on its own, B its share of the scheduler (in units of one
-// B; us per step: 0.164 for k_mul, which is 0.92 of that where nb
+// latency of a step on its own, B its share of the scheduler (us
+// per step: 0.164 for k_mul, which is 0.92 of that where nb
 // fills the group, 0.173 and 0.178 for one round, 0.16 for two and 0.15 for
 // three, whose steps share the staging).  k_mul_lo's blocks of eight warps come
 // in pairs of warps per scheduler, and with 13 to 15 warps per SM the third

@@ -47,6 +47,10 @@ void ntt_tables_destroy(NttTables* T);
 mi_status launch_mul_ntt(const uint64_t* a, const uint64_t* b, uint64_t* r, uint32_t n, uint32_t m,
                          const NttMulParams& P, cudaStream_t st, bool low = false);
 
+// Whether n instances, per_sm blocks of which fit an SM, are launched as a
+// programmatic dependent launch.
+bool ntt_dependent(uint32_t n, int per_sm);
+
 // Whether launch_mul_ntt runs n products of m limbs on clusters (a block per
 // prime), where a call takes little more than the latency of one prime.
 bool ntt_small_batch(uint32_t n, uint32_t m);

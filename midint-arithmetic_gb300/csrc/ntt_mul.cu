@@ -103,6 +103,23 @@ bool cluster_fits(uint32_t n, int np, int lg) {
     return uint64_t(n) * uint32_t(np) < uint64_t(sm_count()) * cluster_blocks_per_sm(lg);
 }
 
+}  // namespace
+
+// Up to two instances per SM, a programmatic dependent launch (m = 1024, n =
+// 152 18.5 -> 16.5 us, n = 304 28.7 -> 26.6), unless three and more blocks fit an
+// SM but not all of two launches: the blocks that become resident early, during
+// the launch before, then leave some SMs three and others one (n = 240 37.2 us
+// against 28.7).  Above that a plain one: early blocks pile up on some SMs (m =
+// 512, n = 600 40.9 us against 26.8), and with a fixed stride over the
+// instances those with one instance more end up on the same ones (1024 of m =
+// 1024 108 us against 99.6).
+bool ntt_dependent(uint32_t n, int per_sm) {
+    const uint32_t sms = uint32_t(sm_count());
+    return n <= 2 * sms && (n <= sms || per_sm <= 2 || 2 * n <= sms * uint32_t(per_sm) || n == 2 * sms);
+}
+
+namespace {
+
 template <int LG, int NP>
 mi_status launch_lg(const uint64_t* a, const uint64_t* b, uint64_t* r, uint32_t n, uint32_t m, uint32_t rlen,
                     const NttMulParams& P, cudaStream_t st) {
@@ -122,14 +139,7 @@ mi_status launch_lg(const uint64_t* a, const uint64_t* b, uint64_t* r, uint32_t 
     MI_TRY(site[low].get(kern, S::NT, S::SMEM, &per_sm));
     uint64_t blocks = uint64_t(sm_count()) * uint64_t(per_sm);
     if (blocks > n) blocks = n;
-    // Up to two instances per SM, a programmatic dependent launch (m = 1024,
-    // n = 152 18.5 -> 16.5 us, n = 304 28.7 -> 27.3).  Above that a plain one:
-    // the blocks of a dependent launch become resident one by one during the
-    // previous launch's tail and pile up on some SMs (m = 512, n = 600 40.9 us
-    // against 26.8), and with a fixed stride over the instances those with one
-    // instance more end up on the same ones (1024 of m = 1024 108 us against
-    // 99.6).
-    if (n <= 2 * uint32_t(sm_count())) {
+    if (ntt_dependent(n, per_sm)) {
         MI_CUDA_TRY(launch_pdl(kern, dim3(uint32_t(blocks)), dim3(S::NT), S::SMEM, st, a, b, r, n, m, rlen, P));
         return MI_OK;
     }

@@ -257,7 +257,7 @@ mi_status launch_lg(const uint64_t* a, const uint64_t* b, uint64_t* r, uint32_t 
     MI_TRY(site.get(kern, NT, smem, &per_sm));
     uint64_t blocks = uint64_t(sm_count()) * uint64_t(per_sm);
     if (blocks > n) blocks = n;
-    if (n <= 2 * uint32_t(sm_count())) {  // as the products do (ntt_mul.cu)
+    if (ntt_dependent(n, per_sm)) {  // as the products do
         MI_CUDA_TRY(launch_pdl(kern, dim3(uint32_t(blocks)), dim3(NT), smem, st, a, b, r, n, m, P));
         return MI_OK;
     }

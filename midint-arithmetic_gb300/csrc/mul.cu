@@ -16,10 +16,13 @@
 // of fewer than 16 threads serve only those launches (mul_flex.cu the others:
 // over the host link 100000 x 4 limbs take 88 us here, 140 there).
 #include <cstdio>
+#include <map>
+#include <mutex>
 
 #include "common.cuh"
 #include "kernels.h"
 #include "mul_core.cuh"
+#include "places.h"
 
 namespace mi {
 namespace {
@@ -130,19 +133,34 @@ __global__ void __launch_bounds__(MulShape<NT, WB>::BLOCK, MulShape<NT, WB>::MIN
     }
 }
 
+// The current device's shared memory, looked up once per device (four queries
+// cost a launch about a microsecond).
+mi_status smem_limits(SmemLimits* out) {
+    static std::mutex mu;
+    static std::map<int, SmemLimits> known;
+    int dev = 0, per_sm = 0, reserved = 0, per_block = 0;
+    MI_CUDA_TRY(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mu);
+    const auto it = known.find(dev);
+    if (it != known.end()) {
+        *out = it->second;
+        return MI_OK;
+    }
+    MI_CUDA_TRY(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+    MI_CUDA_TRY(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev));
+    MI_CUDA_TRY(cudaDeviceGetAttribute(&per_block, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    *out = known[dev] = SmemLimits{size_t(per_sm), size_t(reserved), size_t(per_block)};
+    return MI_OK;
+}
+
 // Dynamic shared memory that leaves room for at most max_per_sm blocks of a
 // kernel per SM (at least `smem`, at most the per-block maximum).
 mi_status capped_smem(size_t smem, uint32_t max_per_sm, size_t* out) {
     *out = smem;
     if (max_per_sm == 0) return MI_OK;
-    int dev = 0, per_sm = 0, reserved = 0, per_block = 0;
-    MI_CUDA_TRY(cudaGetDevice(&dev));
-    MI_CUDA_TRY(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
-    MI_CUDA_TRY(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev));
-    MI_CUDA_TRY(cudaDeviceGetAttribute(&per_block, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    // max_per_sm + 1 blocks of `need` bytes (plus the reservation) overflow the SM
-    const size_t need = size_t(per_sm) / (max_per_sm + 1) + 1024 - size_t(reserved);
-    if (need > *out) *out = need < size_t(per_block) ? need : size_t(per_block);
+    SmemLimits L;
+    MI_TRY(smem_limits(&L));
+    *out = smem_for_places(L, smem, max_per_sm);
     return MI_OK;
 }
 

@@ -51,6 +51,10 @@ uint32_t add_size_class(uint64_t bytes);
 mi_status launch_mul_classic(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32,
                              bool full, cudaStream_t st, uint32_t max_per_sm = 0);
 
+// Dynamic shared memory that leaves room for at most max_per_sm blocks of a
+// kernel per SM (at least `smem`, at most the per-block maximum; 0: `smem`).
+mi_status capped_smem(size_t smem, uint32_t max_per_sm, size_t* out);
+
 // Dynamic shared memory (at least *smem) for a launch of one-warp blocks that
 // keeps the next launch's early blocks from crowding one scheduler.
 mi_status balanced_smem(uint64_t blocks, uint32_t resident, size_t* smem);

@@ -153,17 +153,6 @@ mi_status smem_limits(SmemLimits* out) {
     return MI_OK;
 }
 
-// Dynamic shared memory that leaves room for at most max_per_sm blocks of a
-// kernel per SM (at least `smem`, at most the per-block maximum).
-mi_status capped_smem(size_t smem, uint32_t max_per_sm, size_t* out) {
-    *out = smem;
-    if (max_per_sm == 0) return MI_OK;
-    SmemLimits L;
-    MI_TRY(smem_limits(&L));
-    *out = smem_for_places(L, smem, max_per_sm);
-    return MI_OK;
-}
-
 template <int NT, bool VEC, bool WB>
 mi_status launch_shape(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32,
                        cudaStream_t st, uint32_t max_per_sm) {
@@ -210,6 +199,15 @@ mi_status dispatch(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n
 }
 
 }  // namespace
+
+mi_status capped_smem(size_t smem, uint32_t max_per_sm, size_t* out) {
+    *out = smem;
+    if (max_per_sm == 0) return MI_OK;
+    SmemLimits L;
+    MI_TRY(smem_limits(&L));
+    *out = smem_for_places(L, smem, max_per_sm);
+    return MI_OK;
+}
 
 // A launch of w one-warp blocks per SM where `resident` fit: the next launch of
 // a stream of them starts early on the places that are left, its last blocks

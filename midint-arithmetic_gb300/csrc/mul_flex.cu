@@ -65,8 +65,8 @@ __global__ void __launch_bounds__(32, MB)
 
 }  // namespace
 
-// Blocks of a shape resident per SM: 16 to 21 for the registers, and what the
-// shared memory allows.
+// Blocks of a shape resident per SM: 18 for the registers of the launches that
+// do not fill the GPU, and what the shared memory allows.
 static uint32_t flex_resident(const FlexShape& S) {
     return std::min<uint32_t>(18, uint32_t(228 * 1024 / (S.smem() + 1024)));
 }
@@ -77,13 +77,10 @@ static uint32_t flex_resident(const FlexShape& S) {
 // per step: 0.164 for k_mul, which is 0.92 of that where nb
 // fills the group, 0.173 and 0.178 for one round, 0.16 for two and 0.15 for
 // three, whose steps share the staging).  k_mul_lo's blocks of eight warps come
-// in pairs of warps per scheduler, and with 13 to 15 warps per SM the third
-// block of a launch meets the first of the next (4256 x 233 words 35.4 us,
-// 4864 x 233 25.5).  More rounds need more shared memory: a second wave of
+// in pairs of warps per scheduler.  More rounds need more shared memory: a second wave of
 // blocks costs its own latency.  Power-of-two groups of fewer than 16 threads
 // serve no launches here.  Against what this replaced, the same with
-// warps / 4 unrounded: 1824 x 177 words 24.4 -> 15.5, 3952 x 177 42.8 -> 30.0,
-// low halves of 3648 x 233 32.5 -> 21.7, 1824 x 511 62 -> 43.
+// warps / 4 unrounded: 1824 x 177 words 24.4 -> 15.5, 3952 x 177 42.8 -> 30.0.
 uint32_t flex_rounds(uint32_t n, uint32_t n32, bool full, double* us) {
     constexpr double kA[2] = {0.18, 0.145}, kB[2] = {0.166, 0.164};  // [full]: the power-of-two groups
     constexpr double kFlexA[2][4] = {{0, 0.16, 0.20, 0.19}, {0, 0.18, 0.18, 0.19}};  // [full][rounds]
@@ -97,7 +94,7 @@ uint32_t flex_rounds(uint32_t n, uint32_t n32, bool full, double* us) {
     if (threads >= 16) {
         const double w = std::ceil(double(n) * threads / 32) / sms;  // warps per SM
         double k = std::ceil(w / 4);
-        if (!full) k = w > 12 && w < 16 ? 6 : 2 * std::ceil(w / 8);
+        if (!full) k = 2 * std::ceil(w / 8);
         best = steps * (kA[full] + kB[full] * k);
         if (nb == (full ? threads : 2 * threads)) best *= 0.92;
     }

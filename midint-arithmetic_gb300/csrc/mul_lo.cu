@@ -61,11 +61,23 @@ __global__ void __launch_bounds__(NH > 256 ? NH : 256, 3)
     }
 }
 
+// Places per SM for n products of NH threads: two where the launch's blocks of
+// eight warps take more than one and a half and less than two of the three that
+// fit, else as many as fit (0).  With the third free, early blocks of the next
+// launch of a stream took it beside two of this one, and the next launch's last
+// blocks found one scheduler with six warps (in a stream 2280 x 383
+// words 52.2 us, with two places 37.2; 4560 x 255 35.5 and 25.3; a call alone is
+// the same, 48.8 and 37.0 with its launch).
+uint32_t lo_places(uint32_t n, uint32_t threads) {
+    const double blocks = double(n) * threads / 256 / sm_count();
+    return threads <= 256 && blocks > 1.5 && blocks <= 2 ? 2 : 0;
+}
+
 template <bool VEC>
 mi_status dispatch(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32, cudaStream_t st) {
     switch (lo_threads(n32)) {
 #define MI_LO_CASE(NH) \
-    case NH: return launch_lo<NH>(k_mul_lo<NH, VEC>, a, b, r, n, n32, st);
+    case NH: return launch_lo<NH>(k_mul_lo<NH, VEC>, a, b, r, n, n32, st, lo_places(n, NH));
         MI_LO_CASE(16) MI_LO_CASE(32) MI_LO_CASE(64) MI_LO_CASE(128) MI_LO_CASE(256)
 #undef MI_LO_CASE
         default: return set_error(MI_EINVAL, "mul: %u u32 limbs outside the range of the power-of-two groups", n32);

@@ -24,13 +24,15 @@ using LoKernel = void (*)(const uint32_t*, const uint32_t*, uint32_t*, uint32_t,
 // with pdl_wait) with launch_pdl.
 template <int NH>
 mi_status launch_lo(LoKernel kern, const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32,
-                    cudaStream_t st) {
+                    cudaStream_t st, uint32_t max_per_sm = 0) {
     using S = LoShape<NH>;
-    MI_TRY(ensure_dyn_smem(kern, S::SMEM));
+    size_t smem = S::SMEM;
+    MI_TRY(capped_smem(S::SMEM, max_per_sm, &smem));
+    MI_TRY(ensure_dyn_smem(kern, smem));
     uint64_t blocks = (uint64_t(n) + S::IPB - 1) / S::IPB;
     const uint64_t cap = uint64_t(sm_count()) * 32;
     if (blocks > cap) blocks = cap;
-    MI_CUDA_TRY(launch_pdl(kern, dim3(uint32_t(blocks)), dim3(S::BLOCK), S::SMEM, st, a, b, r, n, n32));
+    MI_CUDA_TRY(launch_pdl(kern, dim3(uint32_t(blocks)), dim3(S::BLOCK), smem, st, a, b, r, n, n32));
     return MI_OK;
 }
 

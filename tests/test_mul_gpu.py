@@ -191,3 +191,18 @@ def test_mul_balanced_launches(ctx, devmem, m, full, n):
     want = O.mul(a, b, m, full)
     for _ in range(2):
         assert np.array_equal(gpu_mul(ctx, devmem, a, b, m, full, limb_bits=32), want)
+
+
+@pytest.mark.parametrize("m", [193, 255, 256, 383, 511])
+def test_mul_lo_places(ctx, devmem, m):
+    # low halves of 25 to 64 blocks in batches on either side of those whose
+    # launches keep two places per SM (more than one and a half blocks, at most
+    # two), two launches in a row
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    per_block = 256 // (16 if m <= 256 else 32)
+    for blocks in (sms * 3 // 2, sms * 3 // 2 + 1, 2 * sms, 2 * sms + 1):
+        n = blocks * per_block - 1
+        a, b = carry_stress(n, m, seed=blocks + m, dtype=np.uint32)
+        want = O.mul(a, b, m, False)
+        for _ in range(2):
+            assert np.array_equal(gpu_mul(ctx, devmem, a, b, m, False, limb_bits=32), want), n

@@ -14,7 +14,7 @@
 // the group owns limbs [t*Q, t*Q+Q).  GS*Q >= limbs; limbs beyond the instance
 // are zero and never stored.  A block of max(256, GS) threads holds 256/GS
 // groups and strides over the batch.  (Rows that allow no 16-byte access: the
-// group's limbs are dealt in rows instead, k_add_rows.)
+// group's limbs are mostly dealt in rows instead, k_add_rows.)
 #include <cstdio>
 
 #include "common.cuh"
@@ -75,13 +75,16 @@ __device__ __forceinline__ uint4 pack16(const L* v) {
     return t;
 }
 
-// Loads the chunk [start, start+Q) of one 16-byte aligned instance row, zero
-// beyond m.
-template <typename L, int Q>
+// How a thread reaches its limbs: whole 16-byte words of a 16-byte aligned row,
+// consecutive limbs one by one on other rows, or dealt in rows (k_add_rows).
+enum Access : int { WORDS16, LIMBS, ROWS };
+
+// Loads the chunk [start, start+Q) of one instance row, zero beyond m.
+template <typename L, int Q, int ACCESS>
 __device__ __forceinline__ void load_chunk(const L* __restrict__ row, uint32_t start, uint32_t m, bool valid,
                                            L (&v)[Q]) {
     constexpr int PER = 16 / sizeof(L);
-    if (valid && start + Q <= m) {
+    if (ACCESS == WORDS16 && valid && start + Q <= m) {
         const uint4* p = reinterpret_cast<const uint4*>(row + start);
 #pragma unroll
         for (int k = 0; k < Q / PER; ++k) {
@@ -94,12 +97,12 @@ __device__ __forceinline__ void load_chunk(const L* __restrict__ row, uint32_t s
     for (int q = 0; q < Q; ++q) v[q] = (valid && start + q < m) ? ld_stream(row + start + q) : L(0);
 }
 
-template <typename L, int Q>
+template <typename L, int Q, int ACCESS>
 __device__ __forceinline__ void store_chunk(L* __restrict__ row, uint32_t start, uint32_t m, bool valid,
                                             const L (&v)[Q]) {
     constexpr int PER = 16 / sizeof(L);
     if (!valid) return;
-    if (start + Q <= m) {
+    if (ACCESS == WORDS16 && start + Q <= m) {
         uint4* p = reinterpret_cast<uint4*>(row + start);
 #pragma unroll
         for (int k = 0; k < Q / PER; ++k) __stcs(p + k, pack16<L, Q>(&v[k * PER]));
@@ -139,7 +142,7 @@ __device__ __forceinline__ uint64_t group_shift_up(uint64_t v, uint32_t t, uint6
     }
 }
 
-template <typename L, int Q, int GS, int OP>
+template <typename L, int Q, int GS, int ACCESS, int OP>
 __global__ void __launch_bounds__(GS > 256 ? GS : 256)
     k_add(const L* __restrict__ a, const L* __restrict__ b, L* __restrict__ r, uint8_t* __restrict__ carry,
           uint32_t n, uint32_t m) {
@@ -159,8 +162,8 @@ __global__ void __launch_bounds__(GS > 256 ? GS : 256)
         const bool valid = inst < n;
         const uint64_t off = valid ? inst * m : 0;
         L x[Q], y[Q], s[Q];
-        load_chunk<L, Q>(a + off, start, m, valid, x);
-        load_chunk<L, Q>(b + off, start, m, valid, y);
+        load_chunk<L, Q, ACCESS>(a + off, start, m, valid, x);
+        load_chunk<L, Q, ACCESS>(b + off, start, m, valid, y);
         uint32_t gc;
         if constexpr (OP == ADD_PLAIN) {
             gc = group_add<L, Q, GS>(x, y, s, scratch);
@@ -184,7 +187,7 @@ __global__ void __launch_bounds__(GS > 256 ? GS : 256)
             for (int q = 1; q < Q; ++q) sh[q] = hi[q - 1];
             gc = group_add<L, Q, GS>(lo, sh, s, scratch);
         }
-        store_chunk<L, Q>(r + off, start, m, valid, s);
+        store_chunk<L, Q, ACCESS>(r + off, start, m, valid, s);
         if (OP == ADD_PLAIN && carry != nullptr && valid) {
             // The carry-out is the value left at limb position m (a padding
             // limb of zeros plus the carry), or the group's carry-out when the
@@ -618,7 +621,7 @@ mi_status launch_wide(const L* a, const L* b, L* r, uint8_t* carry, uint32_t n, 
     return MI_OK;
 }
 
-template <typename L, int Q, int GS, bool VEC, int OP>
+template <typename L, int Q, int GS, int ACCESS, int OP>
 mi_status launch_one(const L* a, const L* b, L* r, uint8_t* carry, uint32_t n, uint32_t m, cudaStream_t st) {
     constexpr int BLOCK = GS > 256 ? GS : 256;
     constexpr int IPB = BLOCK / GS;
@@ -626,29 +629,30 @@ mi_status launch_one(const L* a, const L* b, L* r, uint8_t* carry, uint32_t n, u
     // Enough blocks for full residency several times over; the kernel strides.
     const uint64_t cap = uint64_t(sm_count()) * 64;
     if (blocks > cap) blocks = cap;
-    if constexpr (VEC)
-        MI_CUDA_TRY(launch_pdl(k_add<L, Q, GS, OP>, dim3(uint32_t(blocks)), dim3(BLOCK), 0, st, a, b, r, carry, n, m));
-    else
+    if constexpr (ACCESS == ROWS)
         MI_CUDA_TRY(
             launch_pdl(k_add_rows<L, Q, GS, OP>, dim3(uint32_t(blocks)), dim3(BLOCK), 0, st, a, b, r, carry, n, m));
+    else
+        MI_CUDA_TRY(launch_pdl(k_add<L, Q, GS, ACCESS, OP>, dim3(uint32_t(blocks)), dim3(BLOCK), 0, st, a, b, r, carry,
+                               n, m));
     return MI_OK;
 }
 
-template <typename L, bool VEC, int OP, int Q>
+template <typename L, int ACCESS, int OP, int Q>
 mi_status dispatch_gs(const L* a, const L* b, L* r, uint8_t* carry, uint32_t n, uint32_t m, uint32_t gs,
                       cudaStream_t st) {
     switch (gs) {
-        case 1: return launch_one<L, Q, 1, VEC, OP>(a, b, r, carry, n, m, st);
-        case 2: return launch_one<L, Q, 2, VEC, OP>(a, b, r, carry, n, m, st);
-        case 4: return launch_one<L, Q, 4, VEC, OP>(a, b, r, carry, n, m, st);
-        case 8: return launch_one<L, Q, 8, VEC, OP>(a, b, r, carry, n, m, st);
-        case 16: return launch_one<L, Q, 16, VEC, OP>(a, b, r, carry, n, m, st);
-        case 32: return launch_one<L, Q, 32, VEC, OP>(a, b, r, carry, n, m, st);
-        case 64: return launch_one<L, Q, 64, VEC, OP>(a, b, r, carry, n, m, st);
-        case 128: return launch_one<L, Q, 128, VEC, OP>(a, b, r, carry, n, m, st);
-        case 256: return launch_one<L, Q, 256, VEC, OP>(a, b, r, carry, n, m, st);
-        case 512: return launch_one<L, Q, 512, VEC, OP>(a, b, r, carry, n, m, st);
-        case 1024: return launch_one<L, Q, 1024, VEC, OP>(a, b, r, carry, n, m, st);
+        case 1: return launch_one<L, Q, 1, ACCESS, OP>(a, b, r, carry, n, m, st);
+        case 2: return launch_one<L, Q, 2, ACCESS, OP>(a, b, r, carry, n, m, st);
+        case 4: return launch_one<L, Q, 4, ACCESS, OP>(a, b, r, carry, n, m, st);
+        case 8: return launch_one<L, Q, 8, ACCESS, OP>(a, b, r, carry, n, m, st);
+        case 16: return launch_one<L, Q, 16, ACCESS, OP>(a, b, r, carry, n, m, st);
+        case 32: return launch_one<L, Q, 32, ACCESS, OP>(a, b, r, carry, n, m, st);
+        case 64: return launch_one<L, Q, 64, ACCESS, OP>(a, b, r, carry, n, m, st);
+        case 128: return launch_one<L, Q, 128, ACCESS, OP>(a, b, r, carry, n, m, st);
+        case 256: return launch_one<L, Q, 256, ACCESS, OP>(a, b, r, carry, n, m, st);
+        case 512: return launch_one<L, Q, 512, ACCESS, OP>(a, b, r, carry, n, m, st);
+        case 1024: return launch_one<L, Q, 1024, ACCESS, OP>(a, b, r, carry, n, m, st);
         default: return set_error(MI_EINVAL, "add: %u limbs exceeds the single-group maximum", m);
     }
 }
@@ -663,9 +667,9 @@ mi_status dispatch_vec(const L* a, const L* b, L* r, uint8_t* carry, uint32_t n,
     uint32_t q = thread_bytes >= 64 ? 4 * QS : (thread_bytes >= 32 ? 2 * QS : QS);
     while (q < 4 * QS && pow2ceil((m + q - 1) / q) > 1024) q *= 2;
     const uint32_t gs = pow2ceil((m + q - 1) / q);
-    if (q == QS) return dispatch_gs<L, true, OP, QS>(a, b, r, carry, n, m, gs, st);
-    if (q == 2 * QS) return dispatch_gs<L, true, OP, 2 * QS>(a, b, r, carry, n, m, gs, st);
-    return dispatch_gs<L, true, OP, 4 * QS>(a, b, r, carry, n, m, gs, st);
+    if (q == QS) return dispatch_gs<L, WORDS16, OP, QS>(a, b, r, carry, n, m, gs, st);
+    if (q == 2 * QS) return dispatch_gs<L, WORDS16, OP, 2 * QS>(a, b, r, carry, n, m, gs, st);
+    return dispatch_gs<L, WORDS16, OP, 4 * QS>(a, b, r, carry, n, m, gs, st);
 }
 
 // Rows per thread of k_add_rows: four (two leave too little in flight, eight too
@@ -691,16 +695,46 @@ uint32_t rows_per_thread(uint32_t m) {
 }
 
 template <typename L, int OP>
-mi_status dispatch_rows(const L* a, const L* b, L* r, uint8_t* carry, uint32_t n, uint32_t m, cudaStream_t st) {
-    const uint32_t q = rows_per_thread<L>(m), gs = pow2ceil((m + q - 1) / q);
+mi_status dispatch_rows(const L* a, const L* b, L* r, uint8_t* carry, uint32_t n, uint32_t m, uint32_t q,
+                        cudaStream_t st) {
+    const uint32_t gs = pow2ceil((m + q - 1) / q);
     switch (q) {
-        case 2: return dispatch_gs<L, false, OP, 2>(a, b, r, carry, n, m, gs, st);
-        case 3: return dispatch_gs<L, false, OP, 3>(a, b, r, carry, n, m, gs, st);
-        case 4: return dispatch_gs<L, false, OP, 4>(a, b, r, carry, n, m, gs, st);
-        case 5: return dispatch_gs<L, false, OP, 5>(a, b, r, carry, n, m, gs, st);
-        case 6: return dispatch_gs<L, false, OP, 6>(a, b, r, carry, n, m, gs, st);
-        default: return dispatch_gs<L, false, OP, 8>(a, b, r, carry, n, m, gs, st);
+        case 2: return dispatch_gs<L, ROWS, OP, 2>(a, b, r, carry, n, m, gs, st);
+        case 3: return dispatch_gs<L, ROWS, OP, 3>(a, b, r, carry, n, m, gs, st);
+        case 4: return dispatch_gs<L, ROWS, OP, 4>(a, b, r, carry, n, m, gs, st);
+        case 5: return dispatch_gs<L, ROWS, OP, 5>(a, b, r, carry, n, m, gs, st);
+        case 6: return dispatch_gs<L, ROWS, OP, 6>(a, b, r, carry, n, m, gs, st);
+        default: return dispatch_gs<L, ROWS, OP, 8>(a, b, r, carry, n, m, gs, st);
     }
+}
+
+// 6a + 10b on rows that allow no 16-byte access.  A row of k_add_rows costs two
+// 64-bit shuffles more than in a plain addition, so lengths that fill the group
+// well take consecutive limbs per thread instead (one shuffle per thread), two
+// or four of them; the others three rows, or five where those pad less (us per
+// 2^22 limbs with the rows of the plain addition against these: 13 limbs 22.3 ->
+// 20.4, 29 21.5 -> 18.7, 63 20.2 -> 17.0, 99 23.1 -> 19.6, 127 23.1 -> 17.0, 129 26.2 -> 20.8,
+// 191 26.4 -> 21.1, 255 23.8 -> 21.5, 333 29.4 -> 24.6, 385 27.4 -> 23.3, 511 24.5 -> 20.3, 641 26.5 ->
+// 22.7, 1001 22.4 -> 19.9, 2049 46.4 -> 28.2, 4095 31.7 -> 29.6).
+struct SixForm {
+    uint32_t up_to;  // limbs
+    int access;
+    uint32_t q;      // rows, or limbs, per thread
+};
+constexpr SixForm kSixForms[] = {
+    {2, ROWS, 2},    {3, ROWS, 3},     {4, ROWS, 2},     {6, ROWS, 3},    {8, ROWS, 4},    {12, ROWS, 3},
+    {16, ROWS, 2},   {24, ROWS, 3},    {29, LIMBS, 4},   {32, ROWS, 2},   {48, ROWS, 3},   {64, LIMBS, 2},
+    {88, ROWS, 3},   {128, LIMBS, 4},  {160, ROWS, 5},   {192, ROWS, 3},  {256, LIMBS, 2}, {384, ROWS, 3},
+    {512, LIMBS, 2}, {768, ROWS, 3},   {1024, LIMBS, 4}, {1280, ROWS, 5}, {1536, ROWS, 3}, {2048, ROWS, 4},
+    {2560, ROWS, 5}, {3072, ROWS, 3},  {kAddMaxLimbs64, ROWS, 4}};
+
+mi_status dispatch_six(const uint64_t* a, const uint64_t* b, uint64_t* r, uint32_t n, uint32_t m, cudaStream_t st) {
+    const SixForm* f = kSixForms;
+    while (m > f->up_to) ++f;  // m <= kAddMaxLimbs64
+    if (f->access == ROWS) return dispatch_rows<uint64_t, ADD_SIX>(a, b, r, nullptr, n, m, f->q, st);
+    const uint32_t gs = pow2ceil((m + f->q - 1) / f->q);
+    return f->q == 2 ? dispatch_gs<uint64_t, LIMBS, ADD_SIX, 2>(a, b, r, nullptr, n, m, gs, st)
+                     : dispatch_gs<uint64_t, LIMBS, ADD_SIX, 4>(a, b, r, nullptr, n, m, gs, st);
 }
 
 }  // namespace
@@ -725,9 +759,9 @@ mi_status launch_add_u64(const uint64_t* a, const uint64_t* b, uint64_t* r, uint
     }
     if (op == ADD_SIX)
         return vec ? dispatch_vec<uint64_t, ADD_SIX>(a, b, r, nullptr, n, limbs, thread_bytes, st)
-                   : dispatch_rows<uint64_t, ADD_SIX>(a, b, r, nullptr, n, limbs, st);
+                   : dispatch_six(a, b, r, n, limbs, st);
     return vec ? dispatch_vec<uint64_t, ADD_PLAIN>(a, b, r, carry, n, limbs, thread_bytes, st)
-               : dispatch_rows<uint64_t, ADD_PLAIN>(a, b, r, carry, n, limbs, st);
+               : dispatch_rows<uint64_t, ADD_PLAIN>(a, b, r, carry, n, limbs, rows_per_thread<uint64_t>(limbs), st);
 }
 
 mi_status launch_add_u32(const uint32_t* a, const uint32_t* b, uint32_t* r, uint8_t* carry, uint32_t n,
@@ -743,7 +777,7 @@ mi_status launch_add_u32(const uint32_t* a, const uint32_t* b, uint32_t* r, uint
         return launch_wide<uint32_t, false, ADD_PLAIN>(a, b, r, carry, n, limbs, *wide, st);
     }
     // Odd limb counts (or 4-byte aligned rows) cannot use 128-bit accesses.
-    return dispatch_rows<uint32_t, ADD_PLAIN>(a, b, r, carry, n, limbs, st);
+    return dispatch_rows<uint32_t, ADD_PLAIN>(a, b, r, carry, n, limbs, rows_per_thread<uint32_t>(limbs), st);
 }
 
 }  // namespace mi

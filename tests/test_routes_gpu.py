@@ -1,0 +1,53 @@
+"""Which kernels a call launches: the call is captured into a graph, which is
+printed, so that nothing runs.  (The results are checked where the operations
+are; here it is the choice between equal results.)"""
+from __future__ import annotations
+
+import ctypes
+import re
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def route(ctx, tmp_path):
+    """route(call): the names of the kernels that call(stream) launches."""
+    cudart = ctypes.CDLL("libcudart.so.13")  # the one that the library is linked with
+    stream = torch.cuda.Stream()
+
+    def check(status):
+        assert status == 0, status
+
+    def run(call):
+        s, graph = ctypes.c_void_p(stream.cuda_stream), ctypes.c_void_p()
+        path = tmp_path / "graph.dot"
+        check(cudart.cudaStreamBeginCapture(s, 2))  # relaxed
+        try:
+            call(stream.cuda_stream)
+        finally:
+            check(cudart.cudaStreamEndCapture(s, ctypes.byref(graph)))
+        check(cudart.cudaGraphDebugDotPrint(graph, str(path).encode(), 1))  # verbose
+        check(cudart.cudaGraphDestroy(graph))
+        # mangled: a name is preceded by its length
+        return {name[:int(n)] for n, name in re.findall(r"(\d+)(k_[A-Za-z0-9_]+)", path.read_text())}
+
+    return run
+
+
+def buffers(words, count=3, offset=0):
+    """Buffers of `words` 32-bit words, `offset` words past a 16-byte boundary."""
+    keep = [torch.zeros(words + 4, dtype=torch.int32, device="cuda:0") for _ in range(count)]
+    return keep, [k.data_ptr() + 4 * offset for k in keep]
+
+
+@pytest.mark.parametrize("m,kernel", [(28, "k_add"), (29, "k_add"), (30, "k_add_rows"), (48, "k_add_rows"),
+                                      (63, "k_add"), (127, "k_add"), (129, "k_add_rows"), (255, "k_add"),
+                                      (333, "k_add_rows"), (511, "k_add"), (1001, "k_add"), (4095, "k_add_rows")])
+def test_add6_on_unaligned_rows(ctx, route, m, kernel):
+    # lengths that fill their group take consecutive limbs per thread
+    keep, (a, b, r) = buffers(2 * m * 100, offset=2)
+    assert route(lambda s: ctx.add6(a, b, r, 100, m, stream=s)) == {kernel}
+    del keep

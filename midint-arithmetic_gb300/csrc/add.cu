@@ -737,6 +737,23 @@ mi_status dispatch_six(const uint64_t* a, const uint64_t* b, uint64_t* r, uint32
                      : dispatch_gs<uint64_t, LIMBS, ADD_SIX, 4>(a, b, r, nullptr, n, m, gs, st);
 }
 
+// A plain addition on rows that allow no 16-byte access.  With operands over the
+// host link and results in device memory (link) consecutive limbs, 16 bytes of
+// them per thread, from 3 u64 or 13 u32 limbs on while they fit a group: the rows'
+// short runs of lanes ask the link for the same 32 bytes more than once (us for
+// 2^20 u64 or 2^21 u32 limbs with rows against these: 5 limbs 152 -> 144, 9 182 ->
+// 144, 17 163 -> 143, 127 144 -> 142; 17 words 179 -> 143, 65 161 -> 143, 1001 155 -> 143;
+// one limb 143 against 150, 9 words 142 against 144).  Results over the link want the
+// rows' contiguous stores (1024 x 2047 words 141 against 301).
+template <typename L>
+mi_status dispatch_plain(const L* a, const L* b, L* r, uint8_t* carry, uint32_t n, uint32_t m, bool link,
+                         cudaStream_t st) {
+    constexpr uint32_t Q = 16 / sizeof(L);
+    if (link && m >= (sizeof(L) == 8 ? 3 : 13) && m <= Q * 1024)
+        return dispatch_gs<L, LIMBS, ADD_PLAIN, int(Q)>(a, b, r, carry, n, m, pow2ceil((m + Q - 1) / Q), st);
+    return dispatch_rows<L, ADD_PLAIN>(a, b, r, carry, n, m, rows_per_thread<L>(m), st);
+}
+
 }  // namespace
 
 uint32_t add_size_class(uint64_t bytes) {
@@ -747,7 +764,7 @@ uint32_t add_size_class(uint64_t bytes) {
 }
 
 mi_status launch_add_u64(const uint64_t* a, const uint64_t* b, uint64_t* r, uint8_t* carry, uint32_t n,
-                         uint32_t limbs, int op, uint32_t thread_bytes, cudaStream_t st, WideState* wide) {
+                         uint32_t limbs, int op, uint32_t thread_bytes, cudaStream_t st, WideState* wide, bool link) {
     const bool vec = aligned16(a) && aligned16(b) && aligned16(r) && (limbs % 2 == 0);
     if (limbs > kAddMaxLimbs64) {
         if (wide == nullptr || wide->status == nullptr) return set_error(MI_EINVAL, "add: no multi-block state");
@@ -761,23 +778,23 @@ mi_status launch_add_u64(const uint64_t* a, const uint64_t* b, uint64_t* r, uint
         return vec ? dispatch_vec<uint64_t, ADD_SIX>(a, b, r, nullptr, n, limbs, thread_bytes, st)
                    : dispatch_six(a, b, r, n, limbs, st);
     return vec ? dispatch_vec<uint64_t, ADD_PLAIN>(a, b, r, carry, n, limbs, thread_bytes, st)
-               : dispatch_rows<uint64_t, ADD_PLAIN>(a, b, r, carry, n, limbs, rows_per_thread<uint64_t>(limbs), st);
+               : dispatch_plain<uint64_t>(a, b, r, carry, n, limbs, link, st);
 }
 
 mi_status launch_add_u32(const uint32_t* a, const uint32_t* b, uint32_t* r, uint8_t* carry, uint32_t n,
-                         uint32_t limbs, uint32_t thread_bytes, cudaStream_t st, WideState* wide) {
+                         uint32_t limbs, uint32_t thread_bytes, cudaStream_t st, WideState* wide, bool link) {
     // An even number of u32 limbs on 8-byte aligned rows is the same bytes as
     // half as many u64 limbs, with the same carry-out.
     if (limbs % 2 == 0 && aligned8(a) && aligned8(b) && aligned8(r))
         return launch_add_u64(reinterpret_cast<const uint64_t*>(a), reinterpret_cast<const uint64_t*>(b),
                               reinterpret_cast<uint64_t*>(r), carry, n, limbs / 2, ADD_PLAIN, thread_bytes, st,
-                              wide);
+                              wide, link);
     if (limbs > 2 * kAddMaxLimbs64) {
         if (wide == nullptr || wide->status == nullptr) return set_error(MI_EINVAL, "add: no multi-block state");
         return launch_wide<uint32_t, false, ADD_PLAIN>(a, b, r, carry, n, limbs, *wide, st);
     }
     // Odd limb counts (or 4-byte aligned rows) cannot use 128-bit accesses.
-    return dispatch_rows<uint32_t, ADD_PLAIN>(a, b, r, carry, n, limbs, rows_per_thread<uint32_t>(limbs), st);
+    return dispatch_plain<uint32_t>(a, b, r, carry, n, limbs, link, st);
 }
 
 }  // namespace mi

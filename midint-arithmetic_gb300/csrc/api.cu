@@ -283,9 +283,9 @@ mi_status wide_status(mi_ctx ctx) {
     return set_error(MI_ETIMEOUT, "a multi-block addition gave up waiting for a predecessor tile");
 }
 
-// Runs `launch(da, db, dr, dcarry, count, stream, max_per_sm)` over a batch of
-// host buffers, with the tuning of operation class `cls` (max_per_sm is the
-// class's zero-copy occupancy cap in mode 1, else 0).  Zero-copy mode 2 with
+// Runs `launch(da, db, dr, dcarry, count, stream, how)` over a batch of host
+// buffers, with the tuning of operation class `cls` (`how`: the class's zero-copy
+// occupancy cap in mode 1, and what the kernel reaches over the host link).  Zero-copy mode 2 with
 // mapped pinned operands: the kernels read the operands in place and only the
 // results go through the staging slots and the copy-out stream (the two
 // directions of the host link then run at once).  Zero-copy mode 1 with
@@ -300,6 +300,10 @@ mi_status wide_status(mi_ctx ctx) {
 // copy-out stream, so copies in both
 // directions and the kernels of neighbouring chunks overlap.
 enum { HOST_ADD = 0, HOST_MUL = 1 };  // operation classes of the host tuning knobs
+struct HostLaunch {
+    uint32_t max_per_sm;
+    bool in, out;  // the operands, the results are host memory
+};
 
 template <typename F>
 mi_status host_pipeline(mi_ctx ctx, int cls, const void* h_a, const void* h_b, void* h_r, uint8_t* h_carry,
@@ -342,7 +346,8 @@ mi_status host_pipeline(mi_ctx ctx, int cls, const void* h_a, const void* h_b, v
         for (int i = 0; i < 4 && go; ++i)
             if (kind[i] == HostKind::Pageable) go = populate_pages(host[i], bytes[i], i >= 2);
         if (go) {
-            MI_TRY(launch(d[0], d[1], d[2], static_cast<uint8_t*>(d[3]), n, ctx->pipe[2], ctx->host_zc_blocks[cls]));
+            MI_TRY(launch(d[0], d[1], d[2], static_cast<uint8_t*>(d[3]), n, ctx->pipe[2],
+                          HostLaunch{ctx->host_zc_blocks[cls], true, true}));
             MI_CUDA_TRY(cudaStreamSynchronize(ctx->pipe[2]));
             return MI_OK;
         }
@@ -385,7 +390,8 @@ mi_status host_pipeline(mi_ctx ctx, int cls, const void* h_a, const void* h_b, v
             // writes the staging slot once its previous copy-out is done
             if (c >= mi_ctx_s::kSlots) MI_CUDA_TRY(cudaStreamWaitEvent(comp, ctx->ev_out[slot], 0));
             MI_TRY(launch(const_cast<char*>(za) + base * in_row, const_cast<char*>(zb) + base * in_row, stg + off_r,
-                          h_carry ? reinterpret_cast<uint8_t*>(stg + off_c) : nullptr, cnt, comp, 0u));
+                          h_carry ? reinterpret_cast<uint8_t*>(stg + off_c) : nullptr, cnt, comp,
+                          HostLaunch{0, true, false}));
         } else {
             // the slot is free once its last reader is done: its copy-out,
             // or in mode 3 the kernel itself
@@ -397,12 +403,13 @@ mi_status host_pipeline(mi_ctx ctx, int cls, const void* h_a, const void* h_b, v
             MI_CUDA_TRY(cudaEventRecord(ctx->ev_in[slot], cin));
             MI_CUDA_TRY(cudaStreamWaitEvent(comp, ctx->ev_in[slot], 0));
             if (zr) {
-                MI_TRY(launch(stg, stg + off_b, zr + base * out_row, zc ? zc + base : nullptr, cnt, comp, 0u));
+                MI_TRY(launch(stg, stg + off_b, zr + base * out_row, zc ? zc + base : nullptr, cnt, comp,
+                              HostLaunch{0, false, true}));
                 MI_CUDA_TRY(cudaEventRecord(ctx->ev_k[slot], comp));
                 continue;
             }
             MI_TRY(launch(stg, stg + off_b, stg + off_r, h_carry ? reinterpret_cast<uint8_t*>(stg + off_c) : nullptr,
-                          cnt, comp, 0u));
+                          cnt, comp, HostLaunch{0, false, false}));
         }
         MI_CUDA_TRY(cudaEventRecord(ctx->ev_k[slot], comp));
         MI_CUDA_TRY(cudaStreamWaitEvent(cout, ctx->ev_k[slot], 0));
@@ -746,9 +753,10 @@ mi_status mi_compat_gpuAdd_u32(int num_instances, uint32_t m, const uint32_t* h_
     const size_t row = size_t(m) * 4;
     const mi_status st = host_pipeline(ctx, HOST_ADD, h_as, h_bs, h_rs, nullptr, uint32_t(num_instances), row, row,
                          [ctx, m, tb = add_bytes(ctx, m, 4)](void* da, void* db, void* dr, uint8_t*, uint32_t cnt,
-                                                              cudaStream_t st, uint32_t) {
+                                                              cudaStream_t st, HostLaunch how) {
                              return launch_add_u32(static_cast<uint32_t*>(da), static_cast<uint32_t*>(db),
-                                                   static_cast<uint32_t*>(dr), nullptr, cnt, m, tb, st, &ctx->wide);
+                                                   static_cast<uint32_t*>(dr), nullptr, cnt, m, tb, st, &ctx->wide,
+                                                   how.in && !how.out);
                          },
                          m > 2 * kAddMaxLimbs64);
     return st == MI_OK && m > 2 * kAddMaxLimbs64 ? wide_status(ctx) : st;
@@ -765,12 +773,12 @@ mi_status mi_compat_gpuMultiply_u64(int num_instances, uint32_t m, const uint64_
                                                                   // kernels see are 8-byte aligned)
     return host_pipeline(ctx, HOST_MUL, h_as, h_bs, h_rs, nullptr, uint32_t(num_instances), row, row,
                          [ctx, m, ntt](void* da, void* db, void* dr, uint8_t*, uint32_t cnt, cudaStream_t st,
-                                       uint32_t cap) {
+                                       HostLaunch how) {
                              if (ntt)
                                  return launch_mul_ntt(static_cast<uint64_t*>(da), static_cast<uint64_t*>(db),
                                                        static_cast<uint64_t*>(dr), cnt, m, ctx->ntt.params, st, true);
                              return launch_mul_classic(static_cast<uint32_t*>(da), static_cast<uint32_t*>(db),
-                                                       static_cast<uint32_t*>(dr), cnt, 2 * m, false, st, cap);
+                                                       static_cast<uint32_t*>(dr), cnt, 2 * m, false, st, how.max_per_sm);
                          });
 }
 
@@ -782,9 +790,9 @@ mi_status mi_compat_gpuMultiply_u32(int num_instances, uint32_t m, const uint32_
     MI_TRY(default_ctx(&ctx));
     const size_t row = size_t(m) * 4;
     return host_pipeline(ctx, HOST_MUL, h_as, h_bs, h_rs, nullptr, uint32_t(num_instances), row, row,
-                         [m](void* da, void* db, void* dr, uint8_t*, uint32_t cnt, cudaStream_t st, uint32_t cap) {
+                         [m](void* da, void* db, void* dr, uint8_t*, uint32_t cnt, cudaStream_t st, HostLaunch how) {
                              return launch_mul_classic(static_cast<uint32_t*>(da), static_cast<uint32_t*>(db),
-                                                       static_cast<uint32_t*>(dr), cnt, m, false, st, cap);
+                                                       static_cast<uint32_t*>(dr), cnt, m, false, st, how.max_per_sm);
                          });
 }
 
@@ -801,7 +809,7 @@ mi_status mi_compat_gpuMulFFT_u16(int num_instances, uint32_t M, const uint16_t*
     const size_t row = size_t(m) * 8;
     // the NTT kernel, storing the low M digits (m limbs) of each product
     return host_pipeline(ctx, HOST_MUL, h_as, h_bs, h_rs, nullptr, uint32_t(num_instances), row, row,
-                         [ctx, m](void* da, void* db, void* dr, uint8_t*, uint32_t cnt, cudaStream_t st, uint32_t) {
+                         [ctx, m](void* da, void* db, void* dr, uint8_t*, uint32_t cnt, cudaStream_t st, HostLaunch) {
                              return launch_mul_ntt(static_cast<uint64_t*>(da), static_cast<uint64_t*>(db),
                                                    static_cast<uint64_t*>(dr), cnt, m, ctx->ntt.params, st, true);
                          });
@@ -895,10 +903,10 @@ mi_status mi_host_add_u64(mi_ctx ctx, const uint64_t* h_a, const uint64_t* h_b, 
     const size_t row = size_t(limbs) * 8;
     const mi_status st = host_pipeline(ctx, HOST_ADD, h_a, h_b, h_r, h_carry, n, row, row,
                          [ctx, limbs, tb = add_bytes(ctx, limbs, 8)](void* da, void* db, void* dr, uint8_t* dc,
-                                                                      uint32_t cnt, cudaStream_t st, uint32_t) {
+                                                                      uint32_t cnt, cudaStream_t st, HostLaunch how) {
                              return launch_add_u64(static_cast<uint64_t*>(da), static_cast<uint64_t*>(db),
                                                    static_cast<uint64_t*>(dr), dc, cnt, limbs, ADD_PLAIN, tb, st,
-                                                   &ctx->wide);
+                                                   &ctx->wide, how.in && !how.out);
                          },
                          limbs > kAddMaxLimbs64);
     return st == MI_OK && limbs > kAddMaxLimbs64 ? wide_status(ctx) : st;
@@ -910,9 +918,9 @@ mi_status mi_host_mul_full_u64(mi_ctx ctx, const uint64_t* h_a, const uint64_t* 
     if (ctx == nullptr) return set_error(MI_EINVAL, "null context");
     const size_t row = size_t(limbs) * 8;
     return host_pipeline(ctx, HOST_MUL, h_a, h_b, h_r, nullptr, n, row, 2 * row,
-                         [limbs](void* da, void* db, void* dr, uint8_t*, uint32_t cnt, cudaStream_t st, uint32_t cap) {
+                         [limbs](void* da, void* db, void* dr, uint8_t*, uint32_t cnt, cudaStream_t st, HostLaunch how) {
                              return launch_mul_classic(static_cast<uint32_t*>(da), static_cast<uint32_t*>(db),
-                                                       static_cast<uint32_t*>(dr), cnt, 2 * limbs, true, st, cap);
+                                                       static_cast<uint32_t*>(dr), cnt, 2 * limbs, true, st, how.max_per_sm);
                          });
 }
 

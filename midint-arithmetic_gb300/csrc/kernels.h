@@ -35,12 +35,14 @@ struct WideState {
 // thread_bytes: operand bytes each thread owns (16, 32 or 64; raised where the
 // instance would need a group of more than 1024 threads).  Instances wider
 // than one group (limbs above kAddMaxLimbs64 u64 limbs) take the multi-block
-// kernel, which needs `wide`.
+// kernel, which needs `wide`.  link: the operands are host memory, read over the
+// host link, and the results are not.
 mi_status launch_add_u64(const uint64_t* a, const uint64_t* b, uint64_t* r, uint8_t* carry, uint32_t n,
                          uint32_t limbs, int op, uint32_t thread_bytes, cudaStream_t st,
-                         WideState* wide = nullptr);
+                         WideState* wide = nullptr, bool link = false);
 mi_status launch_add_u32(const uint32_t* a, const uint32_t* b, uint32_t* r, uint8_t* carry, uint32_t n,
-                         uint32_t limbs, uint32_t thread_bytes, cudaStream_t st, WideState* wide = nullptr);
+                         uint32_t limbs, uint32_t thread_bytes, cudaStream_t st, WideState* wide = nullptr,
+                         bool link = false);
 // Size class of an addition of `bytes` per operand: ceil(log2(u64 limbs)).
 uint32_t add_size_class(uint64_t bytes);
 

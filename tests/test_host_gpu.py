@@ -294,3 +294,28 @@ def test_ordinary_arrays(hctx, mode, n, m):
     odd = np.zeros(4 * n * m + 4, np.uint32)[1:]
     hctx.host_mul_full(a, b, odd[:4 * n * m], n, m)
     assert np.array_equal(odd[:4 * n * m].copy().view(np.uint64), full)
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("n,m", [(700, 1), (700, 3), (700, 5), (300, 13), (300, 127), (9, 2047), (5, 2049), (5, 4095)])
+def test_host_add_on_odd_lengths(hctx, mode, n, m):
+    # rows that allow no 16-byte access, read over the host link or staged
+    hctx.set_tuning(midint.TUNE_HOST_ZERO_COPY, 0, mode)
+    a, b = carry_stress(n, m, seed=n + m)
+    want, carry = O.add(a, b, m)
+    r = torch.zeros(n * m + 1, dtype=torch.int64).pin_memory()
+    c = torch.full((n + 8,), 7, dtype=torch.uint8).pin_memory()
+    hctx.host_add(_pinned(a), _pinned(b), r, c, n, m)
+    assert np.array_equal(r.numpy().view(np.uint64)[:-1], want) and r[-1] == 0
+    assert np.array_equal(c.numpy()[:n], carry) and (c.numpy()[n:] == 7).all()
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+@pytest.mark.parametrize("n,m", [(700, 1), (700, 9), (700, 11), (300, 13), (300, 17), (9, 2049), (5, 4095), (5, 4097),
+                                 (5, 8191)])
+def test_gpuAdd_u32_on_odd_lengths(hctx, pinned, n, m):
+    a, b = carry_stress(n, m, seed=n + m, dtype=np.uint32)
+    keep = [_pinned(x.view(np.int32)) if pinned else x for x in (a, b, np.zeros(n * m, np.uint32))]
+    a2, b2, r = [k.numpy().view(np.uint32) if pinned else k for k in keep]
+    midint.gpuAdd(midint.U32bits, m, n, a2, b2, r)
+    assert np.array_equal(r, O.add(a, b, m)[0])

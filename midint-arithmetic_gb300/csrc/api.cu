@@ -778,7 +778,8 @@ mi_status mi_compat_gpuMultiply_u64(int num_instances, uint32_t m, const uint64_
                                  return launch_mul_ntt(static_cast<uint64_t*>(da), static_cast<uint64_t*>(db),
                                                        static_cast<uint64_t*>(dr), cnt, m, ctx->ntt.params, st, true);
                              return launch_mul_classic(static_cast<uint32_t*>(da), static_cast<uint32_t*>(db),
-                                                       static_cast<uint32_t*>(dr), cnt, 2 * m, false, st, how.max_per_sm);
+                                                       static_cast<uint32_t*>(dr), cnt, 2 * m, false, st, how.max_per_sm,
+                                                       how.in);
                          });
 }
 
@@ -792,7 +793,7 @@ mi_status mi_compat_gpuMultiply_u32(int num_instances, uint32_t m, const uint32_
     return host_pipeline(ctx, HOST_MUL, h_as, h_bs, h_rs, nullptr, uint32_t(num_instances), row, row,
                          [m](void* da, void* db, void* dr, uint8_t*, uint32_t cnt, cudaStream_t st, HostLaunch how) {
                              return launch_mul_classic(static_cast<uint32_t*>(da), static_cast<uint32_t*>(db),
-                                                       static_cast<uint32_t*>(dr), cnt, m, false, st, how.max_per_sm);
+                                                       static_cast<uint32_t*>(dr), cnt, m, false, st, how.max_per_sm, how.in);
                          });
 }
 

@@ -49,9 +49,9 @@ uint32_t add_size_class(uint64_t bytes);
 // Classical multiplication on u32 limb views (a u64 buffer with m limbs is a
 // u32 buffer with 2m limbs).  full: r has 2*n32 limbs per instance, else n32.
 // max_per_sm > 0 caps the full-product kernel's resident blocks per SM (by
-// its shared-memory request).
+// its shared-memory request); link: the operands are read over the host link.
 mi_status launch_mul_classic(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32,
-                             bool full, cudaStream_t st, uint32_t max_per_sm = 0);
+                             bool full, cudaStream_t st, uint32_t max_per_sm = 0, bool link = false);
 
 // Dynamic shared memory that leaves room for at most max_per_sm blocks of a
 // kernel per SM (at least `smem`, at most the per-block maximum; 0: `smem`).
@@ -67,7 +67,7 @@ mi_status balanced_smem(uint64_t blocks, uint32_t resident, size_t* smem);
 // is the modelled time.
 uint32_t flex_rounds(uint32_t n, uint32_t n32, bool full, double* us = nullptr);
 mi_status launch_mul_flex(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32, bool full,
-                          uint32_t rounds, cudaStream_t st);
+                          uint32_t rounds, cudaStream_t st, bool link = false, uint32_t max_per_sm = 0);
 
 // Full products of 25..32 blocks of 8 u32 limbs with one Karatsuba level
 // (mul_kara.cu), and the batches for which that is the fastest form.

@@ -38,7 +38,11 @@ using classic::T;
 // GPU; 18 (96) below that, where two launches then fit the SMs at once and
 // overlap (1500 x 68 limbs 11.5 us against 15.4; 16384 x 68 66.3 against 64.1,
 // low halves of 12000 x 301 words 108 against 104.6).
-template <bool FULL, bool VEC, int MB>
+// LINK: the operands are read over the host link, the warp's rows as one run
+// (low halves between pinned buffers, us: 43690 x 24 limbs 190 -> 162, 131072 x
+// 8 355 -> 232, 65536 x 4 43.8 -> 42.7; in device memory the run's index arithmetic
+// costs more than it saves, 174762 x 3 limbs 8.7 against 11.4).
+template <bool FULL, bool VEC, int MB, bool LINK = false>
 __global__ void __launch_bounds__(32, MB)
     k_mul_flex(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b, uint32_t* __restrict__ r, uint32_t n,
                uint32_t n32, FlexShape S) {
@@ -52,7 +56,13 @@ __global__ void __launch_bounds__(32, MB)
     const uint64_t off = valid ? inst * n32 : 0;
     pdl_wait();  // launched with launch_pdl
     pdl_trigger();
-    if (!L.idle) flex::stage<VEC, 2>({gA4, gB4}, {a + off, b + off}, n32, valid, S, L.t);
+    if constexpr (LINK) {
+        const uint64_t first = uint64_t(blockIdx.x) * S.groups;  // below n: the grid has no more blocks
+        flex::stage_run<VEC, 2>(smem, {a + first * n32, b + first * n32}, n32,
+                                uint32_t(min(uint64_t(S.groups), n - first)), S);
+    } else if (!L.idle) {
+        flex::stage<VEC, 2>({gA4, gB4}, {a + off, b + off}, n32, valid, S, L.t);
+    }
     __syncwarp();
     flex::rounds<FULL>(gA4, gB4, slots + threadIdx.x, S, L.t);
     __syncwarp();
@@ -111,7 +121,7 @@ uint32_t flex_rounds(uint32_t n, uint32_t n32, bool full, double* us) {
 }
 
 mi_status launch_mul_flex(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32, bool full,
-                          uint32_t rounds, cudaStream_t st) {
+                          uint32_t rounds, cudaStream_t st, bool link, uint32_t max_per_sm) {
     const bool vec = aligned16(a) && aligned16(b) && aligned16(r) && (n32 % 4 == 0);
     const FlexShape S = flex_shape(n32, full, rounds, 2);
     const uint64_t blocks = (uint64_t(n) + S.groups - 1) / S.groups;
@@ -121,9 +131,17 @@ mi_status launch_mul_flex(const uint32_t* a, const uint32_t* b, uint32_t* r, uin
          {k_mul_flex<true, false, 16>, k_mul_flex<true, true, 16>}},
         {{k_mul_flex<false, false, 18>, k_mul_flex<false, true, 18>},
          {k_mul_flex<true, false, 18>, k_mul_flex<true, true, 18>}}};
-    const Kernel kern = kernels[blocks <= 16u * uint64_t(sm_count())][full][vec];
+    static constexpr Kernel link_kernels[2] = {k_mul_flex<false, false, 16, true>, k_mul_flex<false, true, 16, true>};
+    const Kernel kern = link && !full ? link_kernels[vec] : kernels[blocks <= 16u * uint64_t(sm_count())][full][vec];
     size_t smem = S.smem();
-    MI_TRY(balanced_smem(blocks, flex_resident(S), &smem));
+    // Over the link few resident blocks, as in mul.cu, for their results to leave
+    // while the others' operands arrive: four warps for each of its blocks of
+    // eight (with 4, 8, 12, 16 and 21 per SM, us: 43690 x 24 limbs 110, 127, 145, 161, 162; 262144
+    // x 1 50.0, 38.8, 38.3, 38.3, 38.4).
+    if (link)
+        MI_TRY(capped_smem(smem, 4 * max_per_sm, &smem));
+    else
+        MI_TRY(balanced_smem(blocks, flex_resident(S), &smem));
     MI_TRY(ensure_dyn_smem(kern, smem));
     MI_CUDA_TRY(launch_pdl(kern, dim3(uint32_t(blocks)), dim3(32), smem, st, a, b, r, n, n32, S));
     return MI_OK;

@@ -4,6 +4,8 @@
 // the shapes mean and why is told in mul_flex.cu.
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "mul_core.cuh"
 
@@ -70,6 +72,45 @@ __device__ __forceinline__ void stage(uint4* const (&g4)[N], const uint32_t* con
             if (v < nv) {
 #pragma unroll
                 for (int k = 0; k < N; ++k) g4[k][(v & 1) * (S.nb + 1) + (v >> 1)] = q[k][i];
+            }
+        }
+    }
+}
+
+// The same for all instances of a warp, `count` of them from the rows on, which
+// are consecutive in memory: the warp reads them as one run.  (stage() reads
+// each row by its own lanes, a part of a 32-byte sector at a time; where the caches
+// do not hold the sector until the next part is read, as over the host link, it
+// is fetched again.)  By all lanes of the warp.
+template <bool VEC, int N>
+__device__ __forceinline__ void stage_run(uint32_t* smem, const uint32_t* const (&row)[N], uint32_t n32, uint32_t count,
+                                          const FlexShape& S) {
+    using E = std::conditional_t<VEC, uint4, uint32_t>;
+    constexpr uint32_t PER = VEC ? 1 : 4;  // elements of a 16-byte half
+    const uint32_t len = VEC ? n32 / 4 : n32, total = count * len, lane = threadIdx.x;
+    const uint32_t inv = ((1u << 22) + len - 1) / len;  // u / len = u inv >> 22: u < 1536, len < 800
+#pragma unroll 1
+    for (uint32_t base = 0; base < total; base += 4 * 32) {
+        E q[N][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+                q[k][i] = __ldcs(reinterpret_cast<const E*>(row[k]) + min(base + lane + i * 32, total - 1));
+        if (base == 0) {  // zeros past the rows, while the first loads are under way
+            for (uint32_t v = lane; v < S.groups * S.stride / 4; v += 32)
+                reinterpret_cast<uint4*>(smem)[v] = make_uint4(0, 0, 0, 0);
+            __syncwarp();
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t u = base + lane + i * 32;
+            if (u < total) {
+                const uint32_t g = (u * inv) >> 22, e = u - g * len, h = e / PER;
+#pragma unroll
+                for (int k = 0; k < N; ++k)
+                    reinterpret_cast<E*>(smem + g * S.stride + 8 * k * (S.nb + 1))
+                        [((h & 1) * (S.nb + 1) + (h >> 1)) * PER + e % PER] = q[k][i];
             }
         }
     }

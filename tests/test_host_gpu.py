@@ -319,3 +319,19 @@ def test_gpuAdd_u32_on_odd_lengths(hctx, pinned, n, m):
     a2, b2, r = [k.numpy().view(np.uint32) if pinned else k for k in keep]
     midint.gpuAdd(midint.U32bits, m, n, a2, b2, r)
     assert np.array_equal(r, O.add(a, b, m)[0])
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 1000])
+@pytest.mark.parametrize("m", [1, 2, 3, 7, 8, 9, 11, 16, 17, 23, 24, 31, 32, 33, 40, 95, 96, 120, 129, 255, 256, 301, 600])
+def test_gpuMultiply_runs_of_rows(m, n):
+    """Low halves of u32 limbs on pinned buffers: one to 32 products per warp, the
+    last warp's partly empty, whole 16-byte words or not, from words past the last
+    row that must not be read into a product."""
+    n = n if m < 256 else min(n, 100)
+    a, b = carry_stress(n, m, seed=n + m, dtype=np.uint32)
+    pad = np.full(64, 0xFFFFFFFF, np.uint32)
+    keep = [_pinned(np.concatenate([x, pad]).view(np.int32)) for x in (a, b, np.zeros(n * m, np.uint32))]
+    a2, b2, r = [k.numpy().view(np.uint32)[:n * m] for k in keep]
+    midint.gpuMultiply(midint.U32bits, m, n, a2, b2, r)
+    assert np.array_equal(r, O.mul(a, b, m, False))
+    assert (keep[2].numpy()[n * m:] == -1).all()

@@ -84,7 +84,11 @@ mi_stream mi_ctx_stream(mi_ctx ctx);
  * ragged_ntt_min limbs (1..257; classical groups hold at most 256), and
  * mi_mul_u64 does so when its operands have at least plain_ntt_min limbs
  * (1..2049; 2049 = never).  Defaults come from the committed tuning table.
- * (mi_mul_lo_u64 has its own crossover, MI_TUNE_LO_NTT_MIN.) */
+ * (mi_mul_lo_u64 has its own crossover, MI_TUNE_LO_NTT_MIN.)
+ * The table's values of plain_ntt_min, MI_TUNE_LO_NTT_MIN and
+ * MI_TUNE_POLY_NTT_MIN are measured on batches that fill the GPU; while a
+ * crossover has the table's value, small batches take the NTT from shorter
+ * operands on.  Any other value is obeyed exactly, whatever the batch. */
 mi_status mi_ctx_set_crossover(mi_ctx ctx, uint32_t ragged_ntt_min, uint32_t plain_ntt_min);
 
 /* Tunable launch choices of a context.  A new context starts from the table
@@ -104,7 +108,9 @@ mi_status mi_ctx_set_crossover(mi_ctx ctx, uint32_t ragged_ntt_min, uint32_t pla
  *                            on (2049 = never)
  *   MI_TUNE_ADD_THREAD_BYTES cls = ceil(log2(u64 limbs)) 0..12 of the
  *                            operands; value = bytes of each operand one
- *                            thread owns: 16, 32 or 64
+ *                            thread owns: 16, 32 or 64 (rows that allow
+ *                            16-byte access; other rows have their own
+ *                            choice by length)
  *   MI_TUNE_HOST_CHUNKS      cls = 0 additions, 1 multiplications; value
  *                            1..64: chunks a host-buffer batch is cut into
  *                            for copy/compute overlap
@@ -195,8 +201,9 @@ mi_status mi_add6_u64(mi_ctx ctx, const uint64_t* a, const uint64_t* b, uint64_t
  *                8-byte aligned rows.
  * mi_mul_full_*: r = a*b                      (n*2*limbs limbs).  From 129
  *                u64 limbs on (even numbers of u32 limbs, 8-byte aligned
- *                rows, and MI_TUNE_PLAIN_NTT_MIN permitting) the exact NTT
- *                kernel, with the same result.
+ *                rows, and MI_TUNE_PLAIN_NTT_MIN permitting), and in small
+ *                batches from fewer while that crossover has the table's
+ *                value, the exact NTT kernel, with the same result.
  * r must not overlap a or b.
  * ------------------------------------------------------------------------- */
 mi_status mi_mul_lo_u64(mi_ctx ctx, const uint64_t* a, const uint64_t* b, uint64_t* r,

@@ -144,17 +144,20 @@ mi_status add_any(mi_ctx ctx, const void* a, const void* b, void* r, uint8_t* ca
 // 212 us against 146, 400 of 380 limbs 61 against 18).
 constexpr uint32_t kFullNttMin = 129;
 
-// The crossover for a batch of n products of m limbs where the context's is
-// ntt_min (which is measured on batches that fill the GPU): a batch small enough for a
-// cluster per product takes the NTT from a third of it on (full products; a
+// Whether n products of m limbs go to the NTT kernels, with the context's
+// crossover `knob` (`table`: the tuning table's) and the length that batches of
+// any size take them from.  The table's crossovers are measured on batches that
+// fill the GPU: a batch small enough for a cluster per product takes the NTT
+// from a third of it on (part = 3, full products; a
 // sixth for low halves, half the classical work), since its time is the
 // latency of one product -- 4.1 to 4.3 us for up to 300 products of up to 128
 // limbs, which the classical groups' own chain of steps passes at some 40
 // limbs (20 products of 24 limbs 4.1 us classical, of 40 5.0, of 64 6.8, of 96
-// 9.1).  A crossover above every size (2049) stays one.
-uint32_t batch_ntt_min(uint32_t n, uint32_t m, uint32_t ntt_min, bool full) {
-    if (ntt_min > kNttMaxLimbs || m > kNttMaxLimbs || !ntt_small_batch(n, m)) return ntt_min;
-    return ntt_min / (full ? 3 : 6);
+// 9.1).  A crossover that the caller set to another value is taken as it is.
+bool takes_ntt(uint32_t n, uint32_t m, uint32_t knob, uint32_t table, uint32_t any_batch, uint32_t part) {
+    if (m > kNttMaxLimbs) return false;
+    if (m >= any_batch) return true;
+    return knob == table && knob <= kNttMaxLimbs && m >= knob / part && ntt_small_batch(n, m);
 }
 
 // Low halves of at least ctx->lo_ntt_min u64 limbs, and full products as
@@ -173,11 +176,12 @@ mi_status mul_any(mi_ctx ctx, const void* a, const void* b, void* r, uint32_t n,
     if (n == 0) return MI_OK;
     MI_TRY(check_ctx(ctx));
     const uint32_t n32 = limbs * uint32_t(limb_bytes / 4);
-    uint32_t ntt_min = batch_ntt_min(n, n32 / 2, full ? ctx->plain_ntt_min : ctx->lo_ntt_min, full);
-    if (full && ntt_min == ctx->plain_ntt_min) ntt_min = std::max(ntt_min, kFullNttMin);
-    if (n32 % 2 == 0 && n32 / 2 >= ntt_min && n32 / 2 <= kNttMaxLimbs && aligned8(a) && aligned8(b) && aligned8(r))
+    const uint32_t m = n32 / 2;
+    if (n32 % 2 == 0 && aligned8(a) && aligned8(b) && aligned8(r) &&
+        (full ? takes_ntt(n, m, ctx->plain_ntt_min, tuned::kPlainNttMin, std::max(ctx->plain_ntt_min, kFullNttMin), 3)
+              : takes_ntt(n, m, ctx->lo_ntt_min, tuned::kLoNttMin, ctx->lo_ntt_min, 6)))
         return launch_mul_ntt(static_cast<const uint64_t*>(a), static_cast<const uint64_t*>(b),
-                              static_cast<uint64_t*>(r), n, n32 / 2, ctx->ntt.params, pick_stream(ctx, stream), !full);
+                              static_cast<uint64_t*>(r), n, m, ctx->ntt.params, pick_stream(ctx, stream), !full);
     return launch_mul_classic(static_cast<const uint32_t*>(a), static_cast<const uint32_t*>(b),
                               static_cast<uint32_t*>(r), n, n32, full, pick_stream(ctx, stream));
 }
@@ -672,9 +676,10 @@ mi_status mi_poly_u64(mi_ctx ctx, const uint64_t* a, const uint64_t* b, uint64_t
     // crossover is measured on batches that fill the GPU: up to eight instances
     // per SM, whose time is the latency of one, the transforms are faster from a
     // quarter of it on (100 x 80 limbs 28.3 us classical against 22.5, 300 x 128
-    // 40.9 against 26.7, 1000 x 80 28.5 against 26.7, 1000 x 64 24.0 against 26.7)
+    // 40.9 against 26.7, 1000 x 80 28.5 against 26.7, 1000 x 64 24.0 against 26.7),
+    // unless the caller set it
     uint32_t ntt_min = ctx->poly_ntt_min;
-    if (ntt_min <= kNttMaxLimbs && n <= 8 * uint32_t(sm_count())) ntt_min /= 4;
+    if (ntt_min == tuned::kPolyNttMin && ntt_min <= kNttMaxLimbs && n <= 8 * uint32_t(sm_count())) ntt_min /= 4;
     if (limbs >= ntt_min && aligned8(a) && aligned8(b) && aligned8(r))
         return launch_poly_ntt(a, b, r, n, limbs, ctx->ntt.params, pick_stream(ctx, stream));
     return launch_poly(reinterpret_cast<const uint32_t*>(a), reinterpret_cast<const uint32_t*>(b),
@@ -727,8 +732,8 @@ mi_status mi_mul_ntt_u64(mi_ctx ctx, const uint64_t* a, const uint64_t* b, uint6
 mi_status mi_mul_u64(mi_ctx ctx, const uint64_t* a, const uint64_t* b, uint64_t* r, uint32_t n, uint32_t limbs,
                      mi_stream stream) {
     if (ctx == nullptr) return set_error(MI_EINVAL, "null context");
-    if (limbs <= kNttMaxLimbs && aligned8(a) && aligned8(b) && aligned8(r) &&
-        limbs >= batch_ntt_min(n, limbs, ctx->plain_ntt_min, true))
+    if (aligned8(a) && aligned8(b) && aligned8(r) &&
+        takes_ntt(n, limbs, ctx->plain_ntt_min, tuned::kPlainNttMin, ctx->plain_ntt_min, 3))
         return mul_ntt(ctx, a, b, r, n, limbs, stream);
     return mul_any(ctx, a, b, r, n, limbs, stream, 8, true);
 }

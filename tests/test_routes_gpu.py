@@ -9,6 +9,8 @@ import re
 import pytest
 import torch
 
+import midint
+
 pytestmark = pytest.mark.gpu
 
 
@@ -31,8 +33,8 @@ def route(ctx, tmp_path):
             check(cudart.cudaStreamEndCapture(s, ctypes.byref(graph)))
         check(cudart.cudaGraphDebugDotPrint(graph, str(path).encode(), 1))  # verbose
         check(cudart.cudaGraphDestroy(graph))
-        # mangled: a name is preceded by its length
-        return {name[:int(n)] for n, name in re.findall(r"(\d+)(k_[A-Za-z0-9_]+)", path.read_text())}
+        # mangled: a (lower-case) name stands between its length and a capital
+        return set(re.findall(r"\d(k_[a-z0-9_]+)(?=[A-Z])", path.read_text()))
 
     return run
 
@@ -50,4 +52,36 @@ def test_add6_on_unaligned_rows(ctx, route, m, kernel):
     # lengths that fill their group take consecutive limbs per thread
     keep, (a, b, r) = buffers(2 * m * 100, offset=2)
     assert route(lambda s: ctx.add6(a, b, r, 100, m, stream=s)) == {kernel}
+    del keep
+
+
+@pytest.fixture
+def own(lib):
+    c = midint.Context(0)
+    yield c
+    c.close()
+
+
+NTT = {"k_ntt_mul", "k_ntt_mul_cluster", "k_poly_ntt"}
+
+
+@pytest.mark.parametrize("knob,call,words,m,n", [
+    (midint.TUNE_PLAIN_NTT_MIN, "mul", 4, 400, 20), (midint.TUNE_PLAIN_NTT_MIN, "mul_full", 4, 400, 20),
+    (midint.TUNE_LO_NTT_MIN, "mul_lo", 2, 200, 20), (midint.TUNE_POLY_NTT_MIN, "poly", 2, 200, 20)])
+def test_crossovers_set_by_the_caller_are_exact(own, route, knob, call, words, m, n):
+    # small batches, which take the transforms at these lengths by themselves
+    keep, (a, b, r) = buffers(words * m * n)
+
+    def names():
+        return route(lambda s: getattr(own, call)(a, b, r, n, m, stream=s))
+
+    table = own.get_tuning(knob)
+    assert names() <= NTT
+    for value in (1025, m + 1):
+        own.set_tuning(knob, 0, value)
+        assert not names() & NTT, value
+    own.set_tuning(knob, 0, m)
+    assert names() <= NTT
+    own.set_tuning(knob, 0, table)
+    assert names() <= NTT
     del keep

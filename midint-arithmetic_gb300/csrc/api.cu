@@ -144,25 +144,36 @@ mi_status add_any(mi_ctx ctx, const void* a, const void* b, void* r, uint8_t* ca
 // 212 us against 146, 400 of 380 limbs 61 against 18).
 constexpr uint32_t kFullNttMin = 129;
 
-// Whether n products of m limbs go to the NTT kernels, with the context's
-// crossover `knob` (`table`: the tuning table's) and the length that batches of
-// any size take them from.  The table's crossovers are measured on batches that
-// fill the GPU: a batch small enough for a cluster per product takes the NTT
-// from a third of it on (part = 3, full products; a
-// sixth for low halves, half the classical work), since its time is the
-// latency of one product -- 4.1 to 4.3 us for up to 300 products of up to 128
-// limbs, which the classical groups' own chain of steps passes at some 40
-// limbs (20 products of 24 limbs 4.1 us classical, of 40 5.0, of 64 6.8, of 96
-// 9.1).  A crossover that the caller set to another value is taken as it is.
-bool takes_ntt(uint32_t n, uint32_t m, uint32_t knob, uint32_t table, uint32_t any_batch, uint32_t part) {
-    if (m > kNttMaxLimbs) return false;
-    if (m >= any_batch) return true;
-    return knob == table && knob <= kNttMaxLimbs && m >= knob / part && ntt_small_batch(n, m);
+// Shorter products that small batches take the NTT for: 4.1 us for up to 300
+// products of up to 128 limbs, against 4.1 us classical for 20 products of 24 limbs,
+// 5.0 of 40, 6.8 of 64, 9.1 of 96; low halves of 48 limbs 6.4.
+constexpr uint32_t kShortNttMin = 42, kShortLoNttMin = 48;
+
+// What the classical launch of a full product takes beside its modelled time (us).
+constexpr double kClassicLaunchUs = 1.8;
+
+// Whether n products of m limbs go to the NTT kernels: by the context's
+// crossover where the caller set it.  While it has the tuning table's value,
+// which is measured on batches that fill the GPU, low halves follow it and
+// small batches take the NTT from fewer limbs on; full products of up to 128
+// limbs take what the two models say is faster (us, classical against NTT: 800 x 42
+// limbs 5.8 against 9.0, 300 x 42 5.7 against 4.2, 1000 x 80 9.9 against 8.3, 1216 x 124
+// 15.0 against 12.4, 3000 x 112 31.7 against 26.6, 10000 x 112 75 against 82, 65536 x
+// 128 455 against 518).
+bool takes_ntt(uint32_t n, uint32_t m, uint32_t knob, bool full, bool vec) {
+    if (m > kNttMaxLimbs || m == 0) return false;
+    if (knob != (full ? tuned::kPlainNttMin : tuned::kLoNttMin)) return m >= knob;
+    if (!full) return m >= knob || (m >= kShortLoNttMin && ntt_small_batch(n, m));
+    if (m >= kFullNttMin) return true;
+    if (m < kShortNttMin) return false;
+    // (the models cost the host 0.2 us, which the smallest batches would show)
+    if (n <= 2 * uint32_t(sm_count())) return true;
+    double classic = 0;
+    kara_pays(n, 2 * m, vec, &classic);
+    return ntt_short_us(n, m) < classic + kClassicLaunchUs;
 }
 
-// Low halves of at least ctx->lo_ntt_min u64 limbs, and full products as
-// above, come from the NTT kernel (same result; its cost grows as L lg L, the
-// classical one's as limbs^2).  An even number of u32 limbs is half as many
+// An even number of u32 limbs is half as many
 // u64 limbs; the NTT kernels read 8-byte words, so rows that are only 4-byte
 // aligned take the classical kernels, which read 32-bit words.
 mi_status mul_any(mi_ctx ctx, const void* a, const void* b, void* r, uint32_t n, uint32_t limbs, mi_stream stream,
@@ -177,9 +188,10 @@ mi_status mul_any(mi_ctx ctx, const void* a, const void* b, void* r, uint32_t n,
     MI_TRY(check_ctx(ctx));
     const uint32_t n32 = limbs * uint32_t(limb_bytes / 4);
     const uint32_t m = n32 / 2;
-    if (n32 % 2 == 0 && aligned8(a) && aligned8(b) && aligned8(r) &&
-        (full ? takes_ntt(n, m, ctx->plain_ntt_min, tuned::kPlainNttMin, std::max(ctx->plain_ntt_min, kFullNttMin), 3)
-              : takes_ntt(n, m, ctx->lo_ntt_min, tuned::kLoNttMin, ctx->lo_ntt_min, 6)))
+    const bool vec = aligned16(a) && aligned16(b) && aligned16(r) && n32 % 4 == 0;
+    uint32_t knob = full ? ctx->plain_ntt_min : ctx->lo_ntt_min;
+    if (full && knob != tuned::kPlainNttMin) knob = std::max(knob, kFullNttMin);
+    if (n32 % 2 == 0 && aligned8(a) && aligned8(b) && aligned8(r) && takes_ntt(n, m, knob, full, vec))
         return launch_mul_ntt(static_cast<const uint64_t*>(a), static_cast<const uint64_t*>(b),
                               static_cast<uint64_t*>(r), n, m, ctx->ntt.params, pick_stream(ctx, stream), !full);
     return launch_mul_classic(static_cast<const uint32_t*>(a), static_cast<const uint32_t*>(b),
@@ -732,8 +744,8 @@ mi_status mi_mul_ntt_u64(mi_ctx ctx, const uint64_t* a, const uint64_t* b, uint6
 mi_status mi_mul_u64(mi_ctx ctx, const uint64_t* a, const uint64_t* b, uint64_t* r, uint32_t n, uint32_t limbs,
                      mi_stream stream) {
     if (ctx == nullptr) return set_error(MI_EINVAL, "null context");
-    if (aligned8(a) && aligned8(b) && aligned8(r) &&
-        takes_ntt(n, limbs, ctx->plain_ntt_min, tuned::kPlainNttMin, ctx->plain_ntt_min, 3))
+    const bool vec = aligned16(a) && aligned16(b) && aligned16(r) && limbs % 2 == 0;
+    if (aligned8(a) && aligned8(b) && aligned8(r) && takes_ntt(n, limbs, ctx->plain_ntt_min, true, vec))
         return mul_ntt(ctx, a, b, r, n, limbs, stream);
     return mul_any(ctx, a, b, r, n, limbs, stream, 8, true);
 }

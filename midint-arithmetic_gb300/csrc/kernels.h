@@ -70,8 +70,9 @@ mi_status launch_mul_flex(const uint32_t* a, const uint32_t* b, uint32_t* r, uin
                           uint32_t rounds, cudaStream_t st, bool link = false, uint32_t max_per_sm = 0);
 
 // Full products of 25..32 blocks of 8 u32 limbs with one Karatsuba level
-// (mul_kara.cu), and the batches for which that is the fastest form.
-bool kara_pays(uint32_t n, uint32_t n32, bool vec);
+// (mul_kara.cu), and the batches for which that is the fastest form; us, where
+// given, is the modelled time of the fastest form.
+bool kara_pays(uint32_t n, uint32_t n32, bool vec, double* us = nullptr);
 mi_status launch_mul_kara(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32,
                           cudaStream_t st);
 

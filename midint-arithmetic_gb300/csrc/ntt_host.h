@@ -51,9 +51,12 @@ mi_status launch_mul_ntt(const uint64_t* a, const uint64_t* b, uint64_t* r, uint
 // programmatic dependent launch.
 bool ntt_dependent(uint32_t n, int per_sm);
 
-// Whether launch_mul_ntt runs n products of m limbs on clusters (a block per
-// prime), where a call takes little more than the latency of one prime.
+// Whether launch_mul_ntt runs n low halves of m limbs on clusters (a block per
+// prime), in less than the latency of the classical groups.
 bool ntt_small_batch(uint32_t n, uint32_t m);
+
+// The modelled time (us) of n full products of at most 128 limbs.
+double ntt_short_us(uint32_t n, uint32_t m);
 
 // One transform or one cyclic convolution on a single prime (device buffers).
 struct NttRawArgs {

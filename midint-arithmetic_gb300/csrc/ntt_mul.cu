@@ -21,6 +21,8 @@
 // carry that the reference does with splitFftReg + baddRegMul2Fft.
 // (ntt_raw below keeps the 64-bit fields of ntt.cuh, so it can run the
 // reference's own primes on its known answers.)
+#include <algorithm>
+#include <cmath>
 #include <cstdio>
 
 #include "common.cuh"
@@ -97,11 +99,16 @@ __global__ void __launch_bounds__((1 << LG) / 8)
 // it the blocks of a cluster wait for one another and for a place (m = 1024,
 // n = 152 22.8 us against 16.5; n = 1024 140 against 89; m = 400, n = 152
 // 13.2 against 11.2; m = 256, n = 300 11.4 against 10.4).
-constexpr uint32_t cluster_blocks_per_sm(int lg) { return lg == 8 ? 16 : lg == 9 ? 7 : lg <= 11 ? 3 : 2; }
-
-bool cluster_fits(uint32_t n, int np, int lg) {
-    return uint64_t(n) * uint32_t(np) < uint64_t(sm_count()) * cluster_blocks_per_sm(lg);
+// 256-point blocks are one warp: m = 96, n = 480 8.1 us against 8.3, n = 600 9.7
+// against 8.3; m = 128, n = 400 8.4 against 10.3, n = 500 10.1 against 10.3; m = 48, n =
+// 600 7.0 against 8.2 (alone 19.0 against 18.1), n = 800 9.0 against 8.3.
+// (Low halves to 16: the caller then prefers the classical form to a block each.)
+constexpr double cluster_blocks_per_sm(int lg, bool low) {
+    return lg == 8 ? (low ? 16 : 13.5) : lg == 9 ? 7 : lg <= 11 ? 3 : 2;
 }
+
+// (blocks: per SM)
+bool cluster_fits(double blocks, int lg, bool low) { return blocks < cluster_blocks_per_sm(lg, low); }
 
 }  // namespace
 
@@ -125,7 +132,7 @@ mi_status launch_lg(const uint64_t* a, const uint64_t* b, uint64_t* r, uint32_t 
                     const NttMulParams& P, cudaStream_t st) {
     using S = NttShape<LG>;
     const bool low = rlen <= m;  // the low half alone
-    if (cluster_fits(n, NP, LG)) {
+    if (cluster_fits(double(n) * NP / sm_count(), LG, low)) {
         auto kern = low ? k_ntt_mul_cluster<LG, NP, true> : k_ntt_mul_cluster<LG, NP, false>;
         static ResidentBlocks site[2];
         int per_sm = 0;
@@ -226,10 +233,27 @@ __global__ void __launch_bounds__((1 << LG) / 8)
 
 }  // namespace
 
+// 256-point transforms: up to the number of blocks per SM whose time reaches the
+// latency of the classical low half, which grows with the limbs (n = 400 of m = 48 5.7
+// us against 6.3, n = 500 6.5 against 6.4; m = 64, n = 600 7.0 against 7.4, n = 800 8.9
+// against 7.5; m = 80, n = 700 7.8 against 8.7; m = 128, n = 450 9.4 against 12.0).  Longer
+// ones: classical 14 us and more, clusters at most 13.
 bool ntt_small_batch(uint32_t n, uint32_t m) {
     int lg = ntt32::kLgMin;
     while ((1u << lg) < 2 * m) ++lg;
-    return lg <= ntt32::kLgMax && cluster_fits(n, 5 - ntt32::ntt_mode(m, m, 1u << lg), lg);
+    const double blocks = double(n) * (5 - ntt32::ntt_mode(m, m, 1u << lg)) / sm_count();
+    return lg <= ntt32::kLgMax && cluster_fits(blocks, lg, true) && (lg > ntt32::kLgMin || blocks < 0.19 * m);
+}
+
+// Clusters: 4.1 us, and from five blocks per SM on 0.45 us for each.  A block
+// per product: by the warps of the busiest scheduler, six at most at a time.
+// Within 10 % of what 13 lengths of 80 to 128 limbs measured in batches of 320 to
+// 10000, 3 % in the middle.
+double ntt_short_us(uint32_t n, uint32_t m) {
+    const int np = 5 - ntt32::ntt_mode(m, m, 256);
+    const double blocks = double(n) * np / sm_count(), k = blocks / (4 * np);  // k: warps per scheduler
+    if (cluster_fits(blocks, 8, false)) return 4.1 + 0.45 * std::max(0.0, blocks - 5) + 0.6 * (np - 3);
+    return np * (k <= 6 ? 1.24 + 0.816 * std::ceil(k) : 1.023 * k);
 }
 
 mi_status launch_mul_ntt(const uint64_t* a, const uint64_t* b, uint64_t* r, uint32_t n, uint32_t m,

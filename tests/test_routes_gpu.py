@@ -85,3 +85,22 @@ def test_crossovers_set_by_the_caller_are_exact(own, route, knob, call, words, m
     own.set_tuning(knob, 0, table)
     assert names() <= NTT
     del keep
+
+
+CLASSIC = {"k_mul", "k_mul_flex", "k_mul_kara", "k_mul_lo"}
+CLUSTER, BLOCKS = {"k_ntt_mul_cluster"}, {"k_ntt_mul"}
+
+
+@pytest.mark.parametrize("call,m,n,kernels", [
+    ("mul", 41, 20, CLASSIC), ("mul", 42, 300, CLUSTER), ("mul", 42, 800, CLASSIC), ("mul", 64, 300, CLUSTER),
+    ("mul", 64, 800, CLASSIC), ("mul", 80, 1000, BLOCKS), ("mul", 112, 3000, BLOCKS), ("mul", 124, 1216, BLOCKS),
+    ("mul", 128, 60000, CLASSIC), ("mul_full", 42, 800, CLASSIC), ("mul_full", 128, 16384, CLASSIC),
+    ("mul_full", 129, 16384, BLOCKS), ("mul_lo", 48, 300, CLUSTER), ("mul_lo", 48, 700, CLASSIC),
+    ("mul_lo", 80, 700, CLUSTER), ("mul_lo", 80, 800, CLASSIC), ("mul_lo", 287, 3000, CLASSIC),
+    ("mul_lo", 288, 3000, BLOCKS)])
+def test_products_by_length_and_batch(own, route, call, m, n, kernels):
+    # short products take the transforms only in batches that are faster there
+    keep, (a, b, r) = buffers((2 if call == "mul_lo" else 4) * m * n)
+    names = route(lambda s: getattr(own, call)(a, b, r, n, m, stream=s))
+    assert names and names <= kernels
+    del keep

@@ -105,7 +105,9 @@ mi_status mi_ctx_set_crossover(mi_ctx ctx, uint32_t ragged_ntt_min, uint32_t pla
  *   MI_TUNE_LO_NTT_MIN       cls ignored; value 1..2049: mi_mul_lo_u64 and
  *                            the u64 gpuMultiply wrapper compute the low
  *                            half with the NTT kernel from this many limbs
- *                            on (2049 = never)
+ *                            on (2049 = never; the wrapper, while this has
+ *                            the table's value, not in large batches that
+ *                            it reads over the host link)
  *   MI_TUNE_ADD_THREAD_BYTES cls = ceil(log2(u64 limbs)) 0..12 of the
  *                            operands; value = bytes of each operand one
  *                            thread owns: 16, 32 or 64 (rows that allow

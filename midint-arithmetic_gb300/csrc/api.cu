@@ -321,6 +321,20 @@ struct HostLaunch {
     bool in, out;  // the operands, the results are host memory
 };
 
+// Whether cnt low halves of m limbs go to the NTT kernel: from the crossover on,
+// but while that has the table's value, which is measured in device memory, not
+// over the host link in batches of more than six per SM: the transforms read
+// their operands once per prime (us between pinned buffers, classical against
+// NTT: 3000 x 300 limbs 185 and 259, 1000 x 400 123 and 180, 3000 x 512 292 and 659;
+// 800 x 300 88 and 84, 256 x 300 55 and 34).  Rows of odd length read classically lose more than
+// that (1000 x 319 154 and 107), and so do the larger groups from 513 limbs on (1000 x
+// 600 233 and 198).
+bool host_takes_ntt(mi_ctx ctx, uint32_t cnt, uint32_t m, HostLaunch how, bool vec) {
+    if (m < ctx->lo_ntt_min || m > kNttMaxLimbs) return false;
+    const bool link = how.in && ctx->lo_ntt_min == tuned::kLoNttMin;
+    return !(link && vec && m % 2 == 0 && m <= 512 && cnt > 6 * uint32_t(sm_count()));
+}
+
 template <typename F>
 mi_status host_pipeline(mi_ctx ctx, int cls, const void* h_a, const void* h_b, void* h_r, uint8_t* h_carry,
                         uint32_t n, size_t in_row, size_t out_row, F launch, bool one_compute_stream = false) {
@@ -786,17 +800,16 @@ mi_status mi_compat_gpuMultiply_u64(int num_instances, uint32_t m, const uint64_
     mi_ctx ctx;
     MI_TRY(default_ctx(&ctx));
     const size_t row = size_t(m) * 8;
-    const bool ntt = m >= ctx->lo_ntt_min && m <= kNttMaxLimbs;  // as mi_mul_lo_u64 picks (the buffers the
-                                                                  // kernels see are 8-byte aligned)
     return host_pipeline(ctx, HOST_MUL, h_as, h_bs, h_rs, nullptr, uint32_t(num_instances), row, row,
-                         [ctx, m, ntt](void* da, void* db, void* dr, uint8_t*, uint32_t cnt, cudaStream_t st,
-                                       HostLaunch how) {
-                             if (ntt)
+                         [ctx, m](void* da, void* db, void* dr, uint8_t*, uint32_t cnt, cudaStream_t st,
+                                  HostLaunch how) {
+                             // (the buffers the kernels see are 8-byte aligned)
+                             if (host_takes_ntt(ctx, cnt, m, how, aligned16(da) && aligned16(db) && aligned16(dr)))
                                  return launch_mul_ntt(static_cast<uint64_t*>(da), static_cast<uint64_t*>(db),
                                                        static_cast<uint64_t*>(dr), cnt, m, ctx->ntt.params, st, true);
                              return launch_mul_classic(static_cast<uint32_t*>(da), static_cast<uint32_t*>(db),
-                                                       static_cast<uint32_t*>(dr), cnt, 2 * m, false, st, how.max_per_sm,
-                                                       how.in);
+                                                       static_cast<uint32_t*>(dr), cnt, 2 * m, false, st,
+                                                       how.max_per_sm, how.in);
                          });
 }
 

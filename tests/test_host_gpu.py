@@ -335,3 +335,18 @@ def test_gpuMultiply_runs_of_rows(m, n):
     midint.gpuMultiply(midint.U32bits, m, n, a2, b2, r)
     assert np.array_equal(r, O.mul(a, b, m, False))
     assert (keep[2].numpy()[n * m:] == -1).all()
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+@pytest.mark.parametrize("m", [287, 288, 301, 320, 512, 514])
+def test_gpuMultiply_either_side_of_the_link_rule(m, pinned):
+    # few products (transforms from 288 limbs on) and more than six per SM,
+    # which stay classical over the host link up to 512 limbs of even length
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    a, b = carry_stress(6 * sms + 1, m, seed=m)
+    want = O.mul(a, b, m, False)
+    for n in (3, 6 * sms, 6 * sms + 1):
+        keep = [_pinned(x) if pinned else x for x in (a[:n * m].copy(), b[:n * m].copy(), np.zeros(n * m, np.uint64))]
+        a2, b2, r = [k.numpy().view(np.uint64) if pinned else k for k in keep]
+        midint.gpuMultiply(midint.U64bits, m, n, a2, b2, r)
+        assert np.array_equal(r, want[:n * m]), n

@@ -174,8 +174,8 @@ mi_status mi_ctx_get_tuning(mi_ctx ctx, int knob, uint32_t cls, uint32_t* value)
  * r may alias a or b exactly (in-place), but must not partially overlap.
  * limbs <= 2^26 u64 limbs (2^27 u32): instances wider than 4096 u64 limbs run
  * a multi-block kernel whose tiles chain their carries by decoupled
- * look-back with bounded waits; such calls on one context must not overlap on
- * the device, and a wait that gave up is reported by mi_ctx_device_status
+ * look-back with bounded waits; such calls on one context, replays of captured
+ * ones among them, must not overlap on the device, and a wait that gave up is reported by mi_ctx_device_status
  * (and by the host-buffer calls) as MI_ETIMEOUT.
  * ------------------------------------------------------------------------- */
 mi_status mi_add_u64(mi_ctx ctx, const uint64_t* a, const uint64_t* b, uint64_t* r,

@@ -587,7 +587,9 @@ __global__ void __launch_bounds__(256, sizeof(L) == 8 ? 4 : 2)
 
 // Rounds of whole instances, at most kWideTiles tiles each; every round takes
 // the next n_tiles values of the tile counter and the other array of state
-// words, clearing the words of the round before.
+// words, clearing the words of the round before.  Under capture the graph clears
+// the captured calls' area before each round instead, so that every replay starts
+// from the same state.
 template <typename L, bool VEC, int OP>
 mi_status launch_wide(const L* a, const L* b, L* r, uint8_t* carry, uint32_t n, uint32_t m, WideState& w,
                       cudaStream_t st) {
@@ -597,23 +599,34 @@ mi_status launch_wide(const L* a, const L* b, L* r, uint8_t* carry, uint32_t n, 
     const uint32_t cap = w.round_tiles < kWideTiles ? w.round_tiles : kWideTiles;
     if (tiles_per > cap) return set_error(MI_EINVAL, "add: %u limbs exceeds the multi-block maximum", m);
     const uint32_t per_round = cap / tiles_per;
+    cudaStreamCaptureStatus capture;
+    MI_CUDA_TRY(cudaStreamIsCapturing(st, &capture));
+    const bool captured = capture != cudaStreamCaptureStatusNone;
+    uint64_t* const area = w.status + (captured ? kWideBytes / 8 : 0);
+    uint64_t* const counter = area + 2 * kWideWords;
+    uint32_t* const err = reinterpret_cast<uint32_t*>(w.status + 2 * kWideWords + 1);
     for (uint32_t i0 = 0; i0 < n; i0 += per_round) {
         const uint32_t k = (n - i0) < per_round ? (n - i0) : per_round;
         const uint32_t n_tiles = k * tiles_per;
         const uint32_t words = k * ((tiles_per + 31) / 32);  // tiles_per >= 2, so at most kWideWords
         const uint64_t o = uint64_t(i0) * m;
+        uint64_t *states = area + w.parity * kWideWords, *old = area + (w.parity ^ 1u) * kWideWords, base = w.issued;
+        uint32_t old_words = w.old_words;
+        if (captured) {  // the words right before the counter, cleared with it
+            states = counter - words, base = 0, old_words = 0;
+            MI_CUDA_TRY(cudaMemsetAsync(states, 0, (size_t(words) + 1) * 8, st));
+        }
         uint8_t* edges = nullptr;
         if (r == a || r == b) {
-            edges = reinterpret_cast<uint8_t*>(w.status + 2 * kWideWords + 2);
+            edges = reinterpret_cast<uint8_t*>(area + 2 * kWideWords + 2);
             MI_CUDA_TRY(launch_pdl(k_wide_edges<L, OP>, dim3((n_tiles + 7) / 8), dim3(256), 0, st, a + o, b + o, m,
                                    tiles_per, n_tiles, edges));
         }
         MI_CUDA_TRY(launch_pdl(k_add_wide<L, V, OP>, dim3(n_tiles), dim3(256), 0, st, a + o, b + o, r + o,
-                               carry ? carry + i0 : nullptr, m, tiles_per, n_tiles,
-                               w.status + w.parity * kWideWords, w.status + (w.parity ^ 1u) * kWideWords,
-                               w.old_words, reinterpret_cast<unsigned long long*>(w.status + 2 * kWideWords),
-                               reinterpret_cast<uint32_t*>(w.status + 2 * kWideWords + 1), w.spin_limit, w.withhold,
-                               w.issued, edges));
+                               carry ? carry + i0 : nullptr, m, tiles_per, n_tiles, states, old, old_words,
+                               reinterpret_cast<unsigned long long*>(counter), err, w.spin_limit, w.withhold, base,
+                               edges));
+        if (captured) continue;
         w.issued += n_tiles;  // every block of the launch takes one counter value
         w.old_words = words;
         w.parity ^= 1u;

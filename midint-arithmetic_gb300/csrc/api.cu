@@ -507,7 +507,7 @@ mi_status mi_ctx_create(int device, mi_ctx* out) {
         ctx->host_page_tables = access != 0 && tables != 0;
     if (st == MI_OK) st = ntt_tables_create(&ctx->ntt);
     if (st == MI_OK) {
-        const size_t wb = kWideBytes;
+        const size_t wb = 2 * kWideBytes;
         if (cudaMalloc(&ctx->wide.status, wb) != cudaSuccess || cudaMemset(ctx->wide.status, 0, wb) != cudaSuccess)
             st = set_error(MI_ENOMEM, "mi_ctx_create: multi-block addition state");
     }

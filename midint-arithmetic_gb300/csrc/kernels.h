@@ -13,15 +13,18 @@ enum AddOp : int { ADD_PLAIN = 0, ADD_SIX = 1 };
 // Device state of the additions wider than one block (decoupled look-back):
 // `status` holds two arrays of kWideWords words of tile states (32 tiles per
 // word, two bits each), then the tile counter, then the error word (set when
-// a bounded wait gave up), then one byte per tile for in-place calls.  One per context; wide additions on one context
-// must not overlap on the device.  The host side keeps which array the next
-// launch takes, how many words of the other the last one used, and the
-// counter values issued so far.
+// a bounded wait gave up), then one byte per tile for in-place calls.  One per
+// context; wide additions on one context must not overlap on the device.  The
+// host side keeps which array the next launch takes, how many words of the
+// other the last one used, and the counter values issued so far.  A call that is
+// captured into a graph takes none of these, which a replay could not follow: it
+// has a second such area, cleared by the graph itself (the error word is the
+// first area's).
 constexpr uint32_t kWideTiles = 1u << 16;  // per launch
 constexpr uint32_t kWideWords = kWideTiles / 2;  // an instance has at least two tiles and starts a word
 constexpr size_t kWideBytes = (2 * size_t(kWideWords) + 2) * 8 + kWideTiles;
 struct WideState {
-    uint64_t* status = nullptr;    // kWideBytes
+    uint64_t* status = nullptr;    // 2 kWideBytes: the area of direct calls, that of captured ones
     uint32_t parity = 0;           // array of the next launch
     uint32_t old_words = 0;        // words of the other array to clear
     uint64_t issued = 0;           // tile counter values taken by earlier launches

@@ -153,3 +153,62 @@ def test_wide_add_words_of_states_and_in_place(wctx, devmem, n, m, bits, op):
     assert wctx.device_status() == midint.MI_OK
     assert np.array_equal(devmem.get(keep_r[0], words, 0, a.dtype), want)
     assert np.array_equal(dc.cpu().numpy(), carry)
+
+
+@pytest.mark.parametrize("n,m,bits,rounds", [(3, 33 * 2048 + 5, 64, False), (5, 4099, 64, False), (3, 9001, 32, False),
+                                             (7, 3 * 2048, 64, True)])
+@pytest.mark.parametrize("op", ["add", "add_in_a", "six"])
+def test_wide_add_captured_and_replayed(wctx, devmem, n, m, bits, rounds, op):
+    # a captured call gives its result at every replay, from the operands of the
+    # moment, and leaves the direct calls before, between and after it right
+    if op == "six" and bits == 32:
+        pytest.skip("6a + 10b is defined on u64 limbs")
+    if rounds:  # two instances per launch
+        wctx.set_tuning(midint.TUNE_WIDE_ROUND_TILES, 0, 6)
+    dtype = np.uint64 if bits == 64 else np.uint32
+    a, b = carry_stress(n, m, seed=n + m, dtype=dtype)
+    words = a.view(np.uint32).size
+    ka, pa = devmem.put(a, 0)
+    kb, pb = devmem.put(b, 0)
+    kr, pr = (ka, pa) if op == "add_in_a" else devmem.empty_words(words, 0)
+    dc = torch.zeros(n, dtype=torch.uint8, device="cuda:0")
+
+    def call(s):
+        if op == "six":
+            wctx.add6(pa, pb, pr, n, m, stream=s)
+        else:
+            wctx.add(pa, pb, pr, n, m, carry=dc.data_ptr(), limb_bits=bits, stream=s)
+
+    def load(x, y):
+        for keep, v in ((ka, x), (kb, y)):
+            keep[:words] = torch.from_numpy(v.view(np.int32).copy()).to("cuda:0")
+
+    def check(x, y):
+        torch.cuda.synchronize()
+        want, carry = (O.add6(x, y, m), np.zeros(n, np.uint8)) if op == "six" else O.add(x, y, m)
+        assert wctx.device_status() == midint.MI_OK
+        assert np.array_equal(devmem.get(kr, words, 0, dtype), want)
+        assert np.array_equal(dc.cpu().numpy(), carry)
+
+    side = torch.cuda.Stream()
+    call(side.cuda_stream)
+    check(a, b)
+    load(a, b)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=side):
+        call(torch.cuda.current_stream().cuda_stream)
+    call(side.cuda_stream)                      # directly, after the capture
+    check(a, b)
+    for i in range(4):
+        x, y = carry_stress(n, m, seed=100 + i, dtype=dtype)
+        load(x, y)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            g.replay()
+        check(x, y)
+        if i % 2:
+            load(x, y)
+            torch.cuda.synchronize()
+            call(side.cuda_stream)
+            check(x, y)

@@ -2,6 +2,9 @@
 and the zero-copy path on mapped pinned buffers give the oracle's results."""
 from __future__ import annotations
 
+import ctypes
+import mmap
+
 import numpy as np
 import pytest
 import torch
@@ -350,3 +353,90 @@ def test_gpuMultiply_either_side_of_the_link_rule(m, pinned):
         a2, b2, r = [k.numpy().view(np.uint64) if pinned else k for k in keep]
         midint.gpuMultiply(midint.U64bits, m, n, a2, b2, r)
         assert np.array_equal(r, want[:n * m]), n
+
+
+def _in_place_device():
+    """Whether the GPU walks the host's page tables (device attributes 88 and 100)."""
+    cudart = ctypes.CDLL("libcudart.so.13")
+    v = ctypes.c_int()
+    for attr in (88, 100):
+        if cudart.cudaDeviceGetAttribute(ctypes.byref(v), attr, 0) != 0 or not v.value:
+            return False
+    return True
+
+
+def _mapped(x: np.ndarray, prot: int, at_end: bool):
+    """x in an anonymous mapping of its own, at its start or so that it ends
+    exactly with its last page, which an inaccessible page follows."""
+    page = mmap.PAGESIZE
+    size = -(-x.nbytes // page) * page
+    mm = mmap.mmap(-1, size + page)
+    base = ctypes.addressof(ctypes.c_char.from_buffer(mm))
+    off = size - x.nbytes if at_end else 0
+    view = np.frombuffer(mm, x.dtype, x.size, off)
+    view[:] = x
+    libc = ctypes.CDLL(None, use_errno=True)
+    libc.mprotect.argtypes = [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int]
+    assert libc.mprotect(base + size, page, 0) == 0
+    assert libc.mprotect(base, size, prot) == 0
+    return view, (mm, libc, base, size + page)
+
+
+def _release(keep):
+    mm, libc, base, size = keep
+    assert libc.mprotect(base, size, mmap.PROT_READ | mmap.PROT_WRITE) == 0
+
+
+def _free_bytes():
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+@pytest.mark.parametrize("at_end", [False, True])
+@pytest.mark.parametrize("n,m", [(1000, 64), (333, 129)])
+def test_ordinary_memory_is_used_in_place(hctx, at_end, n, m):
+    # operands that may only be read and that end at an inaccessible page, a result
+    # in fresh pages; the staging buffers of the copies are never allocated
+    for cls in (0, 1):
+        hctx.set_tuning(midint.TUNE_HOST_ZERO_COPY, cls, 1)
+    a, b = carry_stress(n, m, seed=n)
+    rw = mmap.PROT_READ | mmap.PROT_WRITE
+    (va, ka), (vb, kb) = (_mapped(x, mmap.PROT_READ, at_end) for x in (a, b))
+    vr, kr = _mapped(np.zeros(2 * n * m, np.uint64), rw, at_end)
+    before = _free_bytes()
+    hctx.host_mul_full(va, vb, vr, n, m)
+    after = _free_bytes()
+    assert np.array_equal(vr, O.mul(a, b, m, True))
+    vs, ks = _mapped(np.zeros(n * m, np.uint64), rw, at_end)
+    hctx.host_add(va, vb, vs, None, n, m)
+    assert np.array_equal(vs, O.add(a, b, m)[0])
+    if _in_place_device():
+        assert before - after < n * m * 8, "staged: the copies' buffers were allocated"
+    for k in (ka, kb, kr, ks):
+        _release(k)
+
+
+def test_operands_in_a_private_file_mapping(hctx, tmp_path):
+    # pages of a file, and a result over the 32 MiB that are used in place
+    for cls in (0, 1):
+        hctx.set_tuning(midint.TUNE_HOST_ZERO_COPY, cls, 1)
+    for n, m in ((700, 64), (20000, 64)):
+        a, b = carry_stress(n, m, seed=n)
+        path = tmp_path / f"operand{n}"
+        path.write_bytes(a.tobytes())
+        fa = np.memmap(path, np.uint64, "r")
+        r = np.zeros(2 * n * m, np.uint64)
+        hctx.host_mul_full(fa, b, r, n, m)
+        assert np.array_equal(r, O.mul(a, b, m, True))
+
+
+def test_populating_a_result_that_may_not_be_written_fails():
+    # what sends such a call back to the copies, as any buffer that cannot be used
+    # in place (the copies would then meet the same protection, as before)
+    libc = ctypes.CDLL(None, use_errno=True)
+    libc.madvise.argtypes = [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int]
+    view, keep = _mapped(np.zeros(4096, np.uint64), mmap.PROT_READ, False)
+    populate_read, populate_write = 22, 23
+    assert libc.madvise(keep[2], mmap.PAGESIZE, populate_read) == 0
+    assert libc.madvise(keep[2], mmap.PAGESIZE, populate_write) != 0
+    _release(keep)

@@ -206,3 +206,39 @@ def test_mul_lo_places(ctx, devmem, m):
         want = O.mul(a, b, m, False)
         for _ in range(2):
             assert np.array_equal(gpu_mul(ctx, devmem, a, b, m, False, limb_bits=32), want), n
+
+
+@pytest.fixture
+def classical(ctx):
+    """Full products on the classical kernels at every length and batch."""
+    old = ctx.get_tuning(midint.TUNE_PLAIN_NTT_MIN)
+    ctx.set_tuning(midint.TUNE_PLAIN_NTT_MIN, 0, 2049)
+    yield ctx
+    ctx.set_tuning(midint.TUNE_PLAIN_NTT_MIN, 0, old)
+
+
+@pytest.mark.parametrize("m", [42, 64, 96, 100, 128, 129, 130, 160, 192, 200, 255, 256, 257, 258, 384, 500, 512, 513,
+                               514, 768, 1000, 1024, 1025, 1026, 1500, 2047, 2048])
+@pytest.mark.parametrize("offset", [0, 2])
+def test_classical_full_products(classical, devmem, m, offset):
+    # one warp to 512 threads per product (up to 128, 256, 512, 1024 and 2048
+    # limbs), on rows that are 16-byte aligned (even lengths, no offset) or not:
+    # lengths that small batches, and every batch from 129 limbs on, otherwise
+    # take the transforms for
+    n = 37 if m <= 256 else 9
+    a, b = carry_stress(n, m, seed=m + offset)
+    a[m:2 * m] = b[m:2 * m] = np.uint64(2**64 - 1)
+    got = gpu_mul(classical, devmem, a, b, m, True, offset=offset)
+    assert np.array_equal(got, O.mul(a, b, m, True))
+
+
+@pytest.mark.parametrize("m", [128, 256, 512, 1024, 2048, 4096])
+def test_classical_full_products_of_the_reference(classical, devmem, m):
+    # the reference's own results: the full products behind its fixtures
+    f = golden("ref_full.npz")
+    if f"ha_{m}" not in f.files:
+        pytest.skip("no fixture of this length")
+    n, h = f[f"ha_{m}"].size // m, m // 2
+    a, b = (np.ascontiguousarray(f[k].reshape(n, m)[:, :h]).ravel() for k in (f"ha_{m}", f"hb_{m}"))
+    got = gpu_mul(classical, devmem, a.view(np.uint64), b.view(np.uint64), h // 2, True)
+    assert np.array_equal(got.view(np.uint32), f[f"hmul_{m}"])

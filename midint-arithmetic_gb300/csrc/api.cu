@@ -149,17 +149,16 @@ constexpr uint32_t kFullNttMin = 129;
 // 5.0 of 40, 6.8 of 64, 9.1 of 96; low halves of 48 limbs 6.4.
 constexpr uint32_t kShortNttMin = 42, kShortLoNttMin = 48;
 
-// What the classical launch of a full product takes beside its modelled time (us).
-constexpr double kClassicLaunchUs = 1.8;
-
 // Whether n products of m limbs go to the NTT kernels: by the context's
 // crossover where the caller set it.  While it has the tuning table's value,
 // which is measured on batches that fill the GPU, low halves follow it and
 // small batches take the NTT from fewer limbs on; full products of up to 128
 // limbs take what the two models say is faster (us, classical against NTT: 800 x 42
-// limbs 5.8 against 9.0, 300 x 42 5.7 against 4.2, 1000 x 80 9.9 against 8.3, 1216 x 124
-// 15.0 against 12.4, 3000 x 112 31.7 against 26.6, 10000 x 112 75 against 82, 65536 x
-// 128 455 against 518).
+// limbs 5.8 against 9.0, 300 x 42 5.7 against 4.2, 1500 x 68 11.6 against 12.2, 1000 x 80
+// 9.9 against 8.3, 1216 x 124 15.0 against 12.4, 3000 x 112 31.7 against 26.6, 10000 x
+// 112 75 against 82, 65536 x 128 455 against 518).  Over 600 batches of 42 to 128 limbs
+// the choice costs 0.3 % against the better of the two in the mean, at most 17 % (3300
+// x 112 36.9 against 30.7).
 bool takes_ntt(uint32_t n, uint32_t m, uint32_t knob, bool full, bool vec) {
     if (m > kNttMaxLimbs || m == 0) return false;
     if (knob != (full ? tuned::kPlainNttMin : tuned::kLoNttMin)) return m >= knob;
@@ -170,7 +169,10 @@ bool takes_ntt(uint32_t n, uint32_t m, uint32_t knob, bool full, bool vec) {
     if (n <= 2 * uint32_t(sm_count())) return true;
     double classic = 0;
     kara_pays(n, 2 * m, vec, &classic);
-    return ntt_short_us(n, m) < classic + kClassicLaunchUs;
+    // what a classical launch takes beside its modelled steps: more of it shows
+    // where each scheduler has one warp
+    classic += classic < 10 ? 1.8 : 0.8;
+    return ntt_short_us(n, m) < classic;
 }
 
 // An even number of u32 limbs is half as many

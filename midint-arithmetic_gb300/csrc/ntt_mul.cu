@@ -99,12 +99,12 @@ __global__ void __launch_bounds__((1 << LG) / 8)
 // it the blocks of a cluster wait for one another and for a place (m = 1024,
 // n = 152 22.8 us against 16.5; n = 1024 140 against 89; m = 400, n = 152
 // 13.2 against 11.2; m = 256, n = 300 11.4 against 10.4).
-// 256-point blocks are one warp: m = 96, n = 480 8.1 us against 8.3, n = 600 9.7
-// against 8.3; m = 128, n = 400 8.4 against 10.3, n = 500 10.1 against 10.3; m = 48, n =
+// 256-point blocks are one warp: m = 96, n = 500 8.2 us against 8.3, n = 600 9.7
+// against 8.3; m = 128, n = 420 9.0 against 10.3, n = 500 10.1 against 10.3; m = 48, n =
 // 600 7.0 against 8.2 (alone 19.0 against 18.1), n = 800 9.0 against 8.3.
 // (Low halves to 16: the caller then prefers the classical form to a block each.)
 constexpr double cluster_blocks_per_sm(int lg, bool low) {
-    return lg == 8 ? (low ? 16 : 13.5) : lg == 9 ? 7 : lg <= 11 ? 3 : 2;
+    return lg == 8 ? (low ? 16 : 14) : lg == 9 ? 7 : lg <= 11 ? 3 : 2;
 }
 
 // (blocks: per SM)
@@ -246,14 +246,17 @@ bool ntt_small_batch(uint32_t n, uint32_t m) {
 }
 
 // Clusters: 4.1 us, and from five blocks per SM on 0.45 us for each.  A block
-// per product: by the warps of the busiest scheduler, six at most at a time.
-// Within 10 % of what 13 lengths of 80 to 128 limbs measured in batches of 320 to
-// 10000, 3 % in the middle.
+// per product: the latency of its primes, or 1.025 us for each prime of each warp
+// of the busiest scheduler and what overlaps less while these are few (us for
+// three primes and 1 to 6 warps 8.3, 10.3, 12.3, 14.4, 16.4, 18.5; for five 10.3,
+// 12.4, 17.4, 22.5, 26.6, 30.7), six warps at most at a time.
 double ntt_short_us(uint32_t n, uint32_t m) {
     const int np = 5 - ntt32::ntt_mode(m, m, 256);
     const double blocks = double(n) * np / sm_count(), k = blocks / (4 * np);  // k: warps per scheduler
     if (cluster_fits(blocks, 8, false)) return 4.1 + 0.45 * std::max(0.0, blocks - 5) + 0.6 * (np - 3);
-    return np * (k <= 6 ? 1.24 + 0.816 * std::ceil(k) : 1.023 * k);
+    if (k > 6) return 1.025 * np * k;
+    const double work = np * std::ceil(k);
+    return std::max({8.26, 2.06 * np, 1.025 * work + std::min(2.6, std::max(0.0, 2.6 * (24 - work) / 14))});
 }
 
 mi_status launch_mul_ntt(const uint64_t* a, const uint64_t* b, uint64_t* r, uint32_t n, uint32_t m,

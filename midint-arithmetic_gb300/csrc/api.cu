@@ -158,8 +158,8 @@ constexpr uint32_t kShortNttMin = 42, kShortLoNttMin = 48;
 // 9.9 against 8.3, 1216 x 124 15.0 against 12.4, 3000 x 112 31.7 against 26.6, 10000 x
 // 112 75 against 82, 65536 x 128 455 against 518).  Over 600 batches of 42 to 128 limbs
 // the choice costs 0.3 % against the better of the two in the mean, at most 17 % (3300
-// x 112 36.9 against 30.7).
-bool takes_ntt(uint32_t n, uint32_t m, uint32_t knob, bool full, bool vec) {
+// x 112 36.9 against 30.7).  *form is the classical form where the choice needed it.
+bool takes_ntt(uint32_t n, uint32_t m, uint32_t knob, bool full, bool vec, ClassicForm* form) {
     if (m > kNttMaxLimbs || m == 0) return false;
     if (knob != (full ? tuned::kPlainNttMin : tuned::kLoNttMin)) return m >= knob;
     if (!full) return m >= knob || (m >= kShortLoNttMin && ntt_small_batch(n, m));
@@ -167,19 +167,17 @@ bool takes_ntt(uint32_t n, uint32_t m, uint32_t knob, bool full, bool vec) {
     if (m < kShortNttMin) return false;
     // (the models cost the host 0.2 us, which the smallest batches would show)
     if (n <= 2 * uint32_t(sm_count())) return true;
-    double classic = 0;
-    kara_pays(n, 2 * m, vec, &classic);
+    *form = classic_form(n, 2 * m, true, vec);
     // what a classical launch takes beside its modelled steps: more of it shows
     // where each scheduler has one warp
-    classic += classic < 10 ? 1.8 : 0.8;
-    return ntt_short_us(n, m) < classic;
+    return ntt_short_us(n, m) < form->us + (form->us < 10 ? 1.8 : 0.8);
 }
 
 // An even number of u32 limbs is half as many
 // u64 limbs; the NTT kernels read 8-byte words, so rows that are only 4-byte
 // aligned take the classical kernels, which read 32-bit words.
 mi_status mul_any(mi_ctx ctx, const void* a, const void* b, void* r, uint32_t n, uint32_t limbs, mi_stream stream,
-                  int limb_bytes, bool full) {
+                  int limb_bytes, bool full, uint32_t ntt_from = kFullNttMin) {
     const uint32_t maxl = kMulMaxN32 / (limb_bytes / 4);
     MI_TRY(check_batch(a, b, r, limbs, maxl, full ? "mul_full" : "mul_lo"));
     const size_t in_bytes = size_t(n) * limbs * limb_bytes;
@@ -192,12 +190,13 @@ mi_status mul_any(mi_ctx ctx, const void* a, const void* b, void* r, uint32_t n,
     const uint32_t m = n32 / 2;
     const bool vec = aligned16(a) && aligned16(b) && aligned16(r) && n32 % 4 == 0;
     uint32_t knob = full ? ctx->plain_ntt_min : ctx->lo_ntt_min;
-    if (full && knob != tuned::kPlainNttMin) knob = std::max(knob, kFullNttMin);
-    if (n32 % 2 == 0 && aligned8(a) && aligned8(b) && aligned8(r) && takes_ntt(n, m, knob, full, vec))
+    if (full && knob != tuned::kPlainNttMin) knob = std::max(knob, ntt_from);
+    ClassicForm form;
+    if (n32 % 2 == 0 && aligned8(a) && aligned8(b) && aligned8(r) && takes_ntt(n, m, knob, full, vec, &form))
         return launch_mul_ntt(static_cast<const uint64_t*>(a), static_cast<const uint64_t*>(b),
                               static_cast<uint64_t*>(r), n, m, ctx->ntt.params, pick_stream(ctx, stream), !full);
     return launch_mul_classic(static_cast<const uint32_t*>(a), static_cast<const uint32_t*>(b),
-                              static_cast<uint32_t*>(r), n, n32, full, pick_stream(ctx, stream));
+                              static_cast<uint32_t*>(r), n, n32, full, pick_stream(ctx, stream), 0, false, form);
 }
 
 mi_status mul_ntt(mi_ctx ctx, const uint64_t* a, const uint64_t* b, uint64_t* r, uint32_t n, uint32_t limbs,
@@ -760,10 +759,7 @@ mi_status mi_mul_ntt_u64(mi_ctx ctx, const uint64_t* a, const uint64_t* b, uint6
 mi_status mi_mul_u64(mi_ctx ctx, const uint64_t* a, const uint64_t* b, uint64_t* r, uint32_t n, uint32_t limbs,
                      mi_stream stream) {
     if (ctx == nullptr) return set_error(MI_EINVAL, "null context");
-    const bool vec = aligned16(a) && aligned16(b) && aligned16(r) && limbs % 2 == 0;
-    if (aligned8(a) && aligned8(b) && aligned8(r) && takes_ntt(n, limbs, ctx->plain_ntt_min, true, vec))
-        return mul_ntt(ctx, a, b, r, n, limbs, stream);
-    return mul_any(ctx, a, b, r, n, limbs, stream, 8, true);
+    return mul_any(ctx, a, b, r, n, limbs, stream, 8, true, 1);
 }
 
 // --- reference-shaped host-pointer wrappers ---------------------------------

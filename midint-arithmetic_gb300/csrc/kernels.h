@@ -49,12 +49,23 @@ mi_status launch_add_u32(const uint32_t* a, const uint32_t* b, uint32_t* r, uint
 // Size class of an addition of `bytes` per operand: ceil(log2(u64 limbs)).
 uint32_t add_size_class(uint64_t bytes);
 
+// The form of a batch of classical products: the Karatsuba kernel, or `rounds` of
+// the lane groups (0: the power-of-two groups), and its modelled time.
+struct ClassicForm {
+    bool known = false, kara = false;
+    uint32_t rounds = 0;
+    double us = 0;
+};
+ClassicForm classic_form(uint32_t n, uint32_t n32, bool full, bool vec);
+
 // Classical multiplication on u32 limb views (a u64 buffer with m limbs is a
 // u32 buffer with 2m limbs).  full: r has 2*n32 limbs per instance, else n32.
 // max_per_sm > 0 caps the full-product kernel's resident blocks per SM (by
 // its shared-memory request); link: the operands are read over the host link.
+// form: that of classic_form, where the caller has it (unless max_per_sm > 0).
 mi_status launch_mul_classic(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32,
-                             bool full, cudaStream_t st, uint32_t max_per_sm = 0, bool link = false);
+                             bool full, cudaStream_t st, uint32_t max_per_sm = 0, bool link = false,
+                             ClassicForm form = ClassicForm());
 
 // Dynamic shared memory that leaves room for at most max_per_sm blocks of a
 // kernel per SM (at least `smem`, at most the per-block maximum; 0: `smem`).
@@ -66,16 +77,16 @@ mi_status balanced_smem(uint64_t blocks, uint32_t resident, size_t* smem);
 
 // The same products, full or low half, on groups of any number of lanes
 // (mul_flex.cu): flex_rounds says with how many rounds (1..3), or 0 where the
-// power-of-two groups are faster or hold the product alone; us, where given,
-// is the modelled time.
-uint32_t flex_rounds(uint32_t n, uint32_t n32, bool full, double* us = nullptr);
+// power-of-two groups are faster or hold the product alone; *us is the
+// modelled time.
+uint32_t flex_rounds(uint32_t n, uint32_t n32, bool full, double* us);
 mi_status launch_mul_flex(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32, bool full,
                           uint32_t rounds, cudaStream_t st, bool link = false, uint32_t max_per_sm = 0);
 
 // Full products of 25..32 blocks of 8 u32 limbs with one Karatsuba level
-// (mul_kara.cu), and the batches for which that is the fastest form; us, where
-// given, is the modelled time of the fastest form.
-bool kara_pays(uint32_t n, uint32_t n32, bool vec, double* us = nullptr);
+// (mul_kara.cu), and the batches for which that is faster than the other forms'
+// modelled *us, which then becomes its own.
+bool kara_pays(uint32_t n, uint32_t n32, bool vec, double* us);
 mi_status launch_mul_kara(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32,
                           cudaStream_t st);
 

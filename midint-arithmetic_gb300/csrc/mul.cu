@@ -228,13 +228,22 @@ mi_status balanced_smem(uint64_t blocks, uint32_t resident, size_t* smem) {
     return capped_smem(*smem, uint32_t(places), smem);
 }
 
+ClassicForm classic_form(uint32_t n, uint32_t n32, bool full, bool vec) {
+    ClassicForm f;
+    f.known = true;
+    f.rounds = flex_rounds(n, n32, full, &f.us);
+    f.kara = full && kara_pays(n, n32, vec, &f.us);
+    return f;
+}
+
 mi_status launch_mul_classic(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32, bool full,
-                             cudaStream_t st, uint32_t max_per_sm, bool link) {
+                             cudaStream_t st, uint32_t max_per_sm, bool link, ClassicForm form) {
     const bool vec = aligned16(a) && aligned16(b) && aligned16(r) && (n32 % 4 == 0);
-    if (full && max_per_sm == 0 && kara_pays(n, n32, vec)) return launch_mul_kara(a, b, r, n, n32, st);
     if (!full || max_per_sm == 0) {
-        const uint32_t rounds = flex_rounds(n, n32, full);
-        if (rounds != 0) return launch_mul_flex(a, b, r, n, n32, full, rounds, st, link, max_per_sm);
+        if (!form.known) form = classic_form(n, n32, full, vec);
+        if (form.kara) return launch_mul_kara(a, b, r, n, n32, st);
+        if (form.rounds != 0)
+            return launch_mul_flex(a, b, r, n, n32, full, form.rounds, st, link, max_per_sm);
     }
     if (!full) return launch_mul_lo(a, b, r, n, n32, st);  // half the partial products of a full product
     return vec ? dispatch<true>(a, b, r, n, n32, st, max_per_sm) : dispatch<false>(a, b, r, n, n32, st, max_per_sm);

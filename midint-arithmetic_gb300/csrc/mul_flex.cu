@@ -116,7 +116,7 @@ uint32_t flex_rounds(uint32_t n, uint32_t n32, bool full, double* us) {
         const double cost = double(rounds) * steps * (kFlexA[full][rounds] * waves + kFlexB[full][rounds] * std::ceil(w / 4));
         if (cost < best) best = cost, pick = rounds;
     }
-    if (us != nullptr) *us = best;
+    *us = best;
     return pick;
 }
 

@@ -218,18 +218,13 @@ __global__ void __launch_bounds__(32, 16)
 // 100 33.8 against 35.2, 4000 x 100 34.1 against 31.8, 5000 x 128 48.5 against
 // 46.9, 7000 x 128 56.3 against 61.6, 2280 x 120 21 against 23.7.
 bool kara_pays(uint32_t n, uint32_t n32, bool vec, double* us) {
-    const bool fits = n32 > 24 * T && n32 <= 2 * NT * T;
-    if (!fits && us == nullptr) return false;
-    double other = 0;
-    flex_rounds(n, n32, true, &other);
-    if (us != nullptr) *us = other;
-    if (!fits) return false;
+    if (n32 <= 24 * T || n32 > 2 * NT * T) return false;
     const double w = std::ceil(double(n) / IPB) / sm_count(), steps = 3 * ((n32 + 2 * T - 1) / (2 * T));
     // the first blocks of a second wave crowd the schedulers that free first
     const double k = w <= 16 ? std::ceil(w / 4) : std::max(6.0, std::ceil(w / 4 + 0.1));
     const double own = steps * 0.13 + 0.5 + k * (2.05 + 0.131 * steps);
-    if (own >= (vec ? 0.96 : 0.91) * other) return false;
-    if (us != nullptr) *us = own;
+    if (own >= (vec ? 0.96 : 0.91) * *us) return false;
+    *us = own;
     return true;
 }
 

@@ -113,7 +113,8 @@ def tune_plain_crossover(ctx, stream, dev) -> tuple[int, dict]:
 
     import midint
 
-    sizes = [64, 80, 96, 112, 128, 160, 192, 256, 320, 384, 512, 640, 768, 1024]
+    # (129: the transform length doubles from 128 to 129 and the digit mode changes)
+    sizes = [64, 80, 96, 112, 128, 129, 160, 192, 256, 320, 384, 512, 640, 768, 1024]
     record, ntt_faster = {}, {}
     ctx.set_tuning(midint.TUNE_PLAIN_NTT_MIN, 0, 2049)  # mul_full: classical at every size
     for m in sizes:
@@ -305,13 +306,14 @@ HEADER = """// tuning_table.h -- defaults of the tunable launch choices, written
 namespace mi {{
 namespace tuned {{
 
-// mi_mul_u64: square products of at least this many u64 limbs use the NTT.
+// mi_mul_u64: square products of at least this many u64 limbs use the NTT in
+// batches that fill the GPU (others by the batch while the knob has this value).
 constexpr uint32_t kPlainNttMin = {plain};
 // mi_mul_lo_u64: low halves of products of at least this many u64 limbs come
-// from the NTT kernel (2049 = never).
+// from the NTT kernel (2049 = never); small batches as above.
 constexpr uint32_t kLoNttMin = {lo};
 // mi_poly_u64: composites of at least this many u64 limbs run their four
-// products on the NTT (2049 = never).
+// products on the NTT (2049 = never); small batches as above.
 constexpr uint32_t kPolyNttMin = {poly};
 // Ragged runs: products whose shorter operand has at least this many u64
 // limbs use the NTT kernel (1..257), and so do those from kRaggedNtt40Min

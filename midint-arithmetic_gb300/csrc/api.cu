@@ -156,7 +156,7 @@ constexpr uint32_t kShortNttMin = 42, kShortLoNttMin = 48;
 // limbs take what the two models say is faster (us, classical against NTT: 800 x 42
 // limbs 5.8 against 9.0, 300 x 42 5.7 against 4.2, 1500 x 68 11.6 against 12.2, 1000 x 80
 // 9.9 against 8.3, 1216 x 124 15.0 against 12.4, 3000 x 112 31.7 against 26.6, 10000 x
-// 112 75 against 82, 65536 x 128 455 against 518).  Over 600 batches of 42 to 128 limbs
+// 112 75 against 82, 65536 x 128 454 against 470).  Over 600 batches of 42 to 128 limbs
 // the choice costs 0.3 % against the better of the two in the mean, at most 17 % (3300
 // x 112 36.9 against 30.7).  *form is the classical form where the choice needed it.
 bool takes_ntt(uint32_t n, uint32_t m, uint32_t knob, bool full, bool vec, ClassicForm* form) {

@@ -9,13 +9,14 @@
 namespace mi {
 namespace tuned {
 
-// mi_mul_u64: square products of at least this many u64 limbs use the NTT.
-constexpr uint32_t kPlainNttMin = 128;
+// mi_mul_u64: square products of at least this many u64 limbs use the NTT in
+// batches that fill the GPU (others by the batch while the knob has this value).
+constexpr uint32_t kPlainNttMin = 129;
 // mi_mul_lo_u64: low halves of products of at least this many u64 limbs come
-// from the NTT kernel (2049 = never).
+// from the NTT kernel (2049 = never); small batches as above.
 constexpr uint32_t kLoNttMin = 288;
 // mi_poly_u64: composites of at least this many u64 limbs run their four
-// products on the NTT (2049 = never).
+// products on the NTT (2049 = never); small batches as above.
 constexpr uint32_t kPolyNttMin = 320;
 // Ragged runs: products whose shorter operand has at least this many u64
 // limbs use the NTT kernel (1..257), and so do those from kRaggedNtt40Min

@@ -764,6 +764,15 @@ mi_status dispatch_plain(const L* a, const L* b, L* r, uint8_t* carry, uint32_t 
     constexpr uint32_t Q = 16 / sizeof(L);
     if (link && m >= (sizeof(L) == 8 ? 3 : 13) && m <= Q * 1024)
         return dispatch_gs<L, LIMBS, ADD_PLAIN, int(Q)>(a, b, r, carry, n, m, pow2ceil((m + Q - 1) / Q), st);
+    if constexpr (sizeof(L) == 8) {
+        // lengths a little above three quarters of a group of four rows, whose last
+        // row is nearly empty (us for 2^22, 2^21 and 2^20 limbs with rows against four
+        // limbs per thread: 99 16.7, 10.1, 6.3 against 16.2, 9.5, 5.8; 105 16.7, 10.1, 6.3
+        // against 16.4, 9.7, 6.1; 109 16.6, 9.8, 5.8 against 16.5, 10.0, 6.2; 53 17.2, 10.6,
+        // 6.7 against 17.2, 10.1, 6.2)
+        if (m >= 50 && m <= 54) return launch_one<L, 4, 16, LIMBS, ADD_PLAIN>(a, b, r, carry, n, m, st);
+        if (m >= 97 && m <= 107) return launch_one<L, 4, 32, LIMBS, ADD_PLAIN>(a, b, r, carry, n, m, st);
+    }
     return dispatch_rows<L, ADD_PLAIN>(a, b, r, carry, n, m, rows_per_thread<L>(m), st);
 }
 

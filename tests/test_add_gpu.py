@@ -227,3 +227,19 @@ def test_add_rows_per_thread(ctx, devmem, m, bits):
         ctx.add6(pa, pb, pr, n, m, stream=s)
         torch.cuda.synchronize()
         assert np.array_equal(devmem.get(br, words, off, a.dtype), O.add6(a, b, m))
+
+
+@pytest.mark.parametrize("m", [49, 50, 51, 53, 54, 55, 96, 97, 99, 107, 108, 109])
+def test_add_unaligned_rows_of_four_limbs_per_thread(ctx, devmem, m):
+    # either side of the lengths that take consecutive limbs, in place and not
+    n = 1300
+    a, b = carry_stress(n, m, seed=m)
+    want, carry = O.add(a, b, m)
+    s = torch.cuda.current_stream().cuda_stream
+    for inplace in (False, True):
+        (ba, pa), (bb, pb), (br, pr) = devmem.put(a, 2), devmem.put(b, 2), devmem.empty_words(2 * n * m, 2)
+        dc = torch.full((n + 8,), 7, dtype=torch.uint8, device="cuda:0")
+        ctx.add(pa, pb, pa if inplace else pr, n, m, carry=dc.data_ptr(), stream=s)
+        torch.cuda.synchronize()
+        assert np.array_equal(devmem.get(ba if inplace else br, 2 * n * m, 2), want)
+        assert np.array_equal(dc.cpu().numpy()[:n], carry) and (dc.cpu().numpy()[n:] == 7).all()

@@ -122,6 +122,11 @@ uint32_t flex_rounds(uint32_t n, uint32_t n32, bool full, double* us) {
 
 mi_status launch_mul_flex(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t n, uint32_t n32, bool full,
                           uint32_t rounds, cudaStream_t st, bool link, uint32_t max_per_sm) {
+    // The batches whose rows in flight over the link outgrow the caches (us between
+    // pinned buffers, each lane its rows against one run: 32768 x 8 limbs 82 and 58,
+    // 10922 x 24 56 and 47, 131072 x 4 82 and 62).  Below, and for shorter rows, the
+    // run's arithmetic costs a microsecond (21845 x 5 words 21.1 and 22.2).
+    link = link && !full && n32 > 4 && uint64_t(n) * n32 * 4 >= (n32 <= 8 ? 3u << 20 : 1u << 20);
     const bool vec = aligned16(a) && aligned16(b) && aligned16(r) && (n32 % 4 == 0);
     const FlexShape S = flex_shape(n32, full, rounds, 2);
     const uint64_t blocks = (uint64_t(n) + S.groups - 1) / S.groups;
@@ -132,7 +137,7 @@ mi_status launch_mul_flex(const uint32_t* a, const uint32_t* b, uint32_t* r, uin
         {{k_mul_flex<false, false, 18>, k_mul_flex<false, true, 18>},
          {k_mul_flex<true, false, 18>, k_mul_flex<true, true, 18>}}};
     static constexpr Kernel link_kernels[2] = {k_mul_flex<false, false, 16, true>, k_mul_flex<false, true, 16, true>};
-    const Kernel kern = link && !full ? link_kernels[vec] : kernels[blocks <= 16u * uint64_t(sm_count())][full][vec];
+    const Kernel kern = link ? link_kernels[vec] : kernels[blocks <= 16u * uint64_t(sm_count())][full][vec];
     size_t smem = S.smem();
     // Over the link few resident blocks, as in mul.cu, for their results to leave
     // while the others' operands arrive: four warps for each of its blocks of

@@ -440,3 +440,15 @@ def test_populating_a_result_that_may_not_be_written_fails():
     assert libc.madvise(keep[2], mmap.PAGESIZE, populate_read) == 0
     assert libc.madvise(keep[2], mmap.PAGESIZE, populate_write) != 0
     _release(keep)
+
+
+@pytest.mark.parametrize("m,n", [(5, 157286), (5, 157287), (8, 98303), (8, 98305), (11, 23831), (11, 23833), (24, 10925),
+                                 (95, 2761), (96, 2731)])
+def test_gpuMultiply_runs_of_rows_from_their_size_on(m, n):
+    """Either side of the operand size (1 MB, 3 MB for rows of one block) from
+    which a warp reads its rows as one run."""
+    a, b = carry_stress(n, m, seed=n + m, dtype=np.uint32)
+    keep = [_pinned(x.view(np.int32)) for x in (a, b, np.zeros(n * m, np.uint32))]
+    a2, b2, r = [k.numpy().view(np.uint32) for k in keep]
+    midint.gpuMultiply(midint.U32bits, m, n, a2, b2, r)
+    assert np.array_equal(r, O.mul(a, b, m, False))
